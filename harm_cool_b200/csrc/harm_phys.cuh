@@ -303,20 +303,17 @@ __device__ __forceinline__ void vchar(double gam, const R *pr, const StateT<R> &
 }
 
 // The local Lax-Friedrichs flux of one face (step_ch.c:431-473, HLLF = 0 and
-// LAXF = 1 at :66-67): lf_flux combines the two sides' fluxes F^dir, conserved
-// variables U and wave speeds into F and the face's wave speed ctop;
-// face_side evaluates one side; face_flux is both sides and the combination.
+// LAXF = 1 at :66-67): face_side evaluates one side's fluxes F^dir, conserved
+// variables U and wave speeds; lf_speed is the face's wave speed ctop from the
+// two sides'; F = (Fl + Fr - ctop (Ur - Ul)) / 2 component by component.
 template <class R>
-__device__ __forceinline__ void lf_flux(const R *Fl, const R *Ul, const R &cmaxl, const R &cminl, const R *Fr,
-                                        const R *Ur, const R &cmaxr, const R &cminr, R *F, R &ctop)
+__device__ __forceinline__ R lf_speed(const R &cmaxl, const R &cminl, const R &cmaxr, const R &cminr)
 {
   R t1 = 0. > cmaxl ? R(0.) : cmaxl;
   R cmax = fabs(t1 > cmaxr ? t1 : cmaxr);
   R t2 = 0. > -cminl ? R(0.) : -cminl;
   R cmin = fabs(t2 > -cminr ? t2 : -cminr);
-  ctop = cmax > cmin ? cmax : cmin;
-#pragma unroll
-  for (int k = 0; k < 8; k++) F[k] = 0.5 * (Fl[k] + Fr[k] - ctop * (Ur[k] - Ul[k]));
+  return cmax > cmin ? cmax : cmin;
 }
 
 template <int DIR, class R>
@@ -328,26 +325,6 @@ __device__ __forceinline__ void face_side(double gam, const R *p, const Geo &q, 
   primtoflux(gam, p, s, DIR, q.g, F);
   primtoflux(gam, p, s, 0, q.g, U);
   vchar(gam, p, s, q, DIR, cmax, cmin, fail);
-}
-
-template <int DIR, class R>
-__device__ __forceinline__ void face_flux(double gam, const R *pl, const R *pr, const Geo &q, R *F, R &ctop,
-                                          int *fail)
-{
-  StateT<R> s;
-  R Fl[8], Ul[8], cmaxl, cminl, cmaxr, cminr;
-  get_state(pl, q, s, fail);
-  primtoflux(gam, pl, s, DIR, q.g, Fl);
-  primtoflux(gam, pl, s, 0, q.g, Ul);
-  vchar(gam, pl, s, q, DIR, cmaxl, cminl, fail);
-  get_state(pr, q, s, fail);
-  {
-    R Fr[8], Ur[8];
-    primtoflux(gam, pr, s, DIR, q.g, Fr);
-    primtoflux(gam, pr, s, 0, q.g, Ur);
-    vchar(gam, pr, s, q, DIR, cmaxr, cminr, fail);
-    lf_flux(Fl, Ul, cmaxl, cminl, Fr, Ur, cmaxr, cminr, F, ctop);
-  }
 }
 
 // source() (phys.c:165-207); conn stored as [k][min(nu,j)][max(nu,j)]

@@ -160,24 +160,24 @@ __device__ __forceinline__ float slope_lim_f(int lim, float y1, float y2, float 
   return Dqp;
 }
 
-// the local Lax-Friedrichs flux of one face in float
+// one side of a face in float: fluxes F^dir, conserved variables U, wave speeds
 template <int DIR>
-__device__ __forceinline__ void face_flux_f(float gam, const float *pl, const float *pr, const GeoF &q, float *F,
-                                            float &ctop, int *fail)
+__device__ __forceinline__ void face_side_f(float gam, const float *p, const GeoF &q, float *F, float *U, float &cmax,
+                                            float &cmin, int *fail)
 {
   StateF s;
-  float Fl[8], Ul[8], Fr[8], Ur[8], bsq, cmaxl, cminl, cmaxr, cminr;
-  get_state_f(pl, q, s, fail);
-  fluxes_f<DIR>(gam, pl, s, q.g, Fl, Ul, bsq);
-  vchar_f<DIR>(gam, pl, s, q, bsq, cmaxl, cminl, fail);
-  get_state_f(pr, q, s, fail);
-  fluxes_f<DIR>(gam, pr, s, q.g, Fr, Ur, bsq);
-  vchar_f<DIR>(gam, pr, s, q, bsq, cmaxr, cminr, fail);
+  float bsq;
+  get_state_f(p, q, s, fail);
+  fluxes_f<DIR>(gam, p, s, q.g, F, U, bsq);
+  vchar_f<DIR>(gam, p, s, q, bsq, cmax, cmin, fail);
+}
+
+// the face's wave speed from its two sides' (lf_speed in float)
+__device__ __forceinline__ float lf_speed(float cmaxl, float cminl, float cmaxr, float cminr)
+{
   const float cmax = fabsf(fmaxf(fmaxf(0.f, cmaxl), cmaxr));
   const float cmin = fabsf(fmaxf(fmaxf(0.f, -cminl), -cminr));
-  ctop = fmaxf(cmax, cmin);
-#pragma unroll
-  for (int k = 0; k < 8; k++) F[k] = 0.5f * (Fl[k] + Fr[k] - ctop * (Ur[k] - Ul[k]));
+  return fmaxf(cmax, cmin);
 }
 
 // ---------------------------------------------------------------------------

@@ -10,6 +10,8 @@
 // connection source, U accumulation, the Noble inversion and the floors in
 // double.
 #pragma once
+#include <cuda_pipeline.h>
+
 #include "harm_common.cuh"
 #if HARM_STEP_MIXED
 #include "harm_phys32.cuh"
@@ -28,12 +30,8 @@
 #ifndef HARM_INV_MINB
 #define HARM_INV_MINB 1
 #endif
-// phi planes each block sweeps, for the flux and for the zone kernels:
-// consecutive planes of one (r, theta) tile reuse its geometry and (for the
-// phi-direction fluxes) its stencil from L1
-#ifndef HARM_HB_FLUX
-#define HARM_HB_FLUX 1
-#endif
+// phi planes each block of the zone kernels sweeps: consecutive planes of one
+// (r, theta) tile reuse its geometry from L1
 #ifndef HARM_HB_ZONE
 #define HARM_HB_ZONE 4
 #endif
@@ -60,119 +58,245 @@ __host__ __device__ __forceinline__ int faces_per_row(const Grid &G) { return DI
 template <int DIR>
 __host__ __device__ __forceinline__ int face_rows(const Grid &G) { return DIR == 1 ? G.n1 + 1 : G.n1 + 2; }
 
-// One thread per face of direction DIR.  Face ranges (step_ch.c:407): dir 1
-// i in [istart, istop+1], j in [jstart-1, jstop+1]; dir 2 i in [istart-1,
-// istop+1], j in [jstart, jstop+1] (the polar faces jstart and jstop+1 carry
-// no flux, :412-416); dir 3 i in [istart-1, istop+1], j in [jstart-1, jstop+1].
+// The face fluxes of every direction in one launch.  Face ranges
+// (step_ch.c:407): dir 1 i in [istart, istop+1], j in [jstart-1, jstop+1]; dir 2
+// i in [istart-1, istop+1], j in [jstart, jstop+1] (the polar faces jstart and
+// jstop+1 carry no flux, :412-416); dir 3 i in [istart-1, istop+1], j in
+// [jstart-1, jstop+1].
+//
+// A block holds FLUX_FACES faces of one direction and phi plane, numbered row
+// by row (theta fastest), so that only the plane's last warps have idle lanes.
+// Two threads share a face: the first half of the block evaluates the left
+// sides, the second half the right sides of the same faces.  They hand each
+// other half of their fluxes and conserved variables through shared memory, and
+// each forms and stores four of the face's eight fluxes.  The four zones of a
+// face's stencil and its metric are copied to shared memory asynchronously, all
+// at once, so that a warp waits for one round trip to L2.
+//
+// What bounds it: issue slots and the latency of dependent FP64 instructions.
+// One thread per face held both sides (300 B of spills a thread at 72 registers),
+// waited for its loads a few at a time (5.9 of 13.1 warps per issue stalled on
+// memory) and issued on half of the cycles; in this form 2.7 stall on memory and
+// it issues on 0.62 (FP64) and 0.79 (mixed) of them.  192x192x64, the three
+// directions: FP64 825 -> 699 us (the split alone, without the staging, 893),
+// mixed 447 -> 428; 288x256x256 FP64 6.77 -> 5.62 ms; 128x128 (launch included)
+// 27.7 -> 14.2 us.  64 and 56 registers (8 and 9 blocks) spill again: 756, 810 us.
+constexpr int FLUX_FACES = 64;
+
+#if HARM_STEP_MIXED
+using face_t = float;
+using face_geo = GeoF;
+#else
+using face_t = double;
+using face_geo = Geo;
+#endif
+
+// the metric entries a face of direction DIR reads, as planes of geo (load_geo's order)
+constexpr int FLUX_NG = HARM_STEP_MIXED ? 12 : 14;
+template <int DIR>
+__device__ constexpr int face_plane(int e)
+{
+  // v00 v01 v03 v11 v13 v22 v33, n00 n01 n03, n^{dir dir}, g, alpha, 1/alpha
+  return e < 10 ? e : e == 10 ? (DIR == 1 ? 11 : DIR == 2 ? 13 : 16) : e + 6;
+}
+
+struct FluxShared {
+  union {
+    double p[8][4][FLUX_FACES];      // primitives of zone-2d, zone-d, zone, zone+d of each face
+    face_t x[10][2 * FLUX_FACES];    // four fluxes, four conserved variables, the two wave speeds
+  };
+  face_t g[FLUX_NG][FLUX_FACES];
+  int fail[2 * FLUX_FACES];
+  double red[4];
+};
+
+// one block's faces of direction DIR; returns this thread's Courant limit.
 // REC (the discrete adjoint's recomputation): also keep the wave speed of every
 // face that takes part in the Courant minimum, in ctrec[(DIR - 1) nc + cell].
-template <int DIR, bool FULL, bool REC = false>
-__global__ void __launch_bounds__(128, HARM_FLUX_MINB) k_flux(Grid G, const double *__restrict__ pb, flux_t *__restrict__ F,
-                                              const double *__restrict__ geo, const float *__restrict__ geo32,
-                                              DevScalars *sc, double *__restrict__ ctrec)
+template <int DIR, bool FULL, bool REC>
+__device__ __forceinline__ double flux_block(const Grid &G, int fb, int h, const double *__restrict__ pb,
+                                             flux_t *__restrict__ F, const face_t *__restrict__ geo, DevScalars *sc,
+                                             double *__restrict__ ctrec, FluxShared &S)
 {
-  if (sc->halted) return;
-  // faces of one phi plane numbered row by row (theta fastest), 128 per block,
-  // so that only the plane's last warp has idle lanes
+  const int t = threadIdx.x, side = t / FLUX_FACES, s = t % FLUX_FACES;
   const int nj = faces_per_row<DIR>(G);
-  const int f = blockIdx.x * 128 + threadIdx.y * blockDim.x + threadIdx.x;
+  const int f = fb * FLUX_FACES + s;
   const int j = (DIR == 2 ? G.jstart : G.jstart - 1) + f % nj;
   const int i = (DIR == 1 ? G.istart : G.istart - 1) + f / nj;
-  const int h0 = blockIdx.z * HARM_HB_FLUX, h1 = min(G.n3, h0 + HARM_HB_FLUX);
-  double dtmin = 1.e9;
   const bool in = i <= G.istop + 1;
-  if (in) for (int h = h0; h < h1; h++) {
-    const long c = cidx(G, h, i, j);
-    if (DIR == 2 && (j == G.jstart || j == G.jstop + 1)) {
+  const bool pole = DIR == 2 && (j == G.jstart || j == G.jstop + 1);
+  const bool calc = in && !pole;
+  const long c = cidx(G, h, i, j);
+  if (calc) {
+    // this thread brings two of the face's four zones and half of its metric
+    long o1, o2;
+    if (DIR == 1) { o1 = c + (2 * side - 2) * (long)G.sn2; o2 = o1 + G.sn2; }
+    else if (DIR == 2) { o1 = c + 2 * side - 2; o2 = o1 + 1; }
+    else {
+      o1 = cidx(G, hwrap(G, h + 2 * side - 2), i, j);
+      o2 = cidx(G, hwrap(G, h + 2 * side - 1), i, j);
+    }
 #pragma unroll
-      for (int k = 0; k < 8; k++) F[k * G.nc + c] = 0.;
+    for (int k = 0; k < 8; k++) {
+      __pipeline_memcpy_async(&S.p[k][2 * side][s], pb + k * G.nc + o1, 8);
+      __pipeline_memcpy_async(&S.p[k][2 * side + 1][s], pb + k * G.nc + o2, 8);
+    }
+    const face_t *gp = geo + (long)(DIR - 1) * GEO_N * G.ng + (long)i * G.sn2 + j;
+    if (side == 0) {
+#pragma unroll
+      for (int e = 0; e < FLUX_NG / 2; e++)
+        __pipeline_memcpy_async(&S.g[e][s], gp + face_plane<DIR>(e) * G.ng, sizeof(face_t));
     } else {
-      long o1, o2, o3;  // zone-2d, zone-d, zone+d
-      if (DIR == 1) { o1 = c - 2 * G.sn2; o2 = c - G.sn2; o3 = c + G.sn2; }
-      else if (DIR == 2) { o1 = c - 2; o2 = c - 1; o3 = c + 1; }
-      else {
-        o1 = cidx(G, hwrap(G, h - 2), i, j);
-        o2 = cidx(G, hwrap(G, h - 1), i, j);
-        o3 = cidx(G, hwrap(G, h + 1), i, j);
-      }
+#pragma unroll
+      for (int e = FLUX_NG / 2; e < FLUX_NG; e++)
+        __pipeline_memcpy_async(&S.g[e][s], gp + face_plane<DIR>(e) * G.ng, sizeof(face_t));
+    }
+  }
+  __pipeline_commit();
+  __pipeline_wait_prior(0);
+  __syncthreads();
+  face_t Fs[8], Us[8], cx, cn;
+  face_t p[8];
+  if (calc) {
+    const face_t half = side ? (face_t)-0.5 : (face_t)0.5;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const face_t a = (face_t)S.p[k][side][s], b = (face_t)S.p[k][side + 1][s], e = (face_t)S.p[k][side + 2][s];
 #if HARM_STEP_MIXED
-      float pl[8], pr[8];
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const double *P = pb + k * G.nc;
-        float a = (float)__ldg(P + o1), b = (float)__ldg(P + o2), z = (float)__ldg(P + c), e = (float)__ldg(P + o3);
-        pl[k] = b + 0.5f * slope_lim_f(G.lim, a, b, z);
-        pr[k] = z - 0.5f * slope_lim_f(G.lim, b, z, e);
-      }
-      GeoF q;
-      load_geo_f(geo32 + (long)(DIR - 1) * GEO_N * G.ng, G.ng, (long)i * G.sn2 + j, q);
-      float Fz[8], ctopf;
-      int fail = 0;
-      face_flux_f<DIR>((float)G.gam, pl, pr, q, Fz, ctopf, &fail);
-      const double ctop = (double)ctopf;
+      p[k] = b + half * slope_lim_f(G.lim, a, b, e);
 #else
-      double pl[8], pr[8];
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const double *P = pb + k * G.nc;
-        double a = __ldg(P + o1), b = __ldg(P + o2), z = __ldg(P + c), e = __ldg(P + o3);
-        pl[k] = b + 0.5 * slope_lim(G.lim, a, b, z);
-        pr[k] = z - 0.5 * slope_lim(G.lim, b, z, e);
-      }
-      Geo q;
-      load_geo(geo_at(geo, G, DIR == 1 ? L_FACE1 : DIR == 2 ? L_FACE2 : L_FACE3), G.ng, (long)i * G.sn2 + j, q);
-      double Fz[8], ctop;
-      int fail = 0;
-      face_flux<DIR>(G.gam, pl, pr, q, Fz, ctop, &fail);
+      p[k] = b + half * slope_lim(G.lim, a, b, e);
 #endif
+    }
+  }
+  __syncthreads();  // the stencil's space takes the exchange
+  if (calc) {
+    face_geo q;
+    q.v00 = S.g[0][s]; q.v01 = S.g[1][s]; q.v03 = S.g[2][s]; q.v11 = S.g[3][s]; q.v13 = S.g[4][s];
+    q.v22 = S.g[5][s]; q.v33 = S.g[6][s];
+    q.n00 = S.g[7][s]; q.n01 = S.g[8][s]; q.n03 = S.g[9][s];
+    if (DIR == 1) q.n11 = S.g[10][s];
+    else if (DIR == 2) q.n22 = S.g[10][s];
+    else q.n33 = S.g[10][s];
+    q.g = S.g[11][s];
+    int fail = 0;
+#if HARM_STEP_MIXED
+    face_side_f<DIR>((float)G.gam, p, q, Fs, Us, cx, cn, &fail);
+#else
+    q.alpha = S.g[12][s];
+    q.ialpha = S.g[13][s];
+    face_side<DIR>(G.gam, p, q, Fs, Us, cx, cn, &fail);
+#endif
+    if (side == 0) {
 #pragma unroll
-      for (int k = 0; k < 8; k++) F[k * G.nc + c] = Fz[k];
+      for (int k = 0; k < 4; k++) { S.x[k][t] = Fs[4 + k]; S.x[4 + k][t] = Us[4 + k]; }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; k++) { S.x[k][t] = Fs[k]; S.x[4 + k][t] = Us[k]; }
+    }
+    S.x[8][t] = cx;
+    S.x[9][t] = cn;
+    S.fail[t] = fail;
+  }
+  __syncthreads();
+  double dtmin = 1.e9;
+  if (in && pole) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) F[(4 * side + k) * G.nc + c] = 0.;
+  } else if (in) {
+    const int o = t ^ FLUX_FACES;  // the face's other side
+    const face_t ox = S.x[8][o], on = S.x[9][o];
+    const face_t ctop = side == 0 ? lf_speed(cx, cn, ox, on) : lf_speed(ox, on, cx, cn);
+    if (side == 0) {
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        F[k * G.nc + c] = (face_t)0.5 * (Fs[k] + S.x[k][o] - ctop * (S.x[4 + k][o] - Us[k]));
+      // the code the sides leave, the right one's last
+      const int fail = S.fail[o] ? S.fail[o] : S.fail[t];
       if (fail) record_fail(sc, fail, h + (G.n3 > 1 ? 1 : 0), i, j);
       if (FULL && i >= G.istart && i <= G.istop && j >= G.jstart && j <= G.jstop) {
         const double dxd = DIR == 1 ? G.dx1 : DIR == 2 ? G.dx2 : G.dx3;
-        dtmin = fmin(dtmin, G.cour * dxd / ctop);
-        if (REC) ctrec[(DIR - 1) * G.nc + c] = ctop;
+        dtmin = G.cour * dxd / (double)ctop;
+        if (REC && DIR < 3) ctrec[(DIR - 1) * G.nc + c] = (double)ctop;
       }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        F[(4 + k) * G.nc + c] = (face_t)0.5 * (S.x[k][o] + Fs[4 + k] - ctop * (Us[4 + k] - S.x[4 + k][o]));
     }
   }
+  return dtmin;
+}
+
+// blocks per phi plane of each direction
+struct FluxBlocks {
+  int b1, b2, b3;
+};
+
+template <bool FULL, bool REC, bool THREE_D>
+__global__ void __launch_bounds__(2 * FLUX_FACES, HARM_FLUX_MINB) k_flux(Grid G, FluxBlocks nb,
+                                                                         const double *__restrict__ pb,
+                                                                         flux_t *__restrict__ F1,
+                                                                         flux_t *__restrict__ F2,
+                                                                         flux_t *__restrict__ F3,
+                                                                         const face_t *__restrict__ geo,
+                                                                         DevScalars *sc, double *__restrict__ ctrec)
+{
+  if (sc->halted) return;
+  __shared__ FluxShared S;
+  int b = blockIdx.x, dir;
+  double dtmin;
+  if (b < nb.b1 * G.n3) {
+    dir = 1;
+    dtmin = flux_block<1, FULL, REC>(G, b % nb.b1, b / nb.b1, pb, F1, geo, sc, ctrec, S);
+  } else if (!THREE_D || (b -= nb.b1 * G.n3) < nb.b2 * G.n3) {
+    if (!THREE_D) b -= nb.b1;
+    dir = 2;
+    dtmin = flux_block<2, FULL, REC>(G, b % nb.b2, b / nb.b2, pb, F2, geo, sc, ctrec, S);
+  } else {
+    b -= nb.b2 * G.n3;
+    dir = 3;
+    dtmin = flux_block<3, FULL, REC>(G, b % nb.b3, b / nb.b3, pb, F3, geo, sc, ctrec, S);
+  }
   if (FULL) {
-    __shared__ double red[4];
-    const int t = threadIdx.y * blockDim.x + threadIdx.x;
+    const int t = threadIdx.x;
     double v = warp_min(dtmin);
-    if ((t & 31) == 0) red[t >> 5] = v;
+    if ((t & 31) == 0) S.red[t >> 5] = v;
     __syncthreads();
     if (t == 0) {
-      v = fmin(fmin(red[0], red[1]), fmin(red[2], red[3]));
-      if (v < 1.e9) atomicMin(&sc->ndt_bits[DIR - 1], (unsigned long long)__double_as_longlong(v));
+      v = fmin(fmin(S.red[0], S.red[1]), fmin(S.red[2], S.red[3]));
+      if (v < 1.e9) atomicMin(&sc->ndt_bits[dir - 1], (unsigned long long)__double_as_longlong(v));
     }
   }
 }
 
-
 // ctrec (the adjoint's recomputation of a corrector): keep the direction-1
 // and -2 faces' wave speeds there
 template <bool FULL>
-void launch_flux(const Grid &G, dim3 b, cudaStream_t st, const double *pb, flux_t *F1, flux_t *F2, flux_t *F3,
-                 const double *geo, const float *geo32, DevScalars *sc, double *ctrec = nullptr)
+void launch_flux(const Grid &G, cudaStream_t st, const double *pb, flux_t *F1, flux_t *F2, flux_t *F3,
+                 const double *geo64, const float *geo32, DevScalars *sc, double *ctrec = nullptr)
 {
-  const int gz = (G.n3 + HARM_HB_FLUX - 1) / HARM_HB_FLUX;
-  // 128 faces per block whatever the tile's shape
-  dim3 g1((faces_per_row<1>(G) * face_rows<1>(G) + 127) / 128, 1, gz);
-  dim3 g2((faces_per_row<2>(G) * face_rows<2>(G) + 127) / 128, 1, gz);
-  dim3 g3((faces_per_row<3>(G) * face_rows<3>(G) + 127) / 128, 1, gz);
+#if HARM_STEP_MIXED
+  const float *geo = geo32;
+#else
+  const double *geo = geo64;
+#endif
+  auto blocks = [](int faces) { return (faces + FLUX_FACES - 1) / FLUX_FACES; };
+  const FluxBlocks nb{blocks(faces_per_row<1>(G) * face_rows<1>(G)), blocks(faces_per_row<2>(G) * face_rows<2>(G)),
+                      G.n3 > 1 ? blocks(faces_per_row<3>(G) * face_rows<3>(G)) : 0};
+  const unsigned grid = (unsigned)(nb.b1 + nb.b2 + nb.b3) * G.n3;
+  const int nt = 2 * FLUX_FACES;
 #if !HARM_STEP_MIXED
   if (FULL && ctrec) {
     // ctrec holds directions 1 and 2 (the adjoint that reads it is 2D); a 3D
     // step still gets its phi fluxes, without a record
-    k_flux<1, true, true><<<g1, b, 0, st>>>(G, pb, F1, geo, geo32, sc, ctrec);
-    k_flux<2, true, true><<<g2, b, 0, st>>>(G, pb, F2, geo, geo32, sc, ctrec);
-    if (G.n3 > 1) k_flux<3, true><<<g3, b, 0, st>>>(G, pb, F3, geo, geo32, sc, nullptr);
+    if (G.n3 > 1) k_flux<true, true, true><<<grid, nt, 0, st>>>(G, nb, pb, F1, F2, F3, geo, sc, ctrec);
+    else k_flux<true, true, false><<<grid, nt, 0, st>>>(G, nb, pb, F1, F2, F3, geo, sc, ctrec);
     return;
   }
 #endif
-  k_flux<1, FULL><<<g1, b, 0, st>>>(G, pb, F1, geo, geo32, sc, nullptr);
-  k_flux<2, FULL><<<g2, b, 0, st>>>(G, pb, F2, geo, geo32, sc, nullptr);
-  if (G.n3 > 1) k_flux<3, FULL><<<g3, b, 0, st>>>(G, pb, F3, geo, geo32, sc, nullptr);
+  if (G.n3 > 1) k_flux<FULL, false, true><<<grid, nt, 0, st>>>(G, nb, pb, F1, F2, F3, geo, sc, nullptr);
+  else k_flux<FULL, false, false><<<grid, nt, 0, st>>>(G, nb, pb, F1, F2, F3, geo, sc, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -610,7 +734,7 @@ template <bool FULL>
 void launch_half(Ctx *x, const double *pi, const double *pb, double *pf)
 {
   Bufs B = bufs(x);
-  launch_flux<FULL>(x->G, dim3(x->tbx, x->tby), x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc);
+  launch_flux<FULL>(x->G, x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc);
   launch_update<FULL>(x, pi, pb, pf);
   if (FULL) k_diag_flux<<<1, 1024, 0, x->stream>>>(x->G, B.F1, x->sc);
   launch_bound(x, pf);
@@ -637,7 +761,7 @@ static void launch_half_rec(Ctx *x, const double *pi, const double *pb, double *
   const int s = FULL ? 1 : 0;
   const size_t nc = (size_t)x->G.nc;
   Bufs B = bufs(x);
-  launch_flux<FULL>(x->G, dim3(x->tbx, x->tby), x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc,
+  launch_flux<FULL>(x->G, x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc,
                     FULL ? r.ctop : nullptr);
   cudaMemcpyAsync(r.F1rho[s], B.F1 + RHO * nc, nc * sizeof(double), cudaMemcpyDeviceToDevice, x->stream);
   launch_update<FULL>(x, pi, pb, pf, r.Z[s], r.wz[s]);
@@ -682,8 +806,8 @@ int time_kernels(Ctx *x, int reps, double *ms)
       const bool full = half == 1;
       double *pi = x->p, *pb = full ? x->ph : x->p, *pf = full ? x->p : x->ph;
       const dim3 tile(x->tbx, x->tby);
-      if (full) launch_flux<true>(G, tile, x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc);
-      else launch_flux<false>(G, tile, x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc);
+      if (full) launch_flux<true>(G, x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc);
+      else launch_flux<false>(G, x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc);
       slot[e] = 0; CK(cudaEventRecord(ev[e++], x->stream));
       if (full) launch_update<true>(x, pi, pb, pf);
       else launch_update<false>(x, pi, pb, pf);
