@@ -53,16 +53,16 @@ constexpr int GEO_N = 21;
 // divergence), the adiabatic index (the Noble pressure), u^t (bcon_calc).  An
 // IEEE double division costs about 14 FP64 issue slots on sm_100; with
 // y = 1/b rounded to nearest formed once, div_rn returns the same correctly
-// rounded quotient in 6:
+// rounded quotient in 5:
 //  * q = a y is within two ulps of a/b, and one FMA correction
 //    q + (a - b q) y (Markstein, IBM J. Res. Dev. 34:111-119, 1990) brings it
 //    within one ulp: q is then a faithful quotient;
 //  * for a faithful q the remainder r = a - b q is a double, so fma(-q, b, a)
 //    forms it exactly (Boldo and Daumas, ARITH-16, 2003);
-//  * a/b = q + r/b, so q is the nearest double to a/b exactly when |r| is
-//    below b times half the gap between q and its neighbour on the side of a/b
-//    (a power of two, so that product is exact); otherwise the neighbour is.
-//    a/b is never halfway between two doubles, so there is no tie.
+//  * with y = RN(1/b), a faithful q and that exact remainder, RN(q + r y) is the
+//    correctly rounded a/b (Markstein's theorem, same paper): one more FMA.
+// Five FP64 operations and the range check.  (Comparing |r| with half the gap to
+// q's neighbour instead took one FP64 operation and a dozen integer ones more.)
 // y must be RN(1/b).  Divisors other than b > 0 in [2^-60, 2^61), and
 // numerators outside [2^-800, 2^800] in magnitude (subnormal, huge, inf, NaN),
 // take the IEEE division; a zero numerator gives a y, the signed zero a/b is.
@@ -82,17 +82,7 @@ __device__ __forceinline__ double div_rn(double a, double b, double y)
   double r = fma(-q, b, a);
   q = fma(r, y, q);
   r = fma(-q, b, a);
-  long long iq = __double_as_longlong(q);
-  const bool up = (r > 0.) == (q > 0.);                     // |a/b| > |q|
-  const int eq = (int)((iq >> 52) & 0x7ff);
-  // half the gap to the neighbour towards a/b: a quarter ulp below a power of two
-  const int eh = eq - 53 - ((!up && (iq & 0xfffffffffffffLL) == 0) ? 1 : 0);
-  const double hb = __longlong_as_double((long long)eh << 52) * b;
-  if (fabs(r) > hb) {
-    iq += up ? 1 : -1;
-    q = __longlong_as_double(iq);
-  }
-  return q;
+  return fma(r, y, q);
 }
 
 // div_rn for a divisor formed at run time: its reciprocal is one IEEE division,
