@@ -34,10 +34,10 @@ sys.path.insert(0, ROOT)
 
 def kernels_per_step(n3):
     """Kernel launches of one step: per half step the flux kernel, the corner EMFs,
-    the conserved update and the inversion, bound_prim, the flag flip, the two
-    repair kernels (list and wavefront), bound_prim; the corrector adds the flux
+    the conserved update and the inversion, bound_prim, the flag flip, the
+    repair, bound_prim; the corrector adds the flux
     diagnostics; then the mass diagnostics and the dt update."""
-    return 2 * (1 + 8) + 1 + 2
+    return 2 * (1 + 7) + 1 + 2
 METRIC = "zone-cycles/s 288x256x256 GRMHD step_ch: FP64, mixed precision beside it"
 STATE_BYTES_PER_ZONE_CYCLE = 320  # p read twice, ph written and read, p written; 8 FP64 prims
 

@@ -14,11 +14,11 @@
 // connection planes and two floor planes.
 //
 // One step (step_ch.c:90-140) is, on one stream and without host sync:
-//   predictor : k_flux x3, k_update(dt/2) [flux-CT, source, inversion, floors],
-//               k_bound, k_fu_flip, k_fu_fix, k_bound
-//   corrector : k_flux x3 (+Courant minima), k_update(dt), k_diag_flux,
-//               k_bound, k_fu_flip, k_fu_fix, k_bound
+//   predictor : k_flux, k_emf, k_cons, k_invert (dt/2) [flux-CT, source,
+//               inversion, floors], k_bound, k_fu_flip, k_repair, k_bound
+//   corrector : the same with dt and the Courant minima, and k_diag_flux
 //   k_diag_mass, k_finalize (diagnostic sums, next dt)
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -96,17 +96,15 @@ __global__ void k_bound(Grid G, double *P, signed char *pflag, const double *__r
 // then repairs failed zones in loop order, in place.  Repairs from the edge
 // or corner stencils read only good zones, which the repair never changes;
 // the last-resort average reads every neighbour and so sees earlier repairs.
-// k_fu_flip flips the flags and lists the failed zones.  For a few failures
-// k_fu_fix sorts the list into loop order, precomputes the stencil repairs in
-// parallel and then replays the whole list in order on one thread,
-// recomputing any zone whose stencil choice changed or that needs the
-// last-resort average.  For many failures k_fu_wave repairs them in
-// wavefronts instead: a repair reads only its own phi plane, and within a
-// plane zone (i, j) depends only on (i-1, j-1..j+1) and (i, j-1), all on
-// earlier lines 2i + j = const, so each plane is one block that sweeps those
-// lines in order with a barrier between them -- the loop order's results.
+// k_fu_flip flips the flags and lists the failed zones; k_repair repairs them.
+// For a few failures (up to FIX_LIST_MAX, about 2 us each in the worst case, against
+// some 100 us for a plane) one block sorts the list into loop order, precomputes the
+// stencil repairs in parallel and then replays the whole list in order on one
+// thread, recomputing any zone whose stencil choice changed or that needs the
+// last-resort average.  For more, each phi plane (a repair reads only its own
+// plane) is repaired by repair_plane.
 
-__global__ void k_fu_flip(Grid G, signed char *pflag, int *list, DevScalars *sc)
+__global__ void k_fu_flip(Grid G, signed char *pflag, int *list, DevScalars *sc, int slot)
 {
   if (sc->halted) return;
   const long n = G.nc;
@@ -117,9 +115,8 @@ __global__ void k_fu_flip(Grid G, signed char *pflag, int *list, DevScalars *sc)
     if (nf == 0) {
       int j = (int)(c % G.sn2), i = (int)((c / G.sn2) % G.sn1);
       if (i >= G.istart && i <= G.istop && j >= G.jstart && j <= G.jstop) {
-        int slot = atomicAdd(&sc->nfail, 1);
-        if (slot < FAIL_CAP) list[slot] = (int)c;
-        else sc->fail_overflow = 1;
+        int k = atomicAdd(&sc->nfail[slot], 1);
+        if (k < FAIL_CAP) list[k] = (int)c;
       }
     }
   }
@@ -132,135 +129,282 @@ __device__ __forceinline__ void cell_hij(const Grid &G, long c, int &h, int &i, 
   h = (int)(c / ((long)G.sn2 * G.sn1));
 }
 
-__global__ void __launch_bounds__(NTHR_FIX) k_fu_fix(Grid G, double *P, signed char *pflag, int *list, double *fixbuf,
-                                                     const double *__restrict__ geo, const double *__restrict__ floors,
-                                                     DevScalars *sc)
+// floors of one repaired zone (fixup.c:142-383); true for a gamma failure
+static __device__ bool fix_zone(const Grid &G, const double *__restrict__ geo, const double *__restrict__ floors, int i,
+                                int j, double *v, int *fail)
 {
-  if (sc->halted) return;
+  const long gi = (long)i * G.sn2 + j;
+  Geo q;
+  load_geo(geo_at(geo, G, L_CENT), G.ng, gi, q);
+  return fixup1zone(G.gam, __ldg(floors + gi), __ldg(floors + G.ng + gi), q, v, fail);
+}
+
+// the repair of zone (h, i, j) in place, from the flags and values as they stand
+static __device__ void repair_in_place(const Grid &G, double *P, signed char *pflag, const double *__restrict__ geo,
+                                       const double *__restrict__ floors, DevScalars *sc, int h, int i, int j)
+{
+  const long c = cidx(G, h, i, j);
+  double v[8];
+  repair_zone(G, P, c, stencil_kind(G, pflag, c), v);
+  int fail = 0;
+  const bool g33 = fix_zone(G, geo, floors, i, j, v, &fail);
+  if (fail) record_fail(sc, fail, h + (G.n3 > 1 ? 1 : 0), i, j);
+  for (int k = 0; k < 8; k++) P[k * G.nc + c] = v[k];
+  pflag[c] = g33 ? (signed char)-33 : (signed char)0;
+}
+
+// up to FIX_LIST_MAX failures, by one block
+__device__ void repair_list(const Grid &G, double *P, signed char *pflag, const int *list, int n, double *fixbuf,
+                            const double *__restrict__ geo, const double *__restrict__ floors, DevScalars *sc)
+{
   __shared__ int keys[FIX_LIST_MAX];
   __shared__ signed char kinds[FIX_LIST_MAX];
-  __shared__ int gfail;
-  const int n = sc->nfail;
-  if (n == 0) return;
-  if (n > FIX_LIST_MAX || sc->fail_overflow) return;  // k_fu_wave's case
   const int tid = threadIdx.x;
-  if (tid == 0) gfail = 0;
-  const double *gC = geo_at(geo, G, L_CENT);
-  {
-    // bitonic sort of the failed cells into loop order
-    int m = 1;
-    while (m < n) m <<= 1;
-    for (int t = tid; t < m; t += blockDim.x) keys[t] = t < n ? list[t] : 0x7fffffff;
-    __syncthreads();
-    for (int size = 2; size <= m; size <<= 1)
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        for (int t = tid; t < m; t += blockDim.x) {
-          int u = t ^ stride;
-          if (u > t) {
-            bool up = (t & size) == 0;
-            int a = keys[t], b = keys[u];
-            if ((a > b) == up) { keys[t] = b; keys[u] = a; }
-          }
-        }
-        __syncthreads();
-      }
-    // parallel: stencil repairs from the flags as they stand now
-    for (int t = tid; t < n; t += blockDim.x) {
-      long c = keys[t];
-      int kind = stencil_kind(G, pflag, c);
-      kinds[t] = (signed char)kind;
-      if (kind < 2) {
-        double v[8];
-        repair_zone(G, P, c, kind, v);
-        int h, i, j;
-        cell_hij(G, c, h, i, j);
-        long gi = (long)i * G.sn2 + j;
-        Geo q;
-        load_geo(gC, G.ng, gi, q);
-        int fail = 0;
-        bool g33 = fixup1zone(G.gam, floors[gi], floors[G.ng + gi], q, v, &fail);
-        if (fail) record_fail(sc, fail, h + (G.n3 > 1 ? 1 : 0), i, j);
-        if (g33) kinds[t] = (signed char)(kinds[t] | 4);
-        for (int k = 0; k < 8; k++) fixbuf[(long)t * 8 + k] = v[k];
-      }
+  // loop order: each zone's place is the number of zones before it
+  if (tid < n) {
+    const int me = list[tid];
+    int r = 0;
+    for (int t = 0; t < n; t++) r += list[t] < me;
+    keys[r] = me;
+  }
+  __syncthreads();
+  // parallel: stencil repairs from the flags as they stand now
+  if (tid < n) {
+    const long c = keys[tid];
+    const int kind = stencil_kind(G, pflag, c);
+    kinds[tid] = (signed char)kind;
+    if (kind < 2) {
+      double v[8];
+      repair_zone(G, P, c, kind, v);
+      int h, i, j, fail = 0;
+      cell_hij(G, c, h, i, j);
+      if (fix_zone(G, geo, floors, i, j, v, &fail)) kinds[tid] = (signed char)(kind | 4);
+      if (fail) record_fail(sc, fail, h + (G.n3 > 1 ? 1 : 0), i, j);
+      for (int k = 0; k < 8; k++) fixbuf[(long)tid * 8 + k] = v[k];
     }
-    __syncthreads();
-    // in order, one thread
-    if (tid == 0) {
-      for (int t = 0; t < n; t++) {
-        long c = keys[t];
-        int kind = stencil_kind(G, pflag, c);
-        int pre = kinds[t] & 3;
-        double v[8];
-        bool g33;
-        int h, i, j;
-        cell_hij(G, c, h, i, j);
-        if (kind == pre && kind < 2) {
-          for (int k = 0; k < 8; k++) v[k] = fixbuf[(long)t * 8 + k];
-          g33 = (kinds[t] & 4) != 0;
-        } else {
-          repair_zone(G, P, c, kind, v);
-          long gi = (long)i * G.sn2 + j;
-          Geo q;
-          load_geo(gC, G.ng, gi, q);
-          int fail = 0;
-          g33 = fixup1zone(G.gam, floors[gi], floors[G.ng + gi], q, v, &fail);
-          if (fail) record_fail(sc, fail, h + (G.n3 > 1 ? 1 : 0), i, j);
-        }
-        for (int k = 0; k < 8; k++) P[k * G.nc + c] = v[k];
-        pflag[c] = g33 ? (signed char)-33 : (signed char)0;
+  }
+  __syncthreads();
+  // in order, one thread
+  if (tid == 0) {
+    for (int t = 0; t < n; t++) {
+      const long c = keys[t];
+      const int kind = stencil_kind(G, pflag, c);
+      int h, i, j;
+      cell_hij(G, c, h, i, j);
+      if (kind == (kinds[t] & 3) && kind < 2) {
+        for (int k = 0; k < 8; k++) P[k * G.nc + c] = fixbuf[(long)t * 8 + k];
+        pflag[c] = (kinds[t] & 4) ? (signed char)-33 : (signed char)0;
+      } else {
+        repair_in_place(G, P, pflag, geo, floors, sc, h, i, j);
       }
     }
   }
   __syncthreads();
-  if (tid == 0) {
-    sc->nfail = 0;
-    sc->fail_overflow = 0;
+}
+
+// Device scratch of repair_plane, in buffers that hold nothing between the
+// inversion and the next half step's fluxes.
+struct RepairScratch {
+  double *S;          // [8][nc] repaired zones, committed at the end
+  double *R;          // [2][nc] what the ordered pass needs of each failed zone
+  signed char *kind;  // [nc] stencil kind, or NO_REPAIR
+};
+constexpr signed char NO_REPAIR = 3;
+
+// The density and energy of the failed zones of plane h in loop order, by one
+// block, one thread per row (thread 0 the ghost row below the first).  Row i
+// works on column j = w - 2i at line w: the zones it reads in row i-1 are then
+// done, those in row i+1 still untouched.  A row hands its last result to the
+// next through shared memory; old values and the zones' kinds and floors are
+// loaded PF columns ahead.
+__device__ void repair_lines(const Grid &G, const double *P, const RepairScratch &W, int h)
+{
+  constexpr int PF = 4;
+  __shared__ double ring[2][2][512];
+  const int t = threadIdx.x, i = G.istart - 1 + t;
+  const bool row = t <= G.n1;
+  const int jl = G.jstop + 1;  // last column handed on (a ghost)
+  const double *Pr = P + RHO * G.nc, *Pu = P + UU * G.nc;
+  const long c0 = row ? cidx(G, h, i, 0) : 0;
+  // pipelines over columns: own old value at j + 1, next row's at j + 1, kind and
+  // R at j
+  double or_[PF], ou[PF], nr[PF], nu[PF], ra[PF], rb[PF];
+  signed char kd[PF];
+  auto fetch = [&](int j, double &a, double &b, double &c, double &d, double &e, double &f, signed char &k) {
+    const int jn = min(j + 1, G.sn2 - 1), jk = min(j, G.sn2 - 1);
+    a = Pr[c0 + jn];
+    b = Pu[c0 + jn];
+    c = Pr[c0 + G.sn2 + jn];
+    d = Pu[c0 + G.sn2 + jn];
+    k = t == 0 ? NO_REPAIR : W.kind[c0 + jk];
+    e = W.R[c0 + jk];
+    f = W.R[G.nc + c0 + jk];
+  };
+  // columns run from js: two ahead of the first zone, to gather the row before's values
+  const int js = G.jstart - 2;
+  if (row)
+#pragma unroll
+    for (int q = 0; q < PF; q++) fetch(js + q, or_[q], ou[q], nr[q], nu[q], ra[q], rb[q], kd[q]);
+  double pr0 = 0., pu0 = 0., pr1 = 0., pu1 = 0.;                  // row i-1 (repaired), columns j-1, j
+  double sr = 0., su = 0.;                                        // own (repaired), column j-1
+  double cr = row ? Pr[c0 + js] : 0., cu = row ? Pu[c0 + js] : 0.;  // own (old), column j
+  double n0r = 0., n0u = 0., n1r = 0., n1u = 0.;                  // row i+1 (old), columns j-1, j
+  if (row) { n1r = Pr[c0 + G.sn2 + js]; n1u = Pu[c0 + G.sn2 + js]; }
+  const int w0 = 2 * (G.istart - 1) + js, w1 = 2 * G.istop + jl;
+  int q = 0;
+  for (int w = w0; w <= w1; w++) {
+    const int j = w - 2 * i;
+    if (row && j >= js && j <= jl) {
+      const double pr2 = t > 0 ? ring[(w - 1) & 1][0][t - 1] : 0., pu2 = t > 0 ? ring[(w - 1) & 1][1][t - 1] : 0.;
+      double xr, xu, yr, yu, a, b;
+      signed char kind;
+      // the pipeline's slot of this column, refilled PF columns ahead
+#pragma unroll
+      for (int s = 0; s < PF; s++)
+        if (s == q) {
+          xr = or_[s]; xu = ou[s]; yr = nr[s]; yu = nu[s]; a = ra[s]; b = rb[s]; kind = kd[s];
+          fetch(j + PF, or_[s], ou[s], nr[s], nu[s], ra[s], rb[s], kd[s]);
+        }
+      q = q + 1 == PF ? 0 : q + 1;
+      double vr = cr, vu = cu;
+      if (j >= G.jstart && j <= G.jstop) {
+        if (kind < 2) {
+          vr = a;
+          vu = b;
+        } else if (kind == 2) {
+          // repair_zone's last resort, then fixup1zone's floors for a zone at rest
+          vr = 0.5 * (0.25 * (xr + sr + pr1 + n1r) + 0.25 * (yr + n0r + pr2 + pr0));
+          vu = 0.5 * (0.25 * (xu + su + pu1 + n1u) + 0.25 * (yu + n0u + pu2 + pu0));
+          W.S[RHO * G.nc + c0 + j] = vr;
+          W.S[UU * G.nc + c0 + j] = vu;
+          const double uf = div_rn(vu, UORHOMAX, 1. / UORHOMAX);
+          const double rf = a < uf ? uf : a;
+          if (vr < rf) vr = rf;
+          if (vu < b) vu = b;
+        }
+      }
+      ring[w & 1][0][t] = vr;
+      ring[w & 1][1][t] = vu;
+      pr0 = pr1; pu0 = pu1; pr1 = pr2; pu1 = pu2;
+      n0r = n1r; n0u = n1u; n1r = yr; n1u = yu;
+      sr = vr; su = vu;
+      cr = xr; cu = xu;
+    }
+    __syncthreads();
   }
 }
 
-// many failures: one block per phi plane, wavefronts 2i + j in order
-__global__ void __launch_bounds__(256) k_fu_wave(Grid G, double *P, signed char *pflag,
-                                                 const double *__restrict__ geo, const double *__restrict__ floors,
-                                                 DevScalars *sc)
+// Many failures: plane h by one cluster.  Within a plane zone (i, j) depends
+// only on (i-1, j-1..j+1) and (i, j-1), all on earlier lines 2i + j = const, so
+// sweeping those lines in order gives the loop order's results.  What a last
+// resort reads of its neighbours is their density and energy alone, and it
+// leaves the zone at rest, so that its floors but for u/50 follow from its field.
+// So the ordered pass (repair_lines, a line of a few additions and comparisons)
+// carries only those two, and everything else runs in parallel around it:
+// stencil repairs and floors before, the last resorts' velocities after.  All of
+// it is done on copies and committed at the end: a gamma failure changes a flag
+// that later zones' stencils read, and then the plane is repaired again the plain
+// way, one line after another.  (That plain way for every zone took 3.0 ms a half
+// step for a 256x192 torus with 49,000 failed zones; a step of an ensemble that
+// holds it went from 6.1 to 2.65 ms with this one.)
+template <class Cluster>
+__device__ void repair_plane(const Grid &G, Cluster &cl, double *P, signed char *pflag, const RepairScratch &W, int h,
+                             const double *__restrict__ geo, const double *__restrict__ floors, DevScalars *sc)
+{
+  __shared__ int again;
+  const int rank = (int)cl.block_rank(), tid = rank * blockDim.x + threadIdx.x, nt = (int)cl.num_blocks() * blockDim.x;
+  const bool lines = G.n1 + 1 <= (int)blockDim.x;  // one thread per row
+  if (threadIdx.x == 0) again = lines ? 0 : 1;
+  cl.sync();
+  int *again0 = cl.map_shared_rank(&again, 0);
+  if (lines) {
+    const long base = (long)h * G.ng;
+    int any = 0;
+    for (long g = tid; g < G.ng; g += nt) {
+      const int i = (int)(g / G.sn2), j = (int)(g % G.sn2);
+      const long c = base + g;
+      signed char kind = NO_REPAIR;
+      if (i >= G.istart && i <= G.istop && j >= G.jstart && j <= G.jstop && pflag[c] == 0) {
+        kind = (signed char)stencil_kind(G, pflag, c);
+        any = 1;
+        double v[8];
+        if (kind < 2) {
+          int fail = 0;
+          repair_zone(G, P, c, kind, v);
+          if (fix_zone(G, geo, floors, i, j, v, &fail) || fail) *again0 = 1;
+          for (int k = 0; k < 8; k++) W.S[k * G.nc + c] = v[k];
+          W.R[c] = v[RHO];
+          W.R[G.nc + c] = v[UU];
+        } else {
+          // the floors of a zone at rest with this field (fixup1zone)
+          v[RHO] = v[UU] = v[U1] = v[U2] = v[U3] = 0.;
+          for (int k = B1; k <= B3; k++) v[k] = P[k * G.nc + c];
+          Geo q;
+          load_geo(geo_at(geo, G, L_CENT), G.ng, g, q);
+          State s;
+          int fail = 0;
+          get_state(v, q, s, &fail);
+          const double bsq = dot4(s.bcon, s.bcov);
+          double rf = __ldg(floors + g), uf = __ldg(floors + G.ng + g);
+          if (rf < bsq / BSQORHOMAX) rf = bsq / BSQORHOMAX;
+          if (uf < bsq / BSQOUMAX) uf = bsq / BSQOUMAX;
+          W.R[c] = rf;
+          W.R[G.nc + c] = uf;
+        }
+      }
+      W.kind[c] = kind;
+    }
+    if (!__syncthreads_or(any) && cl.num_blocks() == 1) return;  // (3D) no failure in this plane
+    cl.sync();
+    if (rank == 0) repair_lines(G, P, W, h);
+    cl.sync();
+    for (long g = tid; g < G.ng; g += nt) {
+      const long c = base + g;
+      if (W.kind[c] != 2) continue;
+      double v[8];
+      v[RHO] = W.S[RHO * G.nc + c];
+      v[UU] = W.S[UU * G.nc + c];
+      v[U1] = v[U2] = v[U3] = 0.;
+      for (int k = B1; k <= B3; k++) v[k] = P[k * G.nc + c];
+      int fail = 0;
+      if (fix_zone(G, geo, floors, (int)(g / G.sn2), (int)(g % G.sn2), v, &fail) || fail) *again0 = 1;
+      for (int k = 0; k < 8; k++) W.S[k * G.nc + c] = v[k];
+    }
+    cl.sync();
+    if (!*again0)
+      for (long g = tid; g < G.ng; g += nt) {
+        const long c = base + g;
+        if (W.kind[c] == NO_REPAIR) continue;
+        for (int k = 0; k < 8; k++) P[k * G.nc + c] = W.S[k * G.nc + c];
+      }
+  }
+  if (*again0 && rank == 0) {
+    const int w0 = 2 * G.istart + G.jstart, w1 = 2 * G.istop + G.jstop;
+    for (int w = w0; w <= w1; w++) {
+      // i such that j = w - 2i lies in [jstart, jstop]
+      int ilo = (w - G.jstop + 1) / 2, ihi = (w - G.jstart) / 2;
+      if (ilo < G.istart) ilo = G.istart;
+      if (ihi > G.istop) ihi = G.istop;
+      for (int i = ilo + (int)threadIdx.x; i <= ihi; i += blockDim.x)
+        if (pflag[cidx(G, h, i, w - 2 * i)] == 0) repair_in_place(G, P, pflag, geo, floors, sc, h, i, w - 2 * i);
+      __syncthreads();
+    }
+  }
+  cl.sync();  // no block leaves while another may read its shared memory
+}
+
+__global__ void __launch_bounds__(512) k_repair(Grid G, double *P, signed char *pflag, const int *list, double *fixbuf,
+                                                RepairScratch W, const double *__restrict__ geo,
+                                                const double *__restrict__ floors, DevScalars *sc, int slot)
 {
   if (sc->halted) return;
-  const int n = sc->nfail;
-  if (n == 0) return;  // none, or k_fu_fix has repaired them
-  const int h = blockIdx.x;
-  const double *gC = geo_at(geo, G, L_CENT);
-  const int w0 = 2 * G.istart + G.jstart, w1 = 2 * G.istop + G.jstop;
-  for (int w = w0; w <= w1; w++) {
-    // i such that j = w - 2i lies in [jstart, jstop]
-    int ilo = (w - G.jstop + 1) / 2, ihi = (w - G.jstart) / 2;
-    if (ilo < G.istart) ilo = G.istart;
-    if (ihi > G.istop) ihi = G.istop;
-    for (int i = ilo + (int)threadIdx.x; i <= ihi; i += blockDim.x) {
-      const int j = w - 2 * i;
-      const long c = cidx(G, h, i, j);
-      if (pflag[c] != 0) continue;
-      double v[8];
-      repair_zone(G, P, c, stencil_kind(G, pflag, c), v);
-      const long gi = (long)i * G.sn2 + j;
-      Geo q;
-      load_geo(gC, G.ng, gi, q);
-      int fail = 0;
-      bool g33 = fixup1zone(G.gam, floors[gi], floors[G.ng + gi], q, v, &fail);
-      if (fail) record_fail(sc, fail, h + (G.n3 > 1 ? 1 : 0), i, j);
-      for (int k = 0; k < 8; k++) P[k * G.nc + c] = v[k];
-      pflag[c] = g33 ? (signed char)-33 : (signed char)0;
-    }
-    __syncthreads();
-  }
-  // the last block to finish clears the counters for the next call
-  __shared__ bool last;
-  __threadfence();
-  if (threadIdx.x == 0) last = atomicAdd(&sc->wave_done, 1) == (int)gridDim.x - 1;
-  __syncthreads();
-  if (last && threadIdx.x == 0) {
-    sc->wave_done = 0;
-    sc->nfail = 0;
-    sc->fail_overflow = 0;
+  const int n = sc->nfail[slot];
+  if (n == 0) return;
+  auto cl = cooperative_groups::this_cluster();
+  if (n <= FIX_LIST_MAX) {
+    if (blockIdx.x == 0) repair_list(G, P, pflag, list, n, fixbuf, geo, floors, sc);
+  } else {
+    repair_plane(G, cl, P, pflag, W, (int)(blockIdx.x / cl.num_blocks()), geo, floors, sc);
   }
 }
 
@@ -514,14 +658,28 @@ int launch_bound(Ctx *x, double *P)
   return HARM_OK;
 }
 
-int launch_fixup_utoprim(Ctx *x, double *P, int *nfail_out)
+// slot: 0 the predictor's, 1 the corrector's; its count of failed zones is zero on entry
+int launch_fixup_utoprim(Ctx *x, double *P, int slot, int *nfail_out)
 {
   const Grid &G = x->G;
-  k_fu_flip<<<148 * 8, 256, 0, x->stream>>>(G, x->pflag, x->fail_list, x->sc);
-  // the number of failed zones, kept for the discrete adjoint before the repair clears it
-  if (nfail_out) CK(cudaMemcpyAsync(nfail_out, &x->sc->nfail, sizeof(int), cudaMemcpyDeviceToDevice, x->stream));
-  k_fu_fix<<<1, NTHR_FIX, 0, x->stream>>>(G, P, x->pflag, x->fail_list, x->fix_buf, x->geo, x->floors, x->sc);
-  k_fu_wave<<<G.n3, 256, 0, x->stream>>>(G, P, x->pflag, x->geo, x->floors, x->sc);
+  k_fu_flip<<<148 * 8, 256, 0, x->stream>>>(G, x->pflag, x->fail_list, x->sc, slot);
+  // the number of failed zones, kept for the discrete adjoint
+  if (nfail_out) CK(cudaMemcpyAsync(nfail_out, &x->sc->nfail[slot], sizeof(int), cudaMemcpyDeviceToDevice, x->stream));
+  const RepairScratch W{x->Ubuf, x->emf, (signed char *)(x->emf + 2 * G.nc)};
+  // the one plane of a 2D grid gets a cluster of eight blocks for its parallel
+  // passes; the planes of a 3D grid, one block each, fill the GPU between them
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = G.n3 > 1 ? 1 : 8;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.gridDim = dim3(at.val.clusterDim.x * G.n3);
+  cfg.blockDim = dim3(512);
+  cfg.stream = x->stream;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  CK(cudaLaunchKernelEx(&cfg, k_repair, G, P, x->pflag, (const int *)x->fail_list, x->fix_buf, W,
+                        (const double *)x->geo, (const double *)x->floors, x->sc, slot));
   return HARM_OK;
 }
 
@@ -927,7 +1085,9 @@ static int on_host_array(harm_ctx *h, double *pv, int which)
   } else if (which == 1) {
     launch_bound(x, x->ph);
   } else {
-    launch_fixup_utoprim(x, x->ph);
+    CK(cudaMemsetAsync(&x->sc->nfail[0], 0, sizeof(int), x->stream));
+    rc = launch_fixup_utoprim(x, x->ph, 0);
+    if (rc) return rc;
   }
   CK(cudaGetLastError());
   return get_prims(x, x->ph, pv, nullptr);

@@ -24,8 +24,7 @@ struct DevScalars {
   int fail_code, fail_h, fail_i, fail_j;
   int err;                         // HARM_E_DT when dt < 1e-9
   int halted;                      // set after a failure: later steps do nothing
-  int nfail, fail_overflow;        // failed zones met by the current fixup_utoprim
-  int wave_done;                   // blocks of k_fu_wave finished (reset by the last)
+  int nfail[2];                    // failed zones of the predictor's and the corrector's fixup_utoprim
   unsigned long long divb_bits;    // diagnostics: bits of max |div B| (a positive double)
   long long divb_loc;              // and its first zone in loop order
 };
@@ -52,8 +51,7 @@ struct TrParams {
 };
 
 constexpr int FAIL_CAP = 8192;     // failed zones listed by k_fu_flip
-constexpr int FIX_LIST_MAX = 512;  // up to this many, repaired through the sorted list
-constexpr int NTHR_FIX = 1024;
+constexpr int FIX_LIST_MAX = 32;   // up to this many, repaired through the sorted list
 
 struct Ctx {
   Grid G;
@@ -182,7 +180,7 @@ struct StepRec {
 // kernels shared by both precisions (harm_api.cu)
 int launch_bound(Ctx *x, double *P);
 int get_prims(Ctx *x, const double *src, double *p, signed char *pflag);  // device planes -> host layout
-int launch_fixup_utoprim(Ctx *x, double *P, int *nfail_out = nullptr);
+int launch_fixup_utoprim(Ctx *x, double *P, int slot, int *nfail_out = nullptr);
 void launch_mass(Ctx *x);
 int sync_status(Ctx *x);
 

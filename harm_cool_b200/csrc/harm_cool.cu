@@ -246,6 +246,7 @@ __global__ void __launch_bounds__(128, HARM_COOL_CONS_MINB) k_cons_cool(Grid G, 
   const int j = G.jstart + blockIdx.x * blockDim.x + threadIdx.x;
   const int i = G.istart + blockIdx.y * blockDim.y + threadIdx.y;
   const int h = blockIdx.z;
+  if (h == 0 && i == G.istart && j == G.jstart) sc->nfail[FULL ? 1 : 0] = 0;  // for this half step's repairs
   if (i > G.istop || j > G.jstop) return;
   const double Dt = FULL ? sc->dt : 0.5 * sc->dt;
   const long c = cidx(G, h, i, j);
@@ -357,7 +358,7 @@ void launch_half(Ctx *x, const double *pi, const double *pb, double *pf, bool ro
                                             x->sc);
   if (FULL) k_diag_flux<<<1, 1024, 0, x->stream>>>(G, x->F1, x->sc);
   launch_bound(x, pf);
-  launch_fixup_utoprim(x, pf);
+  launch_fixup_utoprim(x, pf, FULL ? 1 : 0);
   launch_bound(x, pf);
 }
 
@@ -530,7 +531,7 @@ int cool_time_kernels(Ctx *x, int reps, double *ms)
       }
       launch_bound(x, pf);
       slot[e] = 2; CK(cudaEventRecord(ev[e++], x->stream));
-      launch_fixup_utoprim(x, pf);
+      launch_fixup_utoprim(x, pf, half);
       slot[e] = 3; CK(cudaEventRecord(ev[e++], x->stream));
       launch_bound(x, pf);
       slot[e] = 2; CK(cudaEventRecord(ev[e++], x->stream));

@@ -244,6 +244,7 @@ __global__ void __launch_bounds__(2 * FLUX_FACES, HARM_FLUX_MINB) k_flux(Grid G,
 {
   if (sc->halted) return;
   __shared__ FluxShared S;
+  if (blockIdx.x == 0 && threadIdx.x == 0) sc->nfail[FULL ? 1 : 0] = 0;  // for this half step's repairs
   int b = blockIdx.x, dir;
   double dtmin;
   if (b < nb.b1 * G.n3) {
@@ -738,7 +739,7 @@ void launch_half(Ctx *x, const double *pi, const double *pb, double *pf)
   launch_update<FULL>(x, pi, pb, pf);
   if (FULL) k_diag_flux<<<1, 1024, 0, x->stream>>>(x->G, B.F1, x->sc);
   launch_bound(x, pf);
-  launch_fixup_utoprim(x, pf);
+  launch_fixup_utoprim(x, pf, FULL ? 1 : 0);
   launch_bound(x, pf);
 }
 
@@ -770,7 +771,7 @@ static void launch_half_rec(Ctx *x, const double *pi, const double *pb, double *
   launch_bound(x, pf);
   cudaMemcpyAsync(r.X1[s], pf, 8 * nc * sizeof(double), cudaMemcpyDeviceToDevice, x->stream);
   cudaMemcpyAsync(r.fl1[s], x->pflag, nc, cudaMemcpyDeviceToDevice, x->stream);
-  launch_fixup_utoprim(x, pf, r.nfail[s]);
+  launch_fixup_utoprim(x, pf, s, r.nfail[s]);
   launch_bound(x, pf);
 }
 
@@ -818,7 +819,7 @@ int time_kernels(Ctx *x, int reps, double *ms)
       }
       launch_bound(x, pf);
       slot[e] = 2; CK(cudaEventRecord(ev[e++], x->stream));
-      launch_fixup_utoprim(x, pf);
+      launch_fixup_utoprim(x, pf, half);
       slot[e] = 3; CK(cudaEventRecord(ev[e++], x->stream));
       launch_bound(x, pf);
       slot[e] = 2; CK(cudaEventRecord(ev[e++], x->stream));

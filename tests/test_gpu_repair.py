@@ -1,0 +1,81 @@
+"""fixup_utoprim's repair paths at their edges, bit for bit against the oracle: one
+failure, the longest list, one more (the plane repair), every zone; rows that
+fill the ordered pass's block and one row too many for it; several phi planes, one
+of them without failures; and gamma failures, which change the flags that later
+zones' stencils read."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from helpers import active, make_oracle
+
+pytestmark = pytest.mark.gpu
+LIST = 32  # FIX_LIST_MAX
+
+
+@pytest.fixture(scope="module")
+def hc(harm_lib):
+    import harm_cool_b200
+    return harm_cool_b200
+
+
+def repair_both(hc, pr, fail, expect_marks=False):
+    """fixup_utoprim on the same state and flags by the device and by the oracle."""
+    from oracle.pyoracle import oracle_lib
+    dp = ctypes.POINTER(ctypes.c_double)
+    ctx = hc.Context(pr)
+    rng = np.random.default_rng(3)
+    p = np.zeros(pr.shape + (8,))
+    p[..., 0] = 10. ** rng.uniform(-6, 0, pr.shape)
+    p[..., 1] = p[..., 0] * 10. ** rng.uniform(-4, -1, pr.shape)
+    p[..., 2:5] = rng.uniform(-.05, .05, pr.shape + (3,))
+    p[..., 5:8] = 1e-3 * rng.standard_normal(pr.shape + (3,))
+    fl = np.zeros(pr.shape, dtype=np.int8)
+    active(pr, fl)[:, 2:-2, 2:-2] = fail
+    ctx.put_prims(p, fl)
+    a, b = p.copy(), p.copy()
+    o = make_oracle(pr)
+    o.pflag[...] = fl
+    ctx.lib.harm_fixup_utoprim(ctx.h, a.ctypes.data_as(dp))
+    oracle_lib().ora_fixup_utoprim(o.h, b.ctypes.data_as(dp))
+    np.testing.assert_array_equal(active(pr, a)[:, 2:-2, 2:-2], active(pr, b)[:, 2:-2, 2:-2])
+    _, fg = ctx.get_prims(with_flags=True)
+    np.testing.assert_array_equal(active(pr, fg)[:, 2:-2, 2:-2], active(pr, o.pflag)[:, 2:-2, 2:-2])
+    assert (active(pr, fg) == -33).any() == expect_marks
+    ctx.close()
+
+
+def flags(shape, count, seed=1):
+    n1, n2, n3 = shape
+    f = np.zeros(n1 * n2 * n3, dtype=np.int8)
+    f[np.random.default_rng(seed).permutation(f.size)[:count]] = 101
+    return f.reshape(n3, n1, n2)
+
+
+@pytest.mark.parametrize("shape,count", [((20, 24, 1), 1), ((20, 24, 1), LIST), ((20, 24, 1), LIST + 1),
+                                         ((20, 24, 1), 250), ((20, 24, 1), 480), ((7, 9, 1), 63), ((5, 300, 1), 1200),
+                                         ((511, 8, 1), 3000), ((512, 8, 1), 3000), ((12, 10, 4), LIST),
+                                         ((12, 10, 4), LIST + 1), ((12, 10, 4), 480)])
+def test_repairs_match_oracle(shape, count, hc, oracle_built):
+    repair_both(hc, hc.torus_problem(*shape), flags(shape, count))
+
+
+def test_planes_without_failures_stay(hc, oracle_built):
+    f = flags((16, 12, 6), 0)
+    f[1, 3:9, 2:11] = 1
+    f[4] = 2
+    repair_both(hc, hc.torus_problem(16, 12, 6), f)
+
+
+@pytest.mark.parametrize("shape", [(20, 24, 1), (12, 10, 4)])
+def test_gamma_failures_repair_in_loop_order(shape, hc, oracle_built):
+    """A metric whose theta entry is negative in some zones makes their floors
+    fail in gamma, wherever the repair leaves a theta velocity (stencil averages)."""
+    pr = hc.torus_problem(*shape)
+    rng = np.random.default_rng(8)
+    sick = rng.random((shape[0] + 4, shape[1] + 4)) < 0.3
+    g = pr.geometry["gcov"]
+    g[sick, 3, 2, 2] *= -1e4
+    f = flags(shape, shape[0] * shape[1] * shape[2] // 4, seed=5)
+    repair_both(hc, pr, f, expect_marks=True)
