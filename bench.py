@@ -32,12 +32,17 @@ sys.path.insert(0, ROOT)
 
 
 
-def kernels_per_step(n3):
-    """Kernel launches of one step: per half step the flux kernel, the corner EMFs,
-    the conserved update and the inversion, bound_prim, the flag flip, the
-    repair, bound_prim; the corrector adds the flux
-    diagnostics; then the mass diagnostics and the dt update."""
-    return 2 * (1 + 7) + 1 + 2
+def kernels_per_step(n3, cool=False):
+    """Kernel launches of one step.  Per half step: the flux kernel, the corner EMFs,
+    the conserved update, the inversion, bound_prim, the repair and bound_prim in
+    3D; in 2D the flux kernel, the update (one launch) and the repair, and with
+    COOL_EOS a flux kernel per direction and the update in two launches.  Then the
+    sums with the dt update, and with COOL_EOS the tracers."""
+    if cool:
+        return 2 * 5 + 2
+    return 2 * (7 if n3 > 1 else 3) + 1
+
+
 METRIC = "zone-cycles/s 288x256x256 GRMHD step_ch: FP64, mixed precision beside it"
 STATE_BYTES_PER_ZONE_CYCLE = 320  # p read twice, ph written and read, p written; 8 FP64 prims
 
@@ -653,7 +658,7 @@ def run_cool(args):
                     "steps": args.e2e_steps,
                     "path": "harm_run_host: per step upload, step, download, each upload overlapped with the "
                             "previous step's download"},
-            "gpu_launches": kernels_per_step(1) * args.steps,
+            "gpu_launches": kernels_per_step(1, cool=True) * args.steps,
             "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": None, "algorithmic_bytes": alg,
                          "peak_source": peak_kind,

@@ -63,7 +63,7 @@ struct AdjScalars {
 
 // before step n's reverse (run by k_adj_din_bound): dt^{n+1} = min(ndt, 1.3 dt^n),
 // ndt = defcon / (1/n1 + 1/n2) (step_ch.c:126-137); sa is the run state before
-// k_finalize, sb after
+// k_mass, sb after
 __device__ __forceinline__ void adj_dt_pre(const DevScalars *sa, const DevScalars *sb, double defcon, AdjScalars *a)
 {
   const double dt = sa->dt, ndt = sb->ndt;
@@ -190,7 +190,7 @@ __global__ void k_adj_din_bound(Grid G, const double *__restrict__ P, const doub
 
 // ---------------------------------------------------------------------------
 // fixup_utoprim (fixup.c:432-538) transposed.  One block: the failed zones of
-// the half step (pflag != 0 after the first bound_prim) are listed in loop
+// the half step (flag 0 after the first bound_prim) are listed in loop
 // order, the repairs are replayed on a working copy exactly as the step made
 // them (each stencil chosen from the flags as earlier repairs left them), and
 // then undone in reverse order, so a last-resort average that read an earlier
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(FU_THREADS) k_adj_fixup_bound(Grid G, const do
   int m = 0;
   for (long t = a0; t < a1; t++) {
     const int i = G.istart + (int)(t / G.n2), j = G.jstart + (int)(t % G.n2);
-    if (fl1[cidx(G, 0, i, j)] != 0) m++;
+    if (fl1[cidx(G, 0, i, j)] == 0) m++;
   }
   cnt[tid] = m;
   __syncthreads();
@@ -244,12 +244,12 @@ __global__ void __launch_bounds__(FU_THREADS) k_adj_fixup_bound(Grid G, const do
   for (long t = a0; t < a1; t++) {
     const int i = G.istart + (int)(t / G.n2), j = G.jstart + (int)(t % G.n2);
     const long c = cidx(G, 0, i, j);
-    if (fl1[c] != 0) list[o++] = (int)c;
+    if (fl1[c] == 0) list[o++] = (int)c;
   }
   for (long c = tid; c < G.nc; c += FU_THREADS) {
 #pragma unroll
     for (int k = 0; k < 8; k++) W[k * G.nc + c] = X1[k * G.nc + c];
-    Wf[c] = (signed char)(!fl1[c]);  // k_fu_flip
+    Wf[c] = fl1[c];
   }
   __syncthreads();
   if (tid == 0) {

@@ -14,10 +14,11 @@
 // connection planes and two floor planes.
 //
 // One step (step_ch.c:90-140) is, on one stream and without host sync:
-//   predictor : k_flux, k_emf, k_cons, k_invert (dt/2) [flux-CT, source,
-//               inversion, floors], k_bound, k_fu_flip, k_repair, k_bound
-//   corrector : the same with dt and the Courant minima, and k_diag_flux
-//   k_diag_mass, k_finalize (diagnostic sums, next dt)
+//   predictor : k_flux, then k_update or k_emf, k_cons, k_invert (dt/2) [flux-CT,
+//               source, inversion, floors, flags; in 2D the ghosts too],
+//               (3D) k_bound, k_repair, (3D) k_bound
+//   corrector : the same with dt and the Courant minima
+//   k_mass (diagnostic sums, next dt)
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -43,15 +44,10 @@ namespace harm {
 // radial ghosts finally get inflow_check().
 
 template <bool THREE_D>
-__global__ void k_bound(Grid G, double *P, signed char *pflag, const double *__restrict__ geo, DevScalars *sc)
+__device__ void bound_one(const Grid &G, double *P, signed char *pflag, const double *__restrict__ geo,
+                          DevScalars *sc, int h, int t)
 {
-  if (sc->halted) return;
-  const int nrow = THREE_D ? 8 : 4;
-  const int ncell = 4 * G.sn2 + nrow * (G.sn1 - 4);
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int h = blockIdx.y;
-  if (t >= ncell) return;
-  BoundCell b = bound_cell(G, t, nrow);
+  BoundCell b = bound_cell(G, t, THREE_D ? 8 : 4);
   const int i = b.i, j = b.j;
   double v[8];
   signed char fl;
@@ -89,6 +85,22 @@ __global__ void k_bound(Grid G, double *P, signed char *pflag, const double *__r
   pflag[c] = fl;
 }
 
+template <bool THREE_D>
+__host__ __device__ __forceinline__ int bound_cells(const Grid &G)
+{
+  return 4 * G.sn2 + (THREE_D ? 8 : 4) * (G.sn1 - 4);
+}
+
+// slot >= 0: the bound_prim after fixup_utoprim, which only repeats the one before
+// it when that slot's count of failed zones is zero
+template <bool THREE_D>
+__global__ void k_bound(Grid G, double *P, signed char *pflag, const double *__restrict__ geo, DevScalars *sc, int slot)
+{
+  if (sc->halted || (slot >= 0 && sc->nfail[slot] == 0)) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < bound_cells<THREE_D>(G)) bound_one<THREE_D>(G, P, pflag, geo, sc, blockIdx.y, t);
+}
+
 // ---------------------------------------------------------------------------
 // fixup_utoprim() (fixup.c:432-538)
 //
@@ -96,7 +108,8 @@ __global__ void k_bound(Grid G, double *P, signed char *pflag, const double *__r
 // then repairs failed zones in loop order, in place.  Repairs from the edge
 // or corner stencils read only good zones, which the repair never changes;
 // the last-resort average reads every neighbour and so sees earlier repairs.
-// k_fu_flip flips the flags and lists the failed zones; k_repair repairs them.
+// A half step's inversion writes the flags flipped and lists the failed zones
+// (k_fu_flip does both for flags that come from the host); k_repair repairs them.
 // For a few failures (up to FIX_LIST_MAX, about 2 us each in the worst case, against
 // some 100 us for a plane) one block sorts the list into loop order, precomputes the
 // stencil repairs in parallel and then replays the whole list in order on one
@@ -114,10 +127,7 @@ __global__ void k_fu_flip(Grid G, signed char *pflag, int *list, DevScalars *sc,
     pflag[c] = nf;
     if (nf == 0) {
       int j = (int)(c % G.sn2), i = (int)((c / G.sn2) % G.sn1);
-      if (i >= G.istart && i <= G.istop && j >= G.jstart && j <= G.jstop) {
-        int k = atomicAdd(&sc->nfail[slot], 1);
-        if (k < FAIL_CAP) list[k] = (int)c;
-      }
+      if (i >= G.istart && i <= G.istop && j >= G.jstart && j <= G.jstop) list_failed(sc, slot, list, c);
     }
   }
 }
@@ -395,7 +405,8 @@ __device__ void repair_plane(const Grid &G, Cluster &cl, double *P, signed char 
 
 __global__ void __launch_bounds__(512) k_repair(Grid G, double *P, signed char *pflag, const int *list, double *fixbuf,
                                                 RepairScratch W, const double *__restrict__ geo,
-                                                const double *__restrict__ floors, DevScalars *sc, int slot)
+                                                const double *__restrict__ floors, DevScalars *sc, int slot,
+                                                bool rebound)
 {
   if (sc->halted) return;
   const int n = sc->nfail[slot];
@@ -406,19 +417,58 @@ __global__ void __launch_bounds__(512) k_repair(Grid G, double *P, signed char *
   } else {
     repair_plane(G, cl, P, pflag, W, (int)(blockIdx.x / cl.num_blocks()), geo, floors, sc);
   }
+  if (rebound) {  // 2D: the one cluster makes the ghost cells again
+    cl.sync();
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < bound_cells<false>(G); t += gridDim.x * blockDim.x)
+      bound_one<false>(G, P, pflag, geo, sc, 0, t);
+  }
 }
 
 // ---------------------------------------------------------------------------
-// diag_mass() (diag.c:477-580, MDOTTYPE NEU_AGA_GHOST1) partial sums
+// diag_flux() (diag.c:437-465), diag_mass() (diag.c:477-580, MDOTTYPE
+// NEU_AGA_GHOST1) and the next time step (step_ch.c:119-137) in one launch
 
-__global__ void __launch_bounds__(256) k_diag_mass(Grid G, const double *__restrict__ P, const double *__restrict__ geo,
-                                                   double *partials, int nparts, DevScalars *sc)
+constexpr int MASS_THREADS = 256, MASS_PARTS = 148 * 4;
+constexpr int SUM_WARPS = 32;  // the sums add 1024 strided values, warp by warp
+
+constexpr int FLUX_BLOCKS = SUM_WARPS * 32 / MASS_THREADS;
+
+// diag_flux(): sums over the inner radial face, after the mass-flux fix, in the
+// order of 1024 threads' strided sums; block b of FLUX_BLOCKS takes its warps' share
+template <class T>
+__device__ void flux_sums(const Grid &G, const T *__restrict__ F1, double *sums, int b)
 {
-  if (sc->halted) return;
+  const long n = (long)G.n3 * G.n2;
+  const int t0 = b * MASS_THREADS + threadIdx.x;
+  double m = 0., e = 0., l = 0.;
+#pragma unroll 4
+  for (long t = t0; t < n; t += 32 * SUM_WARPS) {
+    int h = (int)(t / G.n2), j = G.jstart + (int)(t % G.n2);
+    long c = cidx(G, h, G.istart, j);
+    double fr = (double)__ldg(F1 + RHO * G.nc + c);
+    if (fr > 0) fr = 0;
+    m += fr * G.dx2 * G.dx3;
+    e += ((double)__ldg(F1 + UU * G.nc + c) - fr) * G.dx2 * G.dx3;
+    l += (double)__ldg(F1 + U3 * G.nc + c) * G.dx2 * G.dx3;
+  }
+  m = warp_sum(m);
+  e = warp_sum(e);
+  l = warp_sum(l);
+  if ((t0 & 31) == 0) {
+    sums[t0 >> 5] = m;
+    sums[SUM_WARPS + (t0 >> 5)] = e;
+    sums[2 * SUM_WARPS + (t0 >> 5)] = l;
+  }
+}
+
+// diag_mass() partial sums of block b of nb
+static __device__ void mass_partial(const Grid &G, const double *P, const double *__restrict__ geo, double *partials,
+                                    int blk, int nb, DevScalars *sc)
+{
   const double *gC = geo_at(geo, G, L_CENT);
   double m = 0., din = 0., dout = 0.;
   const long nact = (long)G.n3 * G.n1 * G.n2;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < nact; t += (long)gridDim.x * blockDim.x) {
+  for (long t = blk * (long)blockDim.x + threadIdx.x; t < nact; t += (long)nb * blockDim.x) {
     int j = G.jstart + (int)(t % G.n2);
     int i = G.istart + (int)((t / G.n2) % G.n1);
     int h = (int)(t / ((long)G.n2 * G.n1));
@@ -426,7 +476,7 @@ __global__ void __launch_bounds__(256) k_diag_mass(Grid G, const double *__restr
     m += P[RHO * G.nc + cidx(G, h, i, j)] * __ldg(gC + 17 * G.ng + gi) * G.dx1 * G.dx2 * G.dx3;
   }
   const long nrad = (long)G.n3 * G.n2;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < 2 * nrad; t += (long)gridDim.x * blockDim.x) {
+  for (long t = blk * (long)blockDim.x + threadIdx.x; t < 2 * nrad; t += (long)nb * blockDim.x) {
     bool inner = t < nrad;
     long u = inner ? t : t - nrad;
     int j = G.jstart + (int)(u % G.n2), h = (int)(u / G.n2);
@@ -453,32 +503,41 @@ __global__ void __launch_bounds__(256) k_diag_mass(Grid G, const double *__restr
   __syncthreads();
   if (threadIdx.x == 0) {
     double a = 0., b = 0., d = 0.;
-    for (int k = 0; k < (int)(blockDim.x >> 5); k++) { a += red[0][k]; b += red[1][k]; d += red[2][k]; }
-    partials[blockIdx.x] = a;
-    partials[nparts + blockIdx.x] = b;
-    partials[2 * nparts + blockIdx.x] = d;
+    for (int k = 0; k < MASS_THREADS / 32; k++) { a += red[0][k]; b += red[1][k]; d += red[2][k]; }
+    partials[blk] = a;
+    partials[MASS_PARTS + blk] = b;
+    partials[2 * MASS_PARTS + blk] = d;
   }
 }
 
-// sums of the partials, mass counters, and the next time step (step_ch.c:119-137)
-__global__ void k_finalize(Grid G, const double *partials, int nparts, DevScalars *sc)
+// sums of the nb partials, mass counters, and the next time step (step_ch.c:119-137)
+static __device__ void finalize(const Grid &G, const double *partials, int nb, DevScalars *sc)
 {
-  if (sc->halted) return;
-  __shared__ double red[3][32];
-  double a = 0., b = 0., d = 0.;
-  for (int t = threadIdx.x; t < nparts; t += blockDim.x) {
-    a += partials[t];
-    b += partials[nparts + t];
-    d += partials[2 * nparts + t];
+  __shared__ double red[3][SUM_WARPS];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double a, b, d;
+  for (int vw = w; vw < SUM_WARPS; vw += MASS_THREADS / 32) {
+    const int t = vw * 32 + lane;
+    a = warp_sum(t < nb ? __ldcg(partials + t) : 0.);
+    b = warp_sum(t < nb ? __ldcg(partials + MASS_PARTS + t) : 0.);
+    d = warp_sum(t < nb ? __ldcg(partials + 2 * MASS_PARTS + t) : 0.);
+    if (lane == 0) { red[0][vw] = a; red[1][vw] = b; red[2][vw] = d; }
   }
-  a = warp_sum(a);
-  b = warp_sum(b);
-  d = warp_sum(d);
-  if ((threadIdx.x & 31) == 0) { red[0][threadIdx.x >> 5] = a; red[1][threadIdx.x >> 5] = b; red[2][threadIdx.x >> 5] = d; }
+  if (w == 0) {
+    const double *sums = partials + 3 * MASS_PARTS;
+    a = warp_sum(__ldcg(sums + lane));
+    b = warp_sum(__ldcg(sums + SUM_WARPS + lane));
+    d = warp_sum(__ldcg(sums + 2 * SUM_WARPS + lane));
+    if (lane == 0) {
+      sc->mdot = a;
+      sc->edot = -b;
+      sc->ldot = d;
+    }
+  }
   __syncthreads();
   if (threadIdx.x != 0) return;
   a = b = d = 0.;
-  for (int k = 0; k < (int)(blockDim.x >> 5); k++) { a += red[0][k]; b += red[1][k]; d += red[2][k]; }
+  for (int k = 0; k < SUM_WARPS; k++) { a += red[0][k]; b += red[1][k]; d += red[2][k]; }
   double dt = sc->dt;
   sc->mass_curr = a;
   sc->mdot_in = b;
@@ -504,6 +563,27 @@ __global__ void k_finalize(Grid G, const double *partials, int nparts, DevScalar
   sc->t = t;
   sc->dt = dt;
   if (sc->fail_code) sc->halted = 1;
+}
+
+// the first FLUX_BLOCKS blocks the flux sums, nb more the mass partial sums; the
+// last block to finish adds them up and sets the next step
+template <class T>
+__global__ void __launch_bounds__(MASS_THREADS) k_mass(Grid G, const double *__restrict__ P, const T *__restrict__ F1,
+                                                       const double *__restrict__ geo, double *partials, int nb,
+                                                       DevScalars *sc)
+{
+  if (sc->halted) return;
+  if (blockIdx.x < FLUX_BLOCKS) flux_sums(G, F1, partials + 3 * MASS_PARTS, blockIdx.x);
+  else mass_partial(G, P, geo, partials, blockIdx.x - FLUX_BLOCKS, nb, sc);
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&sc->ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (threadIdx.x == 0) sc->ticket = 0;
+  finalize(G, partials, nb, sc);
 }
 
 // ---------------------------------------------------------------------------
@@ -647,24 +727,26 @@ int fail_with(int code, const std::string &msg)
   return code;
 }
 
-int launch_bound(Ctx *x, double *P)
+static void launch_bound_slot(Ctx *x, double *P, int slot)
 {
   const Grid &G = x->G;
-  const int nrow = G.n3 > 1 ? 8 : 4;
-  const int ncell = 4 * G.sn2 + nrow * (G.sn1 - 4);
-  dim3 grid((ncell + 127) / 128, G.n3);
-  if (G.n3 > 1) k_bound<true><<<grid, 128, 0, x->stream>>>(G, P, x->pflag, x->geo, x->sc);
-  else k_bound<false><<<grid, 128, 0, x->stream>>>(G, P, x->pflag, x->geo, x->sc);
+  if (G.n3 > 1)
+    k_bound<true><<<dim3((bound_cells<true>(G) + 127) / 128, G.n3), 128, 0, x->stream>>>(G, P, x->pflag, x->geo, x->sc,
+                                                                                       slot);
+  else
+    k_bound<false><<<(bound_cells<false>(G) + 127) / 128, 128, 0, x->stream>>>(G, P, x->pflag, x->geo, x->sc, slot);
+}
+
+int launch_bound(Ctx *x, double *P)
+{
+  launch_bound_slot(x, P, -1);
   return HARM_OK;
 }
 
-// slot: 0 the predictor's, 1 the corrector's; its count of failed zones is zero on entry
-int launch_fixup_utoprim(Ctx *x, double *P, int slot, int *nfail_out)
+// fixup_utoprim()'s repairs; rebound: and the bound_prim() after it
+static int launch_repairs(Ctx *x, double *P, int slot, bool rebound)
 {
   const Grid &G = x->G;
-  k_fu_flip<<<148 * 8, 256, 0, x->stream>>>(G, x->pflag, x->fail_list, x->sc, slot);
-  // the number of failed zones, kept for the discrete adjoint
-  if (nfail_out) CK(cudaMemcpyAsync(nfail_out, &x->sc->nfail[slot], sizeof(int), cudaMemcpyDeviceToDevice, x->stream));
   const RepairScratch W{x->Ubuf, x->emf, (signed char *)(x->emf + 2 * G.nc)};
   // the one plane of a 2D grid gets a cluster of eight blocks for its parallel
   // passes; the planes of a 3D grid, one block each, fill the GPU between them
@@ -679,17 +761,28 @@ int launch_fixup_utoprim(Ctx *x, double *P, int slot, int *nfail_out)
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   CK(cudaLaunchKernelEx(&cfg, k_repair, G, P, x->pflag, (const int *)x->fail_list, x->fix_buf, W,
-                        (const double *)x->geo, (const double *)x->floors, x->sc, slot));
+                        (const double *)x->geo, (const double *)x->floors, x->sc, slot, rebound && G.n3 == 1));
+  if (rebound && G.n3 > 1) launch_bound_slot(x, P, slot);
   return HARM_OK;
 }
 
-// diag_mass(), update_tracers() and the next dt (step_ch.c:119-137)
-void launch_mass(Ctx *x)
+int launch_repair(Ctx *x, double *P, int slot) { return launch_repairs(x, P, slot, true); }
+
+// diag_flux(), diag_mass(), update_tracers() and the next dt (step_ch.c:119-137);
+// the tracers move before the sums, which do not read them, and before the dt update
+template <class T>
+static void launch_mass_t(Ctx *x, const T *F1)
 {
-  k_diag_mass<<<x->nparts, 256, 0, x->stream>>>(x->G, x->p, x->geo, x->partials, x->nparts, x->sc);
+  const Grid &G = x->G;
   if (x->ntr) launch_tracers(x);
-  k_finalize<<<1, 1024, 0, x->stream>>>(x->G, x->partials, x->nparts, x->sc);
+  // a zone per thread up to MASS_PARTS blocks: the same partial sums as that many
+  // blocks would make, of which the rest hold zeros
+  const long n = (long)G.n3 * G.n2 * (G.n1 > 2 ? G.n1 : 2), blocks = (n + MASS_THREADS - 1) / MASS_THREADS;
+  const int nb = (int)(blocks < MASS_PARTS ? blocks : MASS_PARTS);
+  k_mass<T><<<FLUX_BLOCKS + nb, MASS_THREADS, 0, x->stream>>>(G, x->p, F1, x->geo, x->partials, nb, x->sc);
 }
+void launch_mass(Ctx *x, const double *F1) { launch_mass_t(x, F1); }
+void launch_mass(Ctx *x, const float *F1) { launch_mass_t(x, F1); }
 
 void invalidate_graph(Ctx *x)
 {
@@ -780,7 +873,7 @@ extern "C" int harm_create(const harm_params *prm, const double *gcov, const dou
     for (int i = G.istart; i <= G.istop; i++)
       if (coords[((long)i * d.sn2 + G.jstart) * 4 + 1] >= 2. * rH) { G.isrc32 = i; break; }
   }
-  x->nparts = 148 * 4;
+  x->nparts = MASS_PARTS;
   x->tbx = 32;
   x->tby = 4;
   auto al = [&](void **p, size_t b) -> int { CK(cudaMalloc(p, b)); return HARM_OK; };
@@ -800,7 +893,7 @@ extern "C" int harm_create(const harm_params *prm, const double *gcov, const dou
   rc |= al((void **)&x->stage_flag, d.cells());
   rc |= al((void **)&x->fail_list, FAIL_CAP * sizeof(int));
   rc |= al((void **)&x->fix_buf, FAIL_CAP * 8 * sizeof(double));
-  rc |= al((void **)&x->partials, 3 * x->nparts * sizeof(double));
+  rc |= al((void **)&x->partials, (3 * MASS_PARTS + 3 * SUM_WARPS) * sizeof(double));
   rc |= al((void **)&x->sc, sizeof(DevScalars));
   rc |= al((void **)&x->Ubuf, st);
   rc |= al((void **)&x->emf, 3 * G.nc * sizeof(double));
@@ -1086,7 +1179,8 @@ static int on_host_array(harm_ctx *h, double *pv, int which)
     launch_bound(x, x->ph);
   } else {
     CK(cudaMemsetAsync(&x->sc->nfail[0], 0, sizeof(int), x->stream));
-    rc = launch_fixup_utoprim(x, x->ph, 0);
+    k_fu_flip<<<148 * 8, 256, 0, x->stream>>>(G, x->pflag, x->fail_list, x->sc, 0);
+    rc = launch_repairs(x, x->ph, 0, false);
     if (rc) return rc;
   }
   CK(cudaGetLastError());

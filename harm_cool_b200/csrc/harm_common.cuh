@@ -24,6 +24,7 @@ struct DevScalars {
   int fail_code, fail_h, fail_i, fail_j;
   int err;                         // HARM_E_DT when dt < 1e-9
   int halted;                      // set after a failure: later steps do nothing
+  int ticket;                      // blocks of k_mass finished (reset by the last)
   int nfail[2];                    // failed zones of the predictor's and the corrector's fixup_utoprim
   unsigned long long divb_bits;    // diagnostics: bits of max |div B| (a positive double)
   long long divb_loc;              // and its first zone in loop order
@@ -50,7 +51,7 @@ struct TrParams {
   int n3, istart, istop, jstart, jstop, hstart, hstop;
 };
 
-constexpr int FAIL_CAP = 8192;     // failed zones listed by k_fu_flip
+constexpr int FAIL_CAP = 8192;     // failed zones listed
 constexpr int FIX_LIST_MAX = 32;   // up to this many, repaired through the sorted list
 
 struct Ctx {
@@ -104,6 +105,13 @@ __device__ __forceinline__ void record_fail(DevScalars *sc, int code, int h, int
     sc->fail_i = i;
     sc->fail_j = j;
   }
+}
+
+// fixup_utoprim's list of failed zones (slot 0 the predictor's, 1 the corrector's)
+__device__ __forceinline__ void list_failed(DevScalars *sc, int slot, int *list, long c)
+{
+  const int k = atomicAdd(&sc->nfail[slot], 1);
+  if (k < FAIL_CAP) list[k] = (int)c;
 }
 
 __device__ __forceinline__ long cidx(const Grid &G, int h, int i, int j)
@@ -171,7 +179,7 @@ struct StepRec {
   signed char *wz[2];            // which inversion gave it: 0 Utoprim_2d, 1 and 2 the fall-backs, -1 none [nc]
   double *F1rho[2];              // raw radial mass flux [nc] (the no-inflow fix reads its sign)
   double *ctop;                  // the corrector's face wave speeds, directions 1 and 2 [2][nc]
-  signed char *fl1[2];           // pflag after the first bound_prim [nc]
+  signed char *fl1[2];           // the flags after the first bound_prim, flipped: 0 a failed zone [nc]
   int *nfail[2];                 // the failed zones fixup_utoprim then met (device int)
   double *ph;                    // the predictor's final state
   DevScalars *sc[2];             // the run state before k_finalize (the corrector's Courant minima) and after
@@ -180,8 +188,9 @@ struct StepRec {
 // kernels shared by both precisions (harm_api.cu)
 int launch_bound(Ctx *x, double *P);
 int get_prims(Ctx *x, const double *src, double *p, signed char *pflag);  // device planes -> host layout
-int launch_fixup_utoprim(Ctx *x, double *P, int slot, int *nfail_out = nullptr);
-void launch_mass(Ctx *x);
+int launch_repair(Ctx *x, double *P, int slot);  // the failed zones listed in slot, then bound_prim
+void launch_mass(Ctx *x, const double *F1);     // F1: the corrector's radial fluxes
+void launch_mass(Ctx *x, const float *F1);
 int sync_status(Ctx *x);
 
 void launch_tracers(Ctx *x);     // update_tracers() (harm_tracers.cu)

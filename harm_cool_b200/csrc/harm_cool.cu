@@ -292,12 +292,14 @@ __global__ void __launch_bounds__(128, HARM_COOL_CONS_MINB) k_cons_cool(Grid G, 
 }
 
 // the update's second half (step_ch.c:265-268) and fixup() (fixup.c:51-60):
-// Utoprim_5d from the guess pi, no isentropic fall-backs under COOL_EOS
+// Utoprim_5d from the guess pi, no isentropic fall-backs under COOL_EOS; in 2D
+// (PUSH) the zone's ghost cells too
+template <bool PUSH>
 __global__ void __launch_bounds__(128, HARM_COOL_INV_MINB) k_invert_cool(Grid G, const double *__restrict__ pi,
-                                                     const double *__restrict__ Ub, double *__restrict__ pf,
-                                                     signed char *__restrict__ pflag, const double *__restrict__ geo,
+                                                     const double *__restrict__ Ub, ZoneOut O,
+                                                     const double *__restrict__ geo,
                                                      const double *__restrict__ floors, EosDev E, double *lastT,
-                                                     DevScalars *sc)
+                                                     int slot, DevScalars *sc)
 {
   if (sc->halted) return;
   const int j = G.jstart + blockIdx.x * blockDim.x + threadIdx.x;
@@ -320,10 +322,25 @@ __global__ void __launch_bounds__(128, HARM_COOL_INV_MINB) k_invert_cool(Grid G,
   lastT[c] = cur.T;
   signed char fl = (signed char)flag;
   if (fixup1zone(G.gam, __ldg(floors + gi), __ldg(floors + G.ng + gi), q, pz, &fail)) fl = -33;
+  fl = (signed char)(!fl);  // as fixup_utoprim flips the flags
+  if (fl == 0) list_failed(sc, slot, O.list, c);
 #pragma unroll
-  for (int k = 0; k < 8; k++) pf[k * G.nc + c] = pz[k];
-  pflag[c] = fl;
+  for (int k = 0; k < 8; k++) O.pf[k * G.nc + c] = pz[k];
+  O.pflag[c] = fl;
+  if (PUSH && (i == G.istart || i == G.istop || j <= G.jstart + 1 || j >= G.jstop - 1))
+    push_ghosts(G, O, geo, sc, i, j, pz, fl);
   if (fail) record_fail(sc, fail, h + (G.n3 > 1 ? 1 : 0), i, j);
+}
+
+void launch_invert_cool(Ctx *x, const double *pi, double *pf, dim3 zg, dim3 tile, int slot)
+{
+  const ZoneOut O{pf, x->pflag, x->fail_list, nullptr, nullptr};
+  if (x->G.n3 > 1)
+    k_invert_cool<false><<<zg, tile, 0, x->stream>>>(x->G, pi, x->Ubuf, O, x->geo, x->floors, x->eos, x->lastT, slot,
+                                                     x->sc);
+  else
+    k_invert_cool<true><<<zg, tile, 0, x->stream>>>(x->G, pi, x->Ubuf, O, x->geo, x->floors, x->eos, x->lastT, slot,
+                                                    x->sc);
 }
 
 template <bool FULL, bool THREE_D, bool F32>
@@ -354,12 +371,9 @@ void launch_half(Ctx *x, const double *pi, const double *pb, double *pf, bool ro
   const dim3 tile(x->tbx, x->tby);
   const dim3 zg((G.n2 + tile.x - 1) / tile.x, (G.n1 + tile.y - 1) / tile.y, G.n3);
   launch_cons_cool<FULL>(x, pi, pb, zg, tile);
-  k_invert_cool<<<zg, tile, 0, x->stream>>>(G, pi, x->Ubuf, pf, x->pflag, x->geo, x->floors, x->eos, x->lastT,
-                                            x->sc);
-  if (FULL) k_diag_flux<<<1, 1024, 0, x->stream>>>(G, x->F1, x->sc);
-  launch_bound(x, pf);
-  launch_fixup_utoprim(x, pf, FULL ? 1 : 0);
-  launch_bound(x, pf);
+  launch_invert_cool(x, pi, pf, zg, tile, FULL ? 1 : 0);
+  if (G.n3 > 1) launch_bound(x, pf);
+  launch_repair(x, pf, FULL ? 1 : 0);
 }
 
 }  // namespace cool
@@ -370,7 +384,7 @@ int cool_launch_step(Ctx *x)
   const bool rows = x->cool_seed;
   cool::launch_half<false>(x, x->p, x->p, x->ph, rows);
   cool::launch_half<true>(x, x->p, x->ph, x->p, false);
-  launch_mass(x);
+  launch_mass(x, x->F1);
   x->cool_seed = false;
   CK(cudaGetLastError());
   return HARM_OK;
@@ -522,21 +536,16 @@ int cool_time_kernels(Ctx *x, int reps, double *ms)
       slot[e] = 0; CK(cudaEventRecord(ev[e++], x->stream));
       if (full) cool::launch_cons_cool<true>(x, pi, pb, zg, tile);
       else cool::launch_cons_cool<false>(x, pi, pb, zg, tile);
-      cool::k_invert_cool<<<zg, tile, 0, x->stream>>>(G, pi, x->Ubuf, pf, x->pflag, x->geo, x->floors, x->eos,
-                                                      x->lastT, x->sc);
+      cool::launch_invert_cool(x, pi, pf, zg, tile, half);
       slot[e] = 1; CK(cudaEventRecord(ev[e++], x->stream));
-      if (full) {
-        cool::k_diag_flux<<<1, 1024, 0, x->stream>>>(G, x->F1, x->sc);
-        slot[e] = 4; CK(cudaEventRecord(ev[e++], x->stream));
+      if (G.n3 > 1) {
+        launch_bound(x, pf);
+        slot[e] = 2; CK(cudaEventRecord(ev[e++], x->stream));
       }
-      launch_bound(x, pf);
-      slot[e] = 2; CK(cudaEventRecord(ev[e++], x->stream));
-      launch_fixup_utoprim(x, pf, half);
+      launch_repair(x, pf, half);
       slot[e] = 3; CK(cudaEventRecord(ev[e++], x->stream));
-      launch_bound(x, pf);
-      slot[e] = 2; CK(cudaEventRecord(ev[e++], x->stream));
     }
-    launch_mass(x);
+    launch_mass(x, x->F1);
     slot[e] = 4; CK(cudaEventRecord(ev[e++], x->stream));
     CK(cudaEventSynchronize(ev[e - 1]));
     for (int k = 1; k < e; k++) {
@@ -546,7 +555,7 @@ int cool_time_kernels(Ctx *x, int reps, double *ms)
     }
   }
   for (auto &e : ev) cudaEventDestroy(e);
-  const double per_step[HARM_NKERNELS] = {2, 2, 4, 2, 1};
+  const double per_step[HARM_NKERNELS] = {2, 2, 2, 2, 1};
   for (int k = 0; k < HARM_NKERNELS; k++) ms[k] = acc[k] / (reps * per_step[k]);
   return sync_status(x);
 }

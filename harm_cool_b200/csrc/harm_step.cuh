@@ -30,20 +30,12 @@
 #ifndef HARM_INV_MINB
 #define HARM_INV_MINB 1
 #endif
-// phi planes each block of the zone kernels sweeps: consecutive planes of one
-// (r, theta) tile reuse its geometry from L1
-#ifndef HARM_HB_ZONE
-#define HARM_HB_ZONE 4
+#ifndef HARM_UPD_MINB
+#define HARM_UPD_MINB 3
 #endif
 
 namespace harm {
 namespace HARM_VARIANT {
-
-// blocks of tile.x (theta) by tile.y (r) zones, HARM_HB_ZONE phi planes each
-inline dim3 zone_grid_hb(const Grid &G, dim3 tile)
-{
-  return dim3((G.n2 + tile.x - 1) / tile.x, (G.n1 + tile.y - 1) / tile.y, (G.n3 + HARM_HB_ZONE - 1) / HARM_HB_ZONE);
-}
 
 #if HARM_STEP_MIXED
 using flux_t = float;
@@ -427,14 +419,28 @@ __global__ void __launch_bounds__(128) k_emf(Grid G, const flux_t *__restrict__ 
   }
 }
 
+// Where the update takes a corner's EMFs from: the planes k_emf filled, or (2D)
+// the raw face fluxes around the corner.
+struct EmfPlanes {
+  const double *emf;
+  __device__ __forceinline__ double at(const Grid &G, int n, int h, int i, int j) const
+  {
+    return __ldg(emf + n * G.nc + cidx(G, h, i, j));
+  }
+};
+struct EmfFaces {
+  const Flux &FX;
+  __device__ __forceinline__ double at(const Grid &, int, int, int i, int j) const { return FX.emf2(i, j); }
+};
+
 // The flux divergence of the update (step_ch.c:247-263) one conserved
 // component at a time, U[k] += Dt (-dF1/dx1 - dF2/dx2 [- dF3/dx3] + dU[k]), with
 // the same face fluxes zone_fluxes forms (the no-inflow mass-flux fix, and the
-// field components rebuilt from the corner EMFs of flux_ct, read from k_emf's
-// planes), so only one component's six face values are live at a time.
-template <bool THREE_D>
-__device__ __forceinline__ void flux_update(const Flux &FX, const double *__restrict__ emf, int h, int i, int j,
-                                            double Dt, const double *dU, double *U)
+// field components rebuilt from the corner EMFs of flux_ct), so only one
+// component's six face values are live at a time.
+template <bool THREE_D, class Emf>
+__device__ __forceinline__ void flux_update(const Flux &FX, const Emf &emf, int h, int i, int j, double Dt,
+                                            const double *dU, double *U)
 {
   const Grid &G = FX.G;
   const int hp = THREE_D ? hwrap(G, h + 1) : 0;
@@ -465,22 +471,21 @@ __device__ __forceinline__ void flux_update(const Flux &FX, const double *__rest
     const double f3m = THREE_D ? FX.raw(3, k, h, i, j) : 0., f3p = THREE_D ? FX.raw(3, k, hp, i, j) : 0.;
     upd(k, f1m, f1p, f2m, f2p, f3m, f3p);
   }
-  const double *E1 = emf, *E2 = emf + G.nc, *E3 = emf + 2 * G.nc;
   if (!THREE_D) {
-    const double eA = __ldg(E3 + cidx(G, 0, i, j)), eB = __ldg(E3 + cidx(G, 0, i, j + 1));
-    const double eC = __ldg(E3 + cidx(G, 0, i + 1, j)), eD = __ldg(E3 + cidx(G, 0, i + 1, j + 1));
+    const double eA = emf.at(G, 2, 0, i, j), eB = emf.at(G, 2, 0, i, j + 1);
+    const double eC = emf.at(G, 2, 0, i + 1, j), eD = emf.at(G, 2, 0, i + 1, j + 1);
     upd(B1, 0., 0., -0.5 * (eA + eC), -0.5 * (eB + eD), 0., 0.);
     upd(B2, 0.5 * (eA + eB), 0.5 * (eC + eD), 0., 0., 0., 0.);
     upd(B3, FX.raw(1, B3, 0, i, j), FX.raw(1, B3, 0, i + 1, j), FX.raw(2, B3, 0, i, j), FX.raw(2, B3, 0, i, j + 1),
         0., 0.);
   } else {
-    const double e3a = __ldg(E3 + cidx(G, h, i, j)), e3b = __ldg(E3 + cidx(G, h, i, j + 1));
-    const double e3c = __ldg(E3 + cidx(G, h, i + 1, j)), e3d = __ldg(E3 + cidx(G, h, i + 1, j + 1));
-    const double e2a = __ldg(E2 + cidx(G, h, i, j)), e2b = __ldg(E2 + cidx(G, hp, i, j));
-    const double e2c = __ldg(E2 + cidx(G, h, i + 1, j)), e2d = __ldg(E2 + cidx(G, hp, i + 1, j));
+    const double e3a = emf.at(G, 2, h, i, j), e3b = emf.at(G, 2, h, i, j + 1);
+    const double e3c = emf.at(G, 2, h, i + 1, j), e3d = emf.at(G, 2, h, i + 1, j + 1);
+    const double e2a = emf.at(G, 1, h, i, j), e2b = emf.at(G, 1, hp, i, j);
+    const double e2c = emf.at(G, 1, h, i + 1, j), e2d = emf.at(G, 1, hp, i + 1, j);
     upd(B1, 0., 0., -0.5 * (e3a + e3c), -0.5 * (e3b + e3d), 0.5 * (e2a + e2c), 0.5 * (e2b + e2d));
-    const double e1a = __ldg(E1 + cidx(G, h, i, j)), e1b = __ldg(E1 + cidx(G, hp, i, j));
-    const double e1c = __ldg(E1 + cidx(G, h, i, j + 1)), e1d = __ldg(E1 + cidx(G, hp, i, j + 1));
+    const double e1a = emf.at(G, 0, h, i, j), e1b = emf.at(G, 0, hp, i, j);
+    const double e1c = emf.at(G, 0, h, i, j + 1), e1d = emf.at(G, 0, hp, i, j + 1);
     upd(B2, 0.5 * (e3a + e3b), 0.5 * (e3c + e3d), 0., 0., -0.5 * (e1a + e1c), -0.5 * (e1b + e1d));
     upd(B3, -0.5 * (e2a + e2b), -0.5 * (e2c + e2d), 0.5 * (e1a + e1b), 0.5 * (e1c + e1d), 0., 0.);
   }
@@ -494,40 +499,25 @@ __device__ void source(double gam, const double *pb, const Geo &q, const double 
   source_of_state(gam, pb, s, q, conn, ng, gi, dU);
 }
 
-// The zone update (step_ch.c:237-306) in two launches, so that each holds
-// fewer registers and more warps stay resident to cover FP64 latency:
-// k_cons forms U -- flux_ct (step_ch.c:514-629, 726-798), the flux boundary
-// fixes (coord.c:264-324), source() (phys.c:165-207), primtoU of pi and the
-// flux divergence (step_ch.c:247-263) -- into Ub; k_invert runs Utoprim_2d
-// with the isentropic fall-backs (step_ch.c:265-300) and fixup()
-// (fixup.c:142-383).  The order of every floating-point operation is the
-// reference's.
-template <bool FULL, bool THREE_D>
-__global__ void __launch_bounds__(128, HARM_CONS_MINB) k_cons(Grid G, const double *__restrict__ pi,
-                                                              const double *__restrict__ pb,
-                                                              const flux_t *__restrict__ F1,
-                                                              const flux_t *__restrict__ F2,
-                                                              const flux_t *__restrict__ F3,
-                                                              const double *__restrict__ geo,
-                                                              const double *__restrict__ conn,
-                                                              const float *__restrict__ geo32,
-                                                              const float *__restrict__ conn32,
-                                                              const double *__restrict__ emf,
-                                                              double *__restrict__ Ub, DevScalars *sc)
+// What the update of a zone reads besides the state and the fluxes.
+struct ZoneData {
+  const double *geo, *conn;
+  const float *geo32, *conn32;
+  const double *floors, *katm;
+};
+
+// U of zone (h, i, j) after the half step: flux_ct (step_ch.c:514-629,
+// 726-798), the flux boundary fixes (coord.c:264-324), source() (phys.c:165-207),
+// primtoU of pi and the flux divergence (step_ch.c:247-263).  The order of every
+// floating-point operation is the reference's.
+template <bool FULL, bool THREE_D, class Emf>
+__device__ __forceinline__ void cons_zone(const Grid &G, const double *__restrict__ pi, const double *__restrict__ pb,
+                                          const Flux &FX, const Emf &emf, const ZoneData &Z, const Geo &q, double Dt,
+                                          int h, int i, int j, double *U, int *fail)
 {
-  if (sc->halted) return;
-  const int j = G.jstart + blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = G.istart + blockIdx.y * blockDim.y + threadIdx.y;
-  if (i > G.istop || j > G.jstop) return;
-  const double Dt = FULL ? sc->dt : 0.5 * sc->dt;
-  const int h0 = blockIdx.z * HARM_HB_ZONE, h1 = min(G.n3, h0 + HARM_HB_ZONE);
-  for (int h = h0; h < h1; h++) {
   const long c = cidx(G, h, i, j);
   const long gi = (long)i * G.sn2 + j;
-  int fail = 0;
-  Geo q;
-  load_geo(geo_at(geo, G, L_CENT), G.ng, gi, q);
-  double dU[8], U[8];
+  double dU[8];
 #if HARM_STEP_MIXED
   if (i >= G.isrc32) {
     // away from the horizon: the connection source in float (harm_phys32.cuh)
@@ -535,13 +525,13 @@ __global__ void __launch_bounds__(128, HARM_CONS_MINB) k_cons(Grid G, const doub
 #pragma unroll
     for (int k = 0; k < 8; k++) pf32[k] = (float)__ldg(pb + k * G.nc + c);
     GeoF qf;
-    load_geo_f(geo32 + (long)L_CENT * GEO_N * G.ng, G.ng, gi, qf);
-    source_f((float)G.gam, pf32, qf, conn32, G.ng, gi, dU, &fail);
+    load_geo_f(Z.geo32 + (long)L_CENT * GEO_N * G.ng, G.ng, gi, qf);
+    source_f((float)G.gam, pf32, qf, Z.conn32, G.ng, gi, dU, fail);
     double pz[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) pz[k] = __ldg(pi + k * G.nc + c);
     State s;
-    get_state(pz, q, s, &fail);
+    get_state(pz, q, s, fail);
     primtoflux(G.gam, pz, s, 0, q.g, U);
   } else
 #endif
@@ -552,27 +542,54 @@ __global__ void __launch_bounds__(128, HARM_CONS_MINB) k_cons(Grid G, const doub
 #pragma unroll
     for (int k = 0; k < 8; k++) pz[k] = __ldg(pb + k * G.nc + c);
     State s;
-    get_state(pz, q, s, &fail);
-    source_of_state(G.gam, pz, s, q, conn, G.ng, gi, dU);
+    get_state(pz, q, s, fail);
+    source_of_state(G.gam, pz, s, q, Z.conn, G.ng, gi, dU);
     primtoflux(G.gam, pz, s, 0, q.g, U);
   } else {
     {
       double pbz[8];
 #pragma unroll
       for (int k = 0; k < 8; k++) pbz[k] = __ldg(pb + k * G.nc + c);
-      source(G.gam, pbz, q, conn, G.ng, gi, dU, &fail);
+      source(G.gam, pbz, q, Z.conn, G.ng, gi, dU, fail);
     }
     double pz[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) pz[k] = __ldg(pi + k * G.nc + c);
     State s;
-    get_state(pz, q, s, &fail);
+    get_state(pz, q, s, fail);
     primtoflux(G.gam, pz, s, 0, q.g, U);
   }
-  flux_update<THREE_D>(Flux{F1, F2, F3, G}, emf, h, i, j, Dt, dU, U);
+  flux_update<THREE_D>(FX, emf, h, i, j, Dt, dU, U);
+}
+
+// Large grids take the update in two launches, so that each holds fewer
+// registers and more warps stay resident to cover FP64 latency: k_cons forms U
+// into Ub, k_invert inverts it.  Each block sweeps hb phi planes.
+template <bool FULL, bool THREE_D>
+__global__ void __launch_bounds__(128, HARM_CONS_MINB) k_cons(Grid G, const double *__restrict__ pi,
+                                                              const double *__restrict__ pb,
+                                                              const flux_t *__restrict__ F1,
+                                                              const flux_t *__restrict__ F2,
+                                                              const flux_t *__restrict__ F3, ZoneData Z,
+                                                              const double *__restrict__ emf,
+                                                              double *__restrict__ Ub, int hb, DevScalars *sc)
+{
+  if (sc->halted) return;
+  const int j = G.jstart + blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = G.istart + blockIdx.y * blockDim.y + threadIdx.y;
+  if (i > G.istop || j > G.jstop) return;
+  const double Dt = FULL ? sc->dt : 0.5 * sc->dt;
+  const int h0 = blockIdx.z * hb, h1 = min(G.n3, h0 + hb);
+  for (int h = h0; h < h1; h++) {
+    const long c = cidx(G, h, i, j);
+    int fail = 0;
+    Geo q;
+    load_geo(geo_at(Z.geo, G, L_CENT), G.ng, (long)i * G.sn2 + j, q);
+    double U[8];
+    cons_zone<FULL, THREE_D>(G, pi, pb, Flux{F1, F2, F3, G}, EmfPlanes{emf}, Z, q, Dt, h, i, j, U, &fail);
 #pragma unroll
-  for (int k = 0; k < 8; k++) Ub[k * G.nc + c] = U[k];
-  if (fail) record_fail(sc, fail, h + (THREE_D ? 1 : 0), i, j);
+    for (int k = 0; k < 8; k++) Ub[k * G.nc + c] = U[k];
+    if (fail) record_fail(sc, fail, h + (THREE_D ? 1 : 0), i, j);
   }
 }
 
@@ -587,104 +604,153 @@ static __device__ __noinline__ int inversion_fallbacks(double gam, double kap, c
   return flag;
 }
 
-// REC: also keep the inversion's output before fixup() and which inversion
-// gave it (zrec, wrec), for the discrete adjoint's recomputation
-template <bool REC>
-__global__ void __launch_bounds__(128, HARM_INV_MINB) k_invert(Grid G, const double *__restrict__ pi,
-                                                               const double *__restrict__ Ub,
-                                                               double *__restrict__ pf,
-                                                               signed char *__restrict__ pflag,
-                                                               const double *__restrict__ geo,
-                                                               const double *__restrict__ floors,
-                                                               const double *__restrict__ katm, DevScalars *sc,
-                                                               double *__restrict__ zrec,
-                                                               signed char *__restrict__ wrec)
+// What a half step does with a zone's inverted primitives.
+struct ZoneOut {
+  double *pf;
+  signed char *pflag;   // 1 a good zone, 0 a failed one: as fixup_utoprim leaves the flags
+  int *list;            // failed zones, listed for the repair
+  double *zrec;         // (the adjoint) the inversion's output before fixup()
+  signed char *wrec;    // and which inversion gave it
+};
+
+// bound_prim()'s copies of an edge zone of a 2D grid (bounds.c:54-378): every
+// ghost cell there is made from one active zone, the two next to a radial
+// boundary from the edge zone (then inflow_check), the two next to a pole by
+// reflection.  The zone's own thread writes them.
+static __device__ __noinline__ void push_ghosts(const Grid &G, const ZoneOut &O, const double *__restrict__ geo,
+                                                DevScalars *sc, int i, int j, const double *v, signed char fl)
 {
-  if (sc->halted) return;
-  const int j = G.jstart + blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = G.istart + blockIdx.y * blockDim.y + threadIdx.y;
-  if (i > G.istop || j > G.jstop) return;
-  const int h0 = blockIdx.z * HARM_HB_ZONE, h1 = min(G.n3, h0 + HARM_HB_ZONE);
-  for (int h = h0; h < h1; h++) {
+  const int jm = j == G.jstart ? j - 1 : j == G.jstart + 1 ? j - 3 : j == G.jstop ? j + 1 : j == G.jstop - 1 ? j + 3 : -1;
+  const int n = i == G.istart || i == G.istop ? 3 : 1;
+  for (int m = 0; m < 2; m++) {
+    const int jt = m ? jm : j;
+    if (jt < 0) continue;
+    for (int r = 0; r < n; r++) {
+      const int it = i == G.istart ? i - r : i + r;
+      if (m == 0 && r == 0) continue;
+      double w[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) w[k] = v[k];
+      if (m) {
+        w[U2] *= -1.;
+        w[B2] *= -1.;
+      }
+      const long gi = (long)it * G.sn2 + jt;
+      if (r) {
+        Geo q;
+        load_geo(geo_at(geo, G, L_CENT), G.ng, gi, q);
+        int fail = 0;
+        inflow_check(w, q, i == G.istart ? 0 : 1, &fail);
+        if (fail) record_fail(sc, fail, 0, it, jt);
+      }
+#pragma unroll
+      for (int k = 0; k < 8; k++) O.pf[k * G.nc + gi] = w[k];
+      O.pflag[gi] = fl;
+    }
+  }
+}
+
+// Utoprim_2d with the isentropic fall-backs (step_ch.c:265-300) and fixup()
+// (fixup.c:142-383) of one zone; pz holds the guess (pi).  REC: also keep the
+// inversion's output before fixup() and which inversion gave it, for the discrete
+// adjoint's recomputation.  PUSH (2D): write the zone's ghost cells too.
+template <bool REC, bool PUSH>
+__device__ __forceinline__ void invert_zone(const Grid &G, const double *U, const Geo &q, double *pz,
+                                            const ZoneData &Z, const ZoneOut &O, DevScalars *sc, int slot, int h,
+                                            int i, int j)
+{
   const long c = cidx(G, h, i, j);
   const long gi = (long)i * G.sn2 + j;
   int fail = 0;
-  Geo q;
-  load_geo(geo_at(geo, G, L_CENT), G.ng, gi, q);
-  double U[8], pz[8];
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    U[k] = __ldg(Ub + k * G.nc + c);
-    pz[k] = __ldg(pi + k * G.nc + c);
-  }
   int flag = utoprim<0, (bool)HARM_STEP_MIXED>(G.gam, 0., U, q, pz);
   if (REC) {
     int which = 0;
     if (flag) {
       which = 1;
-      flag = utoprim<1>(G.gam, __ldg(katm + i), U, q, pz);
+      flag = utoprim<1>(G.gam, __ldg(Z.katm + i), U, q, pz);
       if (flag) {
         which = 2;
-        flag = utoprim<2>(G.gam, __ldg(katm + i), U, q, pz);
+        flag = utoprim<2>(G.gam, __ldg(Z.katm + i), U, q, pz);
       }
     }
 #pragma unroll
-    for (int k = 0; k < 8; k++) zrec[k * G.nc + c] = pz[k];
-    wrec[c] = (signed char)(flag ? -1 : which);
+    for (int k = 0; k < 8; k++) O.zrec[k * G.nc + c] = pz[k];
+    O.wrec[c] = (signed char)(flag ? -1 : which);
   } else if (flag) {
-    flag = inversion_fallbacks(G.gam, __ldg(katm + i), U, q, pz);
+    flag = inversion_fallbacks(G.gam, __ldg(Z.katm + i), U, q, pz);
   }
   signed char fl = (signed char)flag;
-  if (fixup1zone(G.gam, __ldg(floors + gi), __ldg(floors + G.ng + gi), q, pz, &fail)) fl = -33;
+  if (fixup1zone(G.gam, __ldg(Z.floors + gi), __ldg(Z.floors + G.ng + gi), q, pz, &fail)) fl = -33;
+  // fixup_utoprim's flip of the flags (fixup.c:432-445), and its list
+  fl = (signed char)(!fl);
+  if (fl == 0) list_failed(sc, slot, O.list, c);
 #pragma unroll
-  for (int k = 0; k < 8; k++) pf[k * G.nc + c] = pz[k];
-  pflag[c] = fl;
+  for (int k = 0; k < 8; k++) O.pf[k * G.nc + c] = pz[k];
+  O.pflag[c] = fl;
+  if (PUSH && (i == G.istart || i == G.istop || j <= G.jstart + 1 || j >= G.jstop - 1))
+    push_ghosts(G, O, Z.geo, sc, i, j, pz, fl);
   if (fail) record_fail(sc, fail, h + (G.n3 > 1 ? 1 : 0), i, j);
-  }
 }
 
-// diag_flux() (diag.c:437-465): sums over the inner radial face, after the
-// mass-flux fix; one block, fixed summation order
-__global__ void k_diag_flux(Grid G, const flux_t *__restrict__ F1, DevScalars *sc)
+template <bool REC, bool PUSH>
+__global__ void __launch_bounds__(128, HARM_INV_MINB) k_invert(Grid G, const double *__restrict__ pi,
+                                                               const double *__restrict__ Ub, ZoneData Z, ZoneOut O,
+                                                               int slot, int hb, DevScalars *sc)
 {
   if (sc->halted) return;
-  __shared__ double red[3][32];
-  double m = 0., e = 0., l = 0.;
-  const long n = (long)G.n3 * G.n2;
-  for (long t = threadIdx.x; t < n; t += blockDim.x) {
-    int h = (int)(t / G.n2), j = G.jstart + (int)(t % G.n2);
-    long c = cidx(G, h, G.istart, j);
-    double fr = (double)F1[RHO * G.nc + c];
-    if (fr > 0) fr = 0;
-    m += fr * G.dx2 * G.dx3;
-    e += ((double)F1[UU * G.nc + c] - fr) * G.dx2 * G.dx3;
-    l += (double)F1[U3 * G.nc + c] * G.dx2 * G.dx3;
-  }
-  m = warp_sum(m);
-  e = warp_sum(e);
-  l = warp_sum(l);
-  if ((threadIdx.x & 31) == 0) {
-    red[0][threadIdx.x >> 5] = m;
-    red[1][threadIdx.x >> 5] = e;
-    red[2][threadIdx.x >> 5] = l;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    int nw = blockDim.x >> 5;
-    double a = threadIdx.x < nw ? red[0][threadIdx.x] : 0.;
-    double b = threadIdx.x < nw ? red[1][threadIdx.x] : 0.;
-    double d = threadIdx.x < nw ? red[2][threadIdx.x] : 0.;
-    a = warp_sum(a);
-    b = warp_sum(b);
-    d = warp_sum(d);
-    if (threadIdx.x == 0) {
-      sc->mdot = a;
-      sc->edot = -b;
-      sc->ldot = d;
+  const int j = G.jstart + blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = G.istart + blockIdx.y * blockDim.y + threadIdx.y;
+  if (i > G.istop || j > G.jstop) return;
+  const int h0 = blockIdx.z * hb, h1 = min(G.n3, h0 + hb);
+  for (int h = h0; h < h1; h++) {
+    const long c = cidx(G, h, i, j);
+    Geo q;
+    load_geo(geo_at(Z.geo, G, L_CENT), G.ng, (long)i * G.sn2 + j, q);
+    double U[8], pz[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      U[k] = __ldg(Ub + k * G.nc + c);
+      pz[k] = pi[k * G.nc + c];
     }
+    invert_zone<REC, PUSH>(G, U, q, pz, Z, O, sc, slot, h, i, j);
   }
 }
 
+// Small grids take the whole update in one launch, zones numbered row by row: each
+// launch of a step costs them some 2 us beside the latency of its loads.  With the
+// ghosts, flags and failure list written here, the sums and the dt update in one
+// launch and the repair with its bound_prim in another, a 2D step is 7 launches
+// instead of 22: 128x128 FP64 85.8 -> 69 us, 251x187 mixed 87 -> 71 us.
+template <bool FULL, bool THREE_D, bool REC>
+__global__ void __launch_bounds__(128, HARM_UPD_MINB) k_update(Grid G, const double *pi, const double *pb,
+                                                               const flux_t *__restrict__ F1,
+                                                               const flux_t *__restrict__ F2,
+                                                               const flux_t *__restrict__ F3, ZoneData Z,
+                                                               const double *__restrict__ emf, ZoneOut O,
+                                                               double *__restrict__ Ub, DevScalars *sc)
+{
+  if (sc->halted) return;
+  const int f = blockIdx.x * 128 + threadIdx.x;
+  const int j = G.jstart + f % G.n2, i = G.istart + f / G.n2, h = blockIdx.z;
+  if (i > G.istop) return;
+  const double Dt = FULL ? sc->dt : 0.5 * sc->dt;
+  const long c = cidx(G, h, i, j);
+  int fail = 0;
+  Geo q;
+  load_geo(geo_at(Z.geo, G, L_CENT), G.ng, (long)i * G.sn2 + j, q);
+  double U[8], pz[8];
+  const Flux FX{F1, F2, F3, G};
+  if (THREE_D) cons_zone<FULL, THREE_D>(G, pi, pb, FX, EmfPlanes{emf}, Z, q, Dt, h, i, j, U, &fail);
+  else cons_zone<FULL, THREE_D>(G, pi, pb, FX, EmfFaces{FX}, Z, q, Dt, h, i, j, U, &fail);
+  if (fail) record_fail(sc, fail, h + (THREE_D ? 1 : 0), i, j);
+  if (REC) {
+#pragma unroll
+    for (int k = 0; k < 8; k++) Ub[k * G.nc + c] = U[k];
+  }
+#pragma unroll
+  for (int k = 0; k < 8; k++) pz[k] = pi[k * G.nc + c];
+  invert_zone<REC, !THREE_D>(G, U, q, pz, Z, O, sc, FULL ? 1 : 0, h, i, j);
+}
 
 // ---------------------------------------------------------------------------
 // one step of this variant
@@ -702,52 +768,72 @@ inline Bufs bufs(Ctx *x)
 #endif
 }
 
+// The update in one launch up to this many zones (three resident blocks of 128 on
+// every SM, one wave), in two or three launches above, whose lighter kernels keep
+// more warps resident: 251x187 (47k zones) FP64 update 37 us in one launch against
+// 39 in three with k_emf, before the launches saved around it.
+constexpr long FUSED_ZONES = 148L * HARM_UPD_MINB * 128;
+
+// Ub, zrec, wrec: the adjoint's recomputation keeps U, the inversion's output and
+// which inversion gave it there
 template <bool FULL>
-void launch_update(Ctx *x, const double *pi, const double *pb, double *pf, double *zrec = nullptr,
-                   signed char *wrec = nullptr)
+void launch_update(Ctx *x, const double *pi, const double *pb, double *pf, double *Ub = nullptr,
+                   double *zrec = nullptr, signed char *wrec = nullptr)
 {
   const Grid &G = x->G;
   Bufs B = bufs(x);
-  const dim3 tile(x->tbx, x->tby);
-  const dim3 zg = zone_grid_hb(G, tile);
+  const ZoneData Z{x->geo, x->conn, x->geo32, x->conn32, x->floors, x->katm};
+  const ZoneOut O{pf, x->pflag, x->fail_list, zrec, wrec};
+  const long zones = (long)G.n1 * G.n2 * G.n3;
+  const bool fused = zones <= FUSED_ZONES;
   const dim3 eg(((G.n2 + 1) * (G.n1 + 1) + 127) / 128, 1, G.n3);
-  if (G.n3 > 1) {
-    k_emf<true><<<eg, 128, 0, x->stream>>>(G, B.F1, B.F2, B.F3, x->emf, x->sc);
-    k_cons<FULL, true><<<zg, tile, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, x->geo, x->conn, x->geo32,
-                                                   x->conn32, x->emf, x->Ubuf, x->sc);
-  } else {
-    k_emf<false><<<eg, 128, 0, x->stream>>>(G, B.F1, B.F2, B.F3, x->emf, x->sc);
-    k_cons<FULL, false><<<zg, tile, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, x->geo, x->conn, x->geo32,
-                                                    x->conn32, x->emf, x->Ubuf, x->sc);
-  }
+  if (G.n3 > 1) k_emf<true><<<eg, 128, 0, x->stream>>>(G, B.F1, B.F2, B.F3, x->emf, x->sc);
+  else if (!fused) k_emf<false><<<eg, 128, 0, x->stream>>>(G, B.F1, B.F2, B.F3, x->emf, x->sc);
+  if (fused) {
+    const dim3 ug((G.n1 * G.n2 + 127) / 128, 1, G.n3);
+    if (G.n3 > 1)
+      k_update<FULL, true, false><<<ug, 128, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, O, nullptr, x->sc);
 #if !HARM_STEP_MIXED
-  if (zrec)
-    k_invert<true><<<zg, tile, 0, x->stream>>>(G, pi, x->Ubuf, pf, x->pflag, x->geo, x->floors, x->katm, x->sc,
-                                               zrec, wrec);
-  else
+    else if (zrec)
+      k_update<FULL, false, true><<<ug, 128, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, O, Ub, x->sc);
 #endif
-    k_invert<false><<<zg, tile, 0, x->stream>>>(G, pi, x->Ubuf, pf, x->pflag, x->geo, x->floors, x->katm, x->sc,
-                                                nullptr, nullptr);
+    else
+      k_update<FULL, false, false><<<ug, 128, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, O, nullptr, x->sc);
+    return;
+  }
+  // phi planes a block sweeps: four, whose zones share the tile's geometry in L1,
+  // where that still leaves eight blocks for every SM, one where it does not
+  // (70x50x22: update 82 us with four, 55 with one)
+  const int hb = zones >= 148L * 8 * 128 * 4 ? 4 : 1;
+  const dim3 tile(x->tbx, x->tby);
+  const dim3 zg((G.n2 + tile.x - 1) / tile.x, (G.n1 + tile.y - 1) / tile.y, (G.n3 + hb - 1) / hb);
+  double *U = Ub ? Ub : x->Ubuf;
+  if (G.n3 > 1) k_cons<FULL, true><<<zg, tile, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, U, hb, x->sc);
+  else k_cons<FULL, false><<<zg, tile, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, U, hb, x->sc);
+  if (G.n3 > 1) k_invert<false, false><<<zg, tile, 0, x->stream>>>(G, pi, U, Z, O, FULL ? 1 : 0, hb, x->sc);
+#if !HARM_STEP_MIXED
+  else if (zrec) k_invert<true, true><<<zg, tile, 0, x->stream>>>(G, pi, U, Z, O, FULL ? 1 : 0, hb, x->sc);
+#endif
+  else k_invert<false, true><<<zg, tile, 0, x->stream>>>(G, pi, U, Z, O, FULL ? 1 : 0, hb, x->sc);
 }
 
-// advance() + fixup + bound_prim + fixup_utoprim + bound_prim (step_ch.c:101-117)
+// advance() + fixup + bound_prim + fixup_utoprim + bound_prim (step_ch.c:101-117);
+// in 2D the update writes the ghosts
 template <bool FULL>
 void launch_half(Ctx *x, const double *pi, const double *pb, double *pf)
 {
   Bufs B = bufs(x);
   launch_flux<FULL>(x->G, x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc);
   launch_update<FULL>(x, pi, pb, pf);
-  if (FULL) k_diag_flux<<<1, 1024, 0, x->stream>>>(x->G, B.F1, x->sc);
-  launch_bound(x, pf);
-  launch_fixup_utoprim(x, pf, FULL ? 1 : 0);
-  launch_bound(x, pf);
+  if (x->G.n3 > 1) launch_bound(x, pf);
+  launch_repair(x, pf, FULL ? 1 : 0);
 }
 
 int launch_step(Ctx *x)
 {
   launch_half<false>(x, x->p, x->p, x->ph);
   launch_half<true>(x, x->p, x->ph, x->p);
-  launch_mass(x);
+  launch_mass(x, bufs(x).F1);
   CK(cudaGetLastError());
   return HARM_OK;
 }
@@ -755,34 +841,32 @@ int launch_step(Ctx *x)
 #if !HARM_STEP_MIXED
 // launch_half and launch_step as above, also keeping what the discrete adjoint
 // reads back (StepRec); the same kernels in the same order, so the recomputed
-// step is the step
+// step is the step (2D)
 template <bool FULL>
-static void launch_half_rec(Ctx *x, const double *pi, const double *pb, double *pf, const StepRec &r)
+static int launch_half_rec(Ctx *x, const double *pi, const double *pb, double *pf, const StepRec &r)
 {
   const int s = FULL ? 1 : 0;
   const size_t nc = (size_t)x->G.nc;
   Bufs B = bufs(x);
-  launch_flux<FULL>(x->G, x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc,
-                    FULL ? r.ctop : nullptr);
-  cudaMemcpyAsync(r.F1rho[s], B.F1 + RHO * nc, nc * sizeof(double), cudaMemcpyDeviceToDevice, x->stream);
-  launch_update<FULL>(x, pi, pb, pf, r.Z[s], r.wz[s]);
-  cudaMemcpyAsync(r.Ub[s], x->Ubuf, 8 * nc * sizeof(double), cudaMemcpyDeviceToDevice, x->stream);
-  if (FULL) k_diag_flux<<<1, 1024, 0, x->stream>>>(x->G, B.F1, x->sc);
-  launch_bound(x, pf);
-  cudaMemcpyAsync(r.X1[s], pf, 8 * nc * sizeof(double), cudaMemcpyDeviceToDevice, x->stream);
-  cudaMemcpyAsync(r.fl1[s], x->pflag, nc, cudaMemcpyDeviceToDevice, x->stream);
-  launch_fixup_utoprim(x, pf, s, r.nfail[s]);
-  launch_bound(x, pf);
+  launch_flux<FULL>(x->G, x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc, FULL ? r.ctop : nullptr);
+  CK(cudaMemcpyAsync(r.F1rho[s], B.F1 + RHO * nc, nc * sizeof(double), cudaMemcpyDeviceToDevice, x->stream));
+  launch_update<FULL>(x, pi, pb, pf, r.Ub[s], r.Z[s], r.wz[s]);
+  CK(cudaMemcpyAsync(r.X1[s], pf, 8 * nc * sizeof(double), cudaMemcpyDeviceToDevice, x->stream));
+  CK(cudaMemcpyAsync(r.fl1[s], x->pflag, nc, cudaMemcpyDeviceToDevice, x->stream));
+  CK(cudaMemcpyAsync(r.nfail[s], &x->sc->nfail[s], sizeof(int), cudaMemcpyDeviceToDevice, x->stream));
+  return launch_repair(x, pf, s);
 }
 
 int launch_step_rec(Ctx *x, const StepRec &r)
 {
-  launch_half_rec<false>(x, x->p, x->p, x->ph, r);
+  int rc = launch_half_rec<false>(x, x->p, x->p, x->ph, r);
+  if (rc) return rc;
   cudaMemcpyAsync(r.ph, x->ph, 8 * (size_t)x->G.nc * sizeof(double), cudaMemcpyDeviceToDevice, x->stream);
-  launch_half_rec<true>(x, x->p, x->ph, x->p, r);
+  rc = launch_half_rec<true>(x, x->p, x->ph, x->p, r);
+  if (rc) return rc;
   // the corrector's Courant minima, before k_finalize resets them
   cudaMemcpyAsync(r.sc[0], x->sc, sizeof(DevScalars), cudaMemcpyDeviceToDevice, x->stream);
-  launch_mass(x);
+  launch_mass(x, bufs(x).F1);
   cudaMemcpyAsync(r.sc[1], x->sc, sizeof(DevScalars), cudaMemcpyDeviceToDevice, x->stream);
   CK(cudaGetLastError());
   return HARM_OK;
@@ -791,7 +875,8 @@ int launch_step_rec(Ctx *x, const StepRec &r)
 
 // reps ordinary steps, one kernel at a time with an event after each, so
 // every kernel is timed inside the sequence it runs in; slots: flux, update,
-// bound_prim, fixup_utoprim, diagnostics
+// bound_prim (3D; in 2D the update writes the ghosts), fixup_utoprim with the
+// bound_prim after it, diagnostics
 int time_kernels(Ctx *x, int reps, double *ms)
 {
   const Grid &G = x->G;
@@ -806,25 +891,20 @@ int time_kernels(Ctx *x, int reps, double *ms)
     for (int half = 0; half < 2; half++) {
       const bool full = half == 1;
       double *pi = x->p, *pb = full ? x->ph : x->p, *pf = full ? x->p : x->ph;
-      const dim3 tile(x->tbx, x->tby);
       if (full) launch_flux<true>(G, x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc);
       else launch_flux<false>(G, x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc);
       slot[e] = 0; CK(cudaEventRecord(ev[e++], x->stream));
       if (full) launch_update<true>(x, pi, pb, pf);
       else launch_update<false>(x, pi, pb, pf);
       slot[e] = 1; CK(cudaEventRecord(ev[e++], x->stream));
-      if (full) {
-        k_diag_flux<<<1, 1024, 0, x->stream>>>(G, B.F1, x->sc);
-        slot[e] = 4; CK(cudaEventRecord(ev[e++], x->stream));
+      if (G.n3 > 1) {
+        launch_bound(x, pf);
+        slot[e] = 2; CK(cudaEventRecord(ev[e++], x->stream));
       }
-      launch_bound(x, pf);
-      slot[e] = 2; CK(cudaEventRecord(ev[e++], x->stream));
-      launch_fixup_utoprim(x, pf, half);
+      launch_repair(x, pf, half);
       slot[e] = 3; CK(cudaEventRecord(ev[e++], x->stream));
-      launch_bound(x, pf);
-      slot[e] = 2; CK(cudaEventRecord(ev[e++], x->stream));
     }
-    launch_mass(x);
+    launch_mass(x, B.F1);
     slot[e] = 4; CK(cudaEventRecord(ev[e++], x->stream));
     CK(cudaEventSynchronize(ev[e - 1]));
     for (int k = 1; k < e; k++) {
@@ -834,7 +914,7 @@ int time_kernels(Ctx *x, int reps, double *ms)
     }
   }
   for (auto &e : ev) cudaEventDestroy(e);
-  const double per_step[HARM_NKERNELS] = {2, 2, 4, 2, 1};
+  const double per_step[HARM_NKERNELS] = {2, 2, 2, 2, 1};
   for (int k = 0; k < HARM_NKERNELS; k++) ms[k] = acc[k] / (reps * per_step[k]);
   return sync_status(x);
 }
