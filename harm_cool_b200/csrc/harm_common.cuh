@@ -221,5 +221,8 @@ struct harm_eos {
   double *vals = nullptr;  // [EOS_ND][ntab][nx][ny]
   float *f32 = nullptr;    // xa32[nx], ya32[ny], e32 and p32 [ntab][nx][ny]
   unsigned char *miss = nullptr;  // [ntab][nx][ny] NaN nodes read (harm_eos_track_missing)
+  double2 *cub = nullptr;  // EosDev::cub, cub32, xrec
+  float4 *cub32 = nullptr;
+  double *xrec = nullptr;
   int device = 0;
 };

@@ -31,6 +31,59 @@ __global__ void k_eos_batch(EosDev E, int what, int f32, long n, const int *__re
   lastT[k] = c.T;
 }
 
+// The T-direction cubics of e and p whose interval is the second of a 4-node
+// window, at their left node (EosDev::cub, cub32), formed as eos_value forms them.
+// A Newton step evaluates the same few hundred of them for every zone of a radius,
+// and each cost 12 divisions.  32 and 16 bytes a node beside the 40 and 8 of the
+// values.
+__global__ void k_eos_cubics(EosDev E, double2 *cub, float4 *cub32)
+{
+  const long plane = (long)E.nx * E.ny, n = 2 * E.ntab * plane;
+  for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n; k += (long)gridDim.x * blockDim.x) {
+    const int y = (int)(k % E.ny), y0 = y - 1;
+    if (y0 < 0 || y0 + 3 >= E.ny) continue;
+    double yw[4], ys[4], mm[7];
+    const double *src = E.val + k - 1;  // EOS_E and EOS_P are the first two planes
+    for (int q = 0; q < 4; q++) {
+      yw[q] = E.ya[y0 + q];
+      ys[q] = src[q];
+    }
+    akima_slopes<4>(yw, ys, mm);
+    const AkimaCubic c = akima_cubic<4>(yw, ys, mm, 1);
+    cub[2 * k] = make_double2(c.yi, c.si);
+    cub[2 * k + 1] = make_double2(c.c1, c.c2);
+    if (!cub32) continue;
+    float yf[4], vf[4], mf[7];
+    const float *sf = k < E.ntab * plane ? E.e32 + k - 1 : E.p32 + (k - E.ntab * plane) - 1;
+    for (int q = 0; q < 4; q++) {
+      yf[q] = E.ya32[y0 + q];
+      vf[q] = sf[q];
+    }
+    akima_slopes_f<4>(yf, vf, mf);
+    cub32[k] = akima_cubic_f<4>(yf, vf, mf, 1);
+  }
+}
+
+// the reciprocals of akima_window_rec's divisors at every 4-node window of the rho
+// axis, in its expressions; 0 for a divisor outside div_rec's range
+static std::vector<double> axis_reciprocals(const double *xa, long nx)
+{
+  std::vector<double> rec((size_t)nx * 8, 0.);
+  auto put = [&](long k, int e, double b) {
+    if (b >= ldexp(1., -200) && b <= ldexp(1., 200)) rec[(size_t)k * 8 + e] = 1. / b;
+  };
+  for (long k = 0; k + 3 < nx; k++) {
+    const double *x = xa + k;
+    const double xl1 = x[0] + x[1] - x[2], xr2 = x[3] + x[2] - x[1];
+    put(k, 1, x[0] - xl1);
+    for (int e = 0; e < 3; e++) put(k, e + 2, x[e + 1] - x[e]);
+    put(k, 5, xr2 - x[3]);
+    const double d0 = x[2] - x[1];
+    put(k, 7, d0 * d0);
+  }
+  return rec;
+}
+
 // the power of two that centres a plane's magnitudes (log scale) in the float
 // range; 0 when they span more than float can hold.  NaN nodes (tables filled
 // on demand, nodes not computed yet) stay NaN in the copy and do not count.
@@ -142,6 +195,27 @@ extern "C" int harm_eos_create(const harm_eos_desc *dsc, const double *xaxis, co
   d.hdfac = hdfac ? e->axes + nx + ny : nullptr;
   d.l_unit = dsc->l_unit;
   d.miss = nullptr;
+  // the tables derived from the values; without room for them every evaluation
+  // takes the general way
+  d.cub = nullptr;
+  d.cub32 = nullptr;
+  d.xrec = nullptr;
+  const std::vector<double> rec = harm::axis_reciprocals(xaxis, nx);
+  if (cudaMalloc(&e->cub, 4 * np * sizeof(double2)) == cudaSuccess &&
+      (!f32 || cudaMalloc(&e->cub32, 2 * np * sizeof(float4)) == cudaSuccess) &&
+      cudaMalloc(&e->xrec, rec.size() * sizeof(double)) == cudaSuccess &&
+      cudaMemcpy(e->xrec, rec.data(), rec.size() * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess) {
+    harm::k_eos_cubics<<<148 * 8, 256>>>(d, e->cub, e->cub32);
+    if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+      harm_eos_destroy(e);
+      return fail_with(HARM_E_CUDA, "EOS tables: cubics");
+    }
+    d.cub = e->cub;
+    d.cub32 = e->cub32;
+    d.xrec = e->xrec;
+  } else {
+    cudaGetLastError();  // an allocation that failed
+  }
   *out = e;
   return HARM_OK;
 }
@@ -153,6 +227,9 @@ extern "C" int harm_eos_destroy(harm_eos *e)
   cudaFree(e->vals);
   cudaFree(e->f32);
   cudaFree(e->miss);
+  cudaFree(e->cub);
+  cudaFree(e->cub32);
+  cudaFree(e->xrec);
   delete e;
   return HARM_OK;
 }

@@ -11,7 +11,8 @@
 // expression in the reference's order, the FP64 results are the reference's bit
 // for bit.  Two changes that cannot alter a result:
 //  * an Akima window's cubic is formed only for the interval the evaluation
-//    selects (the reference forms all of them and uses one);
+//    selects (the reference forms all of them and uses one), and those along T of
+//    e and p once per table: a cubic depends on its window's nodes alone.
 //  * the Newton loop stops when a step is refused (the reference repeats the
 //    identical pass until its 300 iterations are spent).
 // The temperature guess that the reference keeps per zone behind the global
@@ -50,6 +51,13 @@ struct EosDev {
   // path) met a NaN node (tables filled on demand leave the nodes not yet
   // generated NaN); null when not tracked
   unsigned char *miss;
+  // The T-direction cubics of e and p, [2][ntab][nx][ny], where the interval's left
+  // node is the second of a 4-node window: {y, s, c1, c2} (AkimaCubic without its
+  // node), formed once by the routines below; null when device memory had no
+  // room.  xrec[nx][8]: the reciprocals of akima_window_rec's divisors.
+  const double2 *cub;  // two per node
+  const float4 *cub32;
+  const double *xrec;
 };
 
 // record the NaN nodes of a loaded row of n nodes, table tab, rho node x, T nodes from y0
@@ -73,36 +81,21 @@ struct AkimaCubic {
   }
 };
 
-// The T-direction cubics of one value plane's window, one per rho row, kept
-// while the window (table, rho window, T window) and each row's interval stay
-// the same: a cubic depends on nothing else, so a kept one is the one the
-// reference forms again.
-struct AkimaRowCache {
-  int tab, x0, y0, sx, sy;  // tab < 0: empty
-  int iv[4];                // each row's interval (-1: none kept)
-  AkimaCubic c[4];
-};
-
 struct EosCursor {
   int tab;          // radial index of the table (cacheT[i])
   double T;         // the zone's temperature guess (*LastT)
   bool memo, m_f32;
   double m_rho, m_u, m_p, m_T;
-  bool keep;             // keep cubics between evaluations
-  AkimaRowCache ce, cp;  // cubics of the e and p windows last used
 };
 
 // a cursor on table tab with guess T, nothing remembered
-__device__ __forceinline__ EosCursor eos_cursor(int tab, double T, bool keep = true)
+__device__ __forceinline__ EosCursor eos_cursor(int tab, double T)
 {
   EosCursor c;
   c.tab = tab;
   c.T = T;
   c.memo = false;
   c.m_f32 = false;
-  c.keep = keep;
-  c.ce.tab = -1;
-  c.cp.tab = -1;
   return c;
 }
 
@@ -212,64 +205,71 @@ __device__ __forceinline__ void akima_window(const double *x, const double *y, d
   }
 }
 
+// a / b for a divisor of the rho axis, y = RN(1/b) or 0 where b lies outside
+// [2^-200, 2^200]: div_rn (harm_phys.cuh) over wider ranges of b, which a table's
+// squared spacings need
+__device__ __forceinline__ double div_rec(double a, double b, double y)
+{
+  const unsigned ea = (unsigned)(__double_as_longlong(a) >> 52) & 0x7ffu;
+  if (y == 0. || ea - 423u > 1200u) return a / b;  // a outside [2^-600, 2^600], zero, inf, NaN
+  double q = a * y;
+  double r = fma(-q, b, a);
+  q = fma(r, y, q);
+  r = fma(-q, b, a);
+  return fma(r, y, q);
+}
+
+// akima_window<4, false> at t in the window's second interval, its divisions by
+// the axis's spacings through their reciprocals rec: those of mm[0] .. mm[6] in
+// order, then that of the squared spacing of the interval
+__device__ __forceinline__ double akima_window_rec(const double *x, const double *y, const double *__restrict__ rec,
+                                                   double t)
+{
+  double mm[7];
+#pragma unroll
+  for (int k = 0; k < 3; k++) mm[k + 2] = div_rec(y[k + 1] - y[k], x[k + 1] - x[k], __ldg(rec + k + 2));
+  const double xl1 = x[0] + x[1] - x[2];
+  const double xl0 = xl1 + x[0] - x[1];
+  const double yl1 = (x[0] - xl1) * (mm[3] - 2.0 * mm[2]) + y[0];
+  mm[1] = div_rec(y[0] - yl1, x[0] - xl1, __ldg(rec + 1));
+  const double xr2 = x[3] + x[2] - x[1];
+  const double yr2 = (2.0 * mm[4] - mm[3]) * (xr2 - x[3]) + y[3];
+  mm[5] = div_rec(yr2 - y[3], xr2 - x[3], __ldg(rec + 5));
+  (void)xl0;  // mm[0] and mm[6] do not enter the second interval's cubic
+  const double si = akima_node(mm[1], mm[2], mm[3], mm[4]), si1 = akima_node(mm[2], mm[3], mm[4], mm[5]);
+  const double d0 = x[2] - x[1], d1 = y[2] - y[1];
+  const double t2 = div_rec(d1, d0, __ldg(rec + 3));
+  AkimaCubic c;
+  c.xi = x[1];
+  c.yi = y[1];
+  c.si = si;
+  c.c1 = div_rec(3.0 * t2 - 2.0 * si - si1, d0, __ldg(rec + 3));
+  c.c2 = div_rec(si + si1 - 2.0 * t2, d0 * d0, __ldg(rec + 7));
+  return c.at(t);
+}
+
 // getvalues at (rho, T) for one value plane: Akima along T on each rho row of
-// the window, then along rho (cache4d.c:1086-1127).  With a cache, a row whose
-// T-interval is the one kept reuses its cubic.
+// the window, then along rho (cache4d.c:1086-1127)
 template <int SX, int SY, bool DER>
 __device__ __noinline__ void eos_value_w(const EosDev &E, const double *__restrict__ plane, int tab, int x0, int y0,
-                                         double rho, double T, double &val, double &der, AkimaRowCache *cache)
+                                         double rho, double T, double &val, double &der)
 {
   double xw[SX], yw[SY], row[SX], rowd[SX];
 #pragma unroll
   for (int k = 0; k < SX; k++) xw[k] = __ldg(E.xa + x0 + k);
 #pragma unroll
   for (int k = 0; k < SY; k++) yw[k] = __ldg(E.ya + y0 + k);
-  if (cache && !(cache->tab == tab && cache->x0 == x0 && cache->y0 == y0 && cache->sx == SX && cache->sy == SY)) {
-    cache->tab = tab;
-    cache->x0 = x0;
-    cache->y0 = y0;
-    cache->sx = SX;
-    cache->sy = SY;
-#pragma unroll
-    for (int r = 0; r < 4; r++) cache->iv[r] = -1;
-  }
-  const int i = akima_interval<SY>(yw, T);
-  // spline_akima_der's points (akima.c:259-298)
-  const double h = T * 1.0E-6;
-  const double tm = T - h, tp = T + h;
-  const int im = DER ? akima_interval<SY>(yw, tm) : i, ip = DER ? akima_interval<SY>(yw, tp) : i;
-#pragma unroll
+#pragma unroll 1
   for (int r = 0; r < SX; r++) {
     const double *src = plane + (long)(x0 + r) * E.ny + y0;
-    double ys[SY], mm[SY + 3];
-    bool have = false;
-    AkimaCubic c;
-    if (cache && cache->iv[r] == i) {
-      c = cache->c[r];
-    } else {
+    double ys[SY];
 #pragma unroll
-      for (int k = 0; k < SY; k++) ys[k] = __ldg(src + k);
-      eos_note_missing<SY>(E, tab, x0 + r, y0, ys);
-      akima_slopes<SY>(yw, ys, mm);
-      have = true;
-      c = akima_cubic<SY>(yw, ys, mm, i);
-      if (cache) {
-        cache->c[r] = c;
-        cache->iv[r] = i;
-      }
-    }
-    row[r] = c.at(T);
-    if (DER) {
-      if ((im != i || ip != i) && !have) {
-#pragma unroll
-        for (int k = 0; k < SY; k++) ys[k] = __ldg(src + k);
-        eos_note_missing<SY>(E, tab, x0 + r, y0, ys);
-        akima_slopes<SY>(yw, ys, mm);
-      }
-      const double vm = im == i ? c.at(tm) : akima_cubic<SY>(yw, ys, mm, im).at(tm);
-      const double vp = ip == i ? c.at(tp) : akima_cubic<SY>(yw, ys, mm, ip).at(tp);
-      rowd[r] = (vp - vm) / (2.0 * h);
-    }
+    for (int k = 0; k < SY; k++) ys[k] = __ldg(src + k);
+    eos_note_missing<SY>(E, tab, x0 + r, y0, ys);
+    double v, d = 0.;
+    akima_window<SY, DER>(yw, ys, T, v, d);
+    row[r] = v;
+    rowd[r] = d;
   }
   double unused;
   akima_window<SX, false>(xw, row, rho, val, unused);
@@ -277,21 +277,51 @@ __device__ __noinline__ void eos_value_w(const EosDev &E, const double *__restri
 }
 
 // returns false outside the table (the reference's getvalues returns 0 there
-// without writing its outputs, cache4d.c:899-911)
+// without writing its outputs, cache4d.c:899-911).  e and p inside a 4 x 4 window
+// with T, its difference points and rho in the second intervals -- all but the
+// table's edges and points on a node -- take the rows' cubics from the table made
+// of them; nothing is marked missing there, so tracked tables go the general way.
+// That leaves two divisions a window of the twelve, and four windows fewer: a
+// 256x256 step's face kernels 300 -> 151 us, the update's two 200 and 470 -> 120
+// and 384 us.
 template <bool DER>
-__device__ __forceinline__ bool eos_value(const EosDev &E, int tab, int d, double rho, int x0, int sx, double T,
-                                          double &val, double &der, AkimaRowCache *cache = nullptr)
+__device__ __noinline__ bool eos_value(const EosDev &E, int tab, int d, double rho, int x0, int sx, double T,
+                                       double &val, double &der)
 {
   if (!(T >= __ldg(E.ya)) || !(T <= __ldg(E.ya + E.ny - 1))) return false;
   int y0, sy;
   eos_window(E.ny, E.ya, T, y0, sy);
+  if (E.cub && !E.miss && d <= EOS_P && sx == 4 && sy == 4) {
+    const double xi = __ldg(E.ya + y0 + 1), xr = __ldg(E.ya + y0 + 2);
+    const double h = T * 1.0E-6;  // spline_akima_der's points (akima.c:259-298)
+    const double tm = T - h, tp = T + h;
+    double xw[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) xw[k] = __ldg(E.xa + x0 + k);
+    const bool inner = (DER ? tm : T) > xi && !((DER ? tp : T) > xr) && T > xi && !(T > xr);
+    if (inner && rho > xw[1] && !(rho > xw[2])) {
+      const double2 *src = E.cub + 2 * ((((long)d * E.ntab + tab) * E.nx + x0) * E.ny + y0 + 1);
+      double row[4], rowd[4];
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        const double2 a = __ldg(src + 2L * r * E.ny), b = __ldg(src + 2L * r * E.ny + 1);
+        const AkimaCubic c{xi, a.x, a.y, b.x, b.y};
+        row[r] = c.at(T);
+        if (DER) rowd[r] = (c.at(tp) - c.at(tm)) / (2.0 * h);
+      }
+      const double *rec = E.xrec + 8 * x0;
+      val = akima_window_rec(xw, row, rec, rho);
+      if (DER) der = akima_window_rec(xw, rowd, rec, rho);
+      return true;
+    }
+  }
   const double *plane = E.val + ((long)d * E.ntab + tab) * E.nx * E.ny;
   if (sx == 4) {
-    if (sy == 4) eos_value_w<4, 4, DER>(E, plane, tab, x0, y0, rho, T, val, der, cache);
-    else eos_value_w<4, 3, DER>(E, plane, tab, x0, y0, rho, T, val, der, cache);
+    if (sy == 4) eos_value_w<4, 4, DER>(E, plane, tab, x0, y0, rho, T, val, der);
+    else eos_value_w<4, 3, DER>(E, plane, tab, x0, y0, rho, T, val, der);
   } else {
-    if (sy == 4) eos_value_w<3, 4, DER>(E, plane, tab, x0, y0, rho, T, val, der, cache);
-    else eos_value_w<3, 3, DER>(E, plane, tab, x0, y0, rho, T, val, der, cache);
+    if (sy == 4) eos_value_w<3, 4, DER>(E, plane, tab, x0, y0, rho, T, val, der);
+    else eos_value_w<3, 3, DER>(E, plane, tab, x0, y0, rho, T, val, der);
   }
   return true;
 }
@@ -305,14 +335,14 @@ __device__ __forceinline__ bool eos_rho_window(const EosDev &E, double rho, int 
 
 // mnewtc<1>(300, x, 1e-6, minx, maxx) on (e - e(rho, T)) / e; returns berr
 static __device__ __noinline__ double eos_newton_T(const EosDev &E, int tab, double rho, bool rho_in, int x0, int sx,
-                                            double e, double &x, double minx, double maxx, AkimaRowCache *ce)
+                                            double e, double &x, double minx, double maxx)
 {
   double best = x, besterr = 1.0E100;
   for (int k = 1; k <= 300; k++) {
     double ecur = CUDART_NAN, dcur = CUDART_NAN;
     if (rho_in) {
       double v, dv;
-      if (eos_value<true>(E, tab, EOS_E, rho, x0, sx, x, v, dv, ce)) { ecur = v; dcur = dv; }
+      if (eos_value<true>(E, tab, EOS_E, rho, x0, sx, x, v, dv)) { ecur = v; dcur = dv; }
     }
     const double F = (e - ecur) / e;
     const double D = -dcur / e;
@@ -352,13 +382,13 @@ static __device__ __noinline__ double eos_pressure(const EosDev &E, EosCursor &c
     int x0 = 0, sx = 4;
     const bool rho_in = eos_rho_window(E, rho, x0, sx);
     double x = c.T;
-    const double berr = eos_newton_T(E, c.tab, rho, rho_in, x0, sx, e, x, minx, maxx, c.keep ? &c.ce : nullptr);
+    const double berr = eos_newton_T(E, c.tab, rho, rho_in, x0, sx, e, x, minx, maxx);
     if (berr > 1.0E-6) p = (E.gam - 1.) * u;
     else {
       double v = CUDART_NAN, unused;
       if (rho_in) {
         double w;
-        if (eos_value<false>(E, c.tab, EOS_P, rho, x0, sx, x, w, unused, c.keep ? &c.cp : nullptr)) v = w;
+        if (eos_value<false>(E, c.tab, EOS_P, rho, x0, sx, x, w, unused)) v = w;
       }
       c.T = x;
       p = v / E.p_unit;
@@ -402,7 +432,7 @@ static __device__ __noinline__ void eos_coolval(const EosDev &E, EosCursor &c, d
     const double minx = E.t_min * (1.0 + hh), maxx = E.t_max * (1.0 - hh);
     rho_in = eos_rho_window(E, rho, x0, sx);
     x = c.T;
-    const double berr = eos_newton_T(E, c.tab, rho, rho_in, x0, sx, e, x, minx, maxx, c.keep ? &c.ce : nullptr);
+    const double berr = eos_newton_T(E, c.tab, rho, rho_in, x0, sx, e, x, minx, maxx);
     gamma_law = berr > 1.0E-6;
   }
   c.memo = false;
@@ -530,14 +560,10 @@ __device__ __forceinline__ void akima_slopes_f(const float *x, const float *y, f
   mm[SI + 2] = __fdividef(yr3 - yr2, xr3 - xr2);
 }
 
-// value (and with DER the derivative) of the cubic of the interval t falls in
-template <int SI, bool DER>
-__device__ __forceinline__ void akima_window_f(const float *x, const float *y, float t, float &v, float &dv)
+// the cubic of interval i: {y, s, c1, c2}
+template <int SI>
+__device__ __forceinline__ float4 akima_cubic_f(const float *x, const float *y, const float *mm, int i)
 {
-  float mm[SI + 3];
-  akima_slopes_f<SI>(x, y, mm);
-  int i = (t > x[1]) ? 1 : 0;
-  if (SI == 4 && t > x[2]) i = 2;
   float xi = x[0], xi1 = x[1], yi = y[0], yi1 = y[1];
   float a0 = mm[0], a1 = mm[1], a2 = mm[2], a3 = mm[3], a4 = mm[4];
   if (i >= 1) { xi = x[1]; xi1 = x[2]; yi = y[1]; yi1 = y[2]; a0 = mm[1]; a1 = mm[2]; a2 = mm[3]; a3 = mm[4]; a4 = mm[5]; }
@@ -546,11 +572,21 @@ __device__ __forceinline__ void akima_window_f(const float *x, const float *y, f
   const float d0 = xi1 - xi;
   const float rd = __fdividef(1.f, d0);
   const float t2 = (yi1 - yi) * rd;
-  const float c1 = (3.f * t2 - 2.f * si - si1) * rd;
-  const float c2 = (si + si1 - 2.f * t2) * rd * rd;
-  const float u = t - xi;
-  v = __fmaf_rn(__fmaf_rn(__fmaf_rn(c2, u, c1), u, si), u, yi);
-  if (DER) dv = __fmaf_rn(__fmaf_rn(3.f * c2, u, 2.f * c1), u, si);
+  return make_float4(yi, si, (3.f * t2 - 2.f * si - si1) * rd, (si + si1 - 2.f * t2) * rd * rd);
+}
+
+// value (and with DER the derivative) of the cubic of the interval t falls in
+template <int SI, bool DER>
+__device__ __forceinline__ void akima_window_f(const float *x, const float *y, float t, float &v, float &dv)
+{
+  float mm[SI + 3];
+  akima_slopes_f<SI>(x, y, mm);
+  int i = (t > x[1]) ? 1 : 0;
+  if (SI == 4 && t > x[2]) i = 2;
+  const float4 c = akima_cubic_f<SI>(x, y, mm, i);
+  const float u = t - (i == 0 ? x[0] : SI == 4 && i == 2 ? x[2] : x[1]);
+  v = __fmaf_rn(__fmaf_rn(__fmaf_rn(c.w, u, c.z), u, c.y), u, c.x);
+  if (DER) dv = __fmaf_rn(__fmaf_rn(3.f * c.w, u, 2.f * c.z), u, c.y);
 }
 
 template <int SX, int SY, bool DER>
@@ -578,13 +614,33 @@ __device__ __noinline__ void eos_value_wf(const EosDev &E, const float *__restri
   if (DER) akima_window_f<SX, false>(xw, rowd, rho, der, unused);
 }
 
+// d: EOS_E or EOS_P; the rows' cubics from their table as in eos_value
 template <bool DER>
-__device__ __forceinline__ bool eos_value_f(const EosDev &E, int tab, const float *planes, float rho, int x0, int sx,
-                                            float T, float &val, float &der)
+__device__ __noinline__ bool eos_value_f(const EosDev &E, int tab, int d, float rho, int x0, int sx, float T,
+                                         float &val, float &der)
 {
   if (!(T >= __ldg(E.ya32)) || !(T <= __ldg(E.ya32 + E.ny - 1))) return false;
   int y0, sy;
   eos_window_f(E.ny, E.ya32, T, y0, sy);
+  if (E.cub32 && !E.miss && sx == 4 && sy == 4) {
+    const float xi = __ldg(E.ya32 + y0 + 1), xr = __ldg(E.ya32 + y0 + 2);
+    if (T > xi && !(T > xr)) {
+      const float4 *src = E.cub32 + (((long)d * E.ntab + tab) * E.nx + x0) * E.ny + y0 + 1;
+      float xw[4], row[4], rowd[4], unused;
+      const float u = T - xi;
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        xw[r] = __ldg(E.xa32 + x0 + r);
+        const float4 w = __ldg(src + (long)r * E.ny);  // y, s, c1, c2
+        row[r] = __fmaf_rn(__fmaf_rn(__fmaf_rn(w.w, u, w.z), u, w.y), u, w.x);
+        if (DER) rowd[r] = __fmaf_rn(__fmaf_rn(3.f * w.w, u, 2.f * w.z), u, w.y);
+      }
+      akima_window_f<4, false>(xw, row, rho, val, unused);
+      if (DER) akima_window_f<4, false>(xw, rowd, rho, der, unused);
+      return true;
+    }
+  }
+  const float *planes = d == EOS_E ? E.e32 : E.p32;
   const float *plane = planes + (long)tab * E.nx * E.ny;
   if (sx == 4) {
     if (sy == 4) eos_value_wf<4, 4, DER>(E, plane, tab, x0, y0, rho, T, val, der);
@@ -605,7 +661,7 @@ static __device__ __noinline__ float eos_newton_T_f(const EosDev &E, int tab, fl
     float ecur = CUDART_NAN_F, dcur = CUDART_NAN_F;
     if (rho_in) {
       float v, dv;
-      if (eos_value_f<true>(E, tab, E.e32, rho, x0, sx, x, v, dv)) { ecur = v; dcur = dv; }
+      if (eos_value_f<true>(E, tab, EOS_E, rho, x0, sx, x, v, dv)) { ecur = v; dcur = dv; }
     }
     const float re = __fdividef(1.f, e);
     const float F = (e - ecur) * re;
@@ -654,7 +710,7 @@ static __device__ __noinline__ double eos_pressure_f(const EosDev &E, EosCursor 
       float v = CUDART_NAN_F, unused;
       if (rho_in) {
         float w;
-        if (eos_value_f<false>(E, c.tab, E.p32, rf, x0, sx, x, w, unused)) v = w;
+        if (eos_value_f<false>(E, c.tab, EOS_P, rf, x0, sx, x, w, unused)) v = w;
       }
       c.T = (double)x;
       p = (double)v / E.sp / E.p_unit;
