@@ -1,5 +1,6 @@
 // The COOL_EOS table generator on the device: abundance() (harm_nu.cuh) at
-// every node of the per-radius (rho, T) tables, one warp per node.
+// every node of the per-radius (rho, T) tables, one block of three or nine warps
+// per node.
 //
 // The reference fills the same tables lazily on the host, node by node, with
 // six worker threads calling its Fortran abundance_() (cooleos.c:171-194,
@@ -10,14 +11,15 @@
 // (where free nucleons are a trace, at a few 1e8 K, the proton-fraction solve
 // runs all 200 of its trials, each over three nested solves).  A thread per
 // node would leave a warp waiting on its slowest lane and run each
-// quadrature's terms one after another; a warp per node keeps its lanes on
-// one control flow and spreads the terms of every quadrature over them
-// (lane_sum, harm_nu.cuh).
+// quadrature's terms one after another; a warp keeps its lanes on one control
+// flow and spreads the terms of every quadrature over them (lane_sum,
+// harm_nu.cuh), and the warps of a node share its independent solves
+// (degeneracies, FuncNb3).
 //
-// Six blocks of four warps per SM (80 registers a thread): the warps' long
-// FP64 latency chains (exp, log, division) need that many to keep the FP64
-// pipe busy; measured 1.13x faster than four blocks at 128 registers, which
-// were 1.44x faster than three at 168.
+// 24 warps per SM (80 registers a thread): the warps' long FP64 latency chains
+// (exp, log, division) need that many to keep the FP64 pipe busy; with one warp a
+// node, measured 1.13x faster than 16 at 128 registers, which were 1.44x faster
+// than 12 at 168.
 //
 // Tables are launched one per kernel over several streams without waiting in
 // between, so the blocks of a table still on its slowest nodes share the SMs
@@ -37,6 +39,15 @@ const Rules *host_rules();
 
 __constant__ Rules c_rules;
 
+constexpr int NODE_WARPS_SM = 24;  // resident warps per SM that the register budget allows (80 registers)
+// Up to this many nodes a node gets nine warps, above it three.  Few nodes wait on
+// the slowest of them, which nine warps finish sooner; many nodes fill the GPU, and
+// then the nine wait for one another too often.  Measured (ms, nine against three;
+// one warp a node before): 288 nodes 84, 165 (485); 2,304 nodes 129, 197 (518);
+// 4,096 nodes 188, 236 (551); 10,368 nodes 397, 403 (727); 20,736 nodes 1756, 1470
+// (2682); 200x200 nodes 4521, 3443 (4908).
+constexpr long TEAM9_MAX = 10000;
+
 // the quadrature rules into shared memory: the lanes of a warp read different
 // nodes of a rule at once, which the constant cache would serialise
 __device__ __forceinline__ void load_rules(Rules &R)
@@ -46,24 +57,25 @@ __device__ __forceinline__ void load_rules(Rules &R)
   __syncthreads();
 }
 
-// node k of the slice [k0, k0 + n) on warp k - k0, with k = (t ny + j) nx + i
+// node k of the slice [k0, k0 + n) on block k - k0, with k = (t ny + j) nx + i
 // for table t, T index j and rho index i; values packed as calc_cache_val
 // packs them (cooleos.c:171-194) at values[t][i][j]: e, p, Qnu, tau,
 // Yee = (n_e- - n_e+) / n_b
-__global__ void __launch_bounds__(128, 6) k_tables(const double *xaxis, int nx, const double *yaxis, int ny,
-                                                const double *hdfac, long k0, long n, double *values)
+template <int TEAM>
+__global__ void __launch_bounds__(TEAM, NODE_WARPS_SM * 32 / TEAM) k_tables(const double *xaxis, int nx,
+                                                                            const double *yaxis, int ny,
+                                                                            const double *hdfac, long k0,
+                                                                            double *values)
 {
   __shared__ Rules R;
   load_rules(R);
-  const long w = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (w >= n) return;  // whole warps: the lanes of a node stay together
-  const long k = k0 + w;
+  const long k = k0 + blockIdx.x;
   const int i = (int)(k % nx);
   const long tj = k / nx;
   const int j = (int)(tj % ny), t = (int)(tj / ny);
   const double rho = xaxis[i];
   const Abundance a = abundance(R, rho, yaxis[j], hdfac[t]);
-  if ((threadIdx.x & 31) == 0) {
+  if (threadIdx.x == 0) {
     double *v = values + 5 * (((long)t * nx + i) * ny + j);
     v[0] = a.e;
     v[1] = a.p;
@@ -73,16 +85,16 @@ __global__ void __launch_bounds__(128, 6) k_tables(const double *xaxis, int nx, 
   }
 }
 
-// abundance() at a list of nodes, a warp per node, for checks against the host
-__global__ void __launch_bounds__(128, 6) k_nodes(const double *rho, const double *T, const double *hdfac, long n,
-                                               double *out)
+// abundance() at a list of nodes, a block per node
+template <int TEAM>
+__global__ void __launch_bounds__(TEAM, NODE_WARPS_SM * 32 / TEAM) k_nodes(const double *rho, const double *T,
+                                                                           const double *hdfac, double *out)
 {
   __shared__ Rules R;
   load_rules(R);
-  const long k = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (k >= n) return;
+  const long k = blockIdx.x;
   const Abundance a = abundance(R, rho[k], T[k], hdfac[k]);
-  if ((threadIdx.x & 31) == 0) {
+  if (threadIdx.x == 0) {
     double *o = out + 7 * k;
     o[0] = a.e;
     o[1] = a.p;
@@ -176,7 +188,10 @@ extern "C" int harm_nu_tables(int device, const double *xaxis, int nx, const dou
   int q = 0;
   for (long k0 = 0; k0 < n; k0 += slice, q = (q + 1) % NS) {
     const long m = (n - k0 < slice) ? n - k0 : slice;
-    nu::k_tables<<<(unsigned)((m + 3) / 4), 128, 0, r.st[q]>>>(dx, nx, dy, ny, dh, k0, m, dv);
+    if (n <= nu::TEAM9_MAX)
+      nu::k_tables<nu::TEAM9><<<(unsigned)m, nu::TEAM9, 0, r.st[q]>>>(dx, nx, dy, ny, dh, k0, dv);
+    else
+      nu::k_tables<nu::TEAM3><<<(unsigned)m, nu::TEAM3, 0, r.st[q]>>>(dx, nx, dy, ny, dh, k0, dv);
     CK(cudaGetLastError());
   }
   for (int s = 1; s < NS; s++) {
@@ -208,7 +223,8 @@ extern "C" int harm_nu_abundance_dev(int device, const double *rho, const double
   CK(cudaMemcpy(dr, rho, n * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(dt, T, n * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(dh, hdfac, n * sizeof(double), cudaMemcpyHostToDevice));
-  nu::k_nodes<<<(unsigned)((n + 3) / 4), 128>>>(dr, dt, dh, n, dout);
+  if (n <= nu::TEAM9_MAX) nu::k_nodes<nu::TEAM9><<<(unsigned)n, nu::TEAM9>>>(dr, dt, dh, dout);
+  else nu::k_nodes<nu::TEAM3><<<(unsigned)n, nu::TEAM3>>>(dr, dt, dh, dout);
   CK(cudaGetLastError());
   CK(cudaMemcpy(out, dout, 7 * n * sizeof(double), cudaMemcpyDeviceToHost));
   return HARM_OK;

@@ -28,9 +28,9 @@
 // inlined at every call site and unrolled, the kernel outgrew the instruction
 // cache and its warps waited on instruction fetch more than on anything else.
 //
-// One node, one warp.  A node is a nest of Newton solves whose every trial
-// evaluates Fermi integrals or rate integrals by Gauss quadrature.  All 32
-// lanes of a warp run the node's scalar code together, with the same values,
+// One node, three or nine warps (degeneracies(), FuncNb3).  A node is a nest of
+// Newton solves whose every trial evaluates Fermi integrals or rate integrals by
+// Gauss quadrature.  All 32 lanes of a warp run the node's scalar code together, with the same values,
 // and split each quadrature's terms between them (lane_sum): lane l adds
 // terms l, l + 32, ... and a butterfly over the lanes combines the partial
 // sums, so that every lane holds the same sum and the control flow stays
@@ -687,14 +687,48 @@ HNU_NOINLINE double net_rate(const Rules &R, double b1, double kt, double nn, do
   return (evep - even - evn) / fabs(evep);
 }
 
-// degeneracies of the nucleons for proton fraction xp (nuclear)
-HNU void nuclear(const Rules &R, double kt, double nb, double xp, double *etan, double *etap)
+// Several warps share a node on the device (node_warps(), a block per node):
+// three, one for each trial point of the proton-fraction solve, or nine, three
+// for each point, one for each of its degeneracy solves.  Every warp runs the
+// node's scalar code with the same values, so all take the same path through the
+// barriers below.
+#if defined(__CUDACC__)
+constexpr int TEAM3 = 96, TEAM9 = 288;  // threads a node
+// results handed between a node's warps: three of the trial points, three for each
+// point's degeneracies
+__device__ __forceinline__ double *team_buf()
+{
+  __shared__ double buf[12];
+  return buf;
+}
+#endif
+
+// degeneracies of the nucleons for proton fraction xp (nuclear) and of the
+// electrons for the net lepton density ne
+HNU void degeneracies(const Rules &R, double kt, double nb, double xp, double ne, double *etan, double *etap,
+                      double *etae)
 {
   double np = nb * xp, nn = nb - np;
   if (np <= 0.0) np = 0.0;
-  *etap = peta(R, kt, np);
   if (nn <= 0.0) nn = 0.0;
+#if defined(__CUDA_ARCH__)
+  if (blockDim.x == TEAM9) {
+    const int w = threadIdx.x >> 5, g = w / 3, r = w - 3 * g;
+    double *buf = team_buf() + 3 + 3 * g;
+    const double v = r == 0 ? peta(R, kt, np) : r == 1 ? neta(R, kt, nn) : eeta(R, kt, ne);
+    if ((threadIdx.x & 31) == 0) buf[r] = v;
+    if (g == 0) asm volatile("bar.sync 1, 96;" ::: "memory");
+    else if (g == 1) asm volatile("bar.sync 2, 96;" ::: "memory");
+    else asm volatile("bar.sync 3, 96;" ::: "memory");
+    *etap = buf[0];
+    *etan = buf[1];
+    *etae = buf[2];
+    return;
+  }
+#endif
+  *etap = peta(R, kt, np);
   *etan = neta(R, kt, nn);
+  *etae = eeta(R, kt, ne);
 }
 
 // the energy balance of the gas at proton fraction xp, with the neutrino
@@ -702,12 +736,14 @@ HNU void nuclear(const Rules &R, double kt, double nb, double xp, double *etan, 
 HNU_NOINLINE double funcnb(const Rules &R, const Nucl &c, double xp)
 {
   const double beta = c.kt / XME;
-  double etan, etap;
-  nuclear(R, c.kt, c.nnucl, xp, &etan, &etap);
   const double nhe = c.ne0 / 2.0;
   const double np = c.nnucl * xp, nn = c.nnucl - np;
   const double ne = c.nnucl * xp + c.ne0;
-  const double etae = eeta(R, c.kt, ne);
+  double etan, etap, etae;
+  degeneracies(R, c.kt, c.nnucl, xp, ne, &etan, &etap, &etae);
+#if defined(__CUDA_ARCH__)
+  if (blockDim.x == TEAM9 && (threadIdx.x >> 5) % 3 != 0) return 0.0;  // one of the point's warps goes on
+#endif
   const double etaep = -etae - 2.0 / beta;
   double b1 = 0.0, b2 = 0.0, nl, nee, nep;
   lepton<1>(R, c.kt, &etae, &nl, &nee, &nep);
@@ -733,7 +769,18 @@ struct FuncNb3 {
   const Nucl &c;
   HNU void operator()(const double *x, double *y) const
   {
+#if defined(__CUDA_ARCH__)
+    // the three points side by side, a point per warp or per three
+    const int w = threadIdx.x >> 5, per = blockDim.x == TEAM9 ? 3 : 1, g = w / per;
+    double *buf = team_buf();
+    const double v = funcnb(R, c, g == 0 ? x[0] : g == 1 ? x[1] : x[2]);
+    if (w == g * per && (threadIdx.x & 31) == 0) buf[g] = v;
+    __syncthreads();
+    for (int i = 0; i < 3; i++) y[i] = buf[i];
+    __syncthreads();
+#else
     for (int i = 0; i < 3; i++) y[i] = funcnb(R, c, x[i]);
+#endif
   }
 };
 
@@ -758,10 +805,9 @@ HNU_NOINLINE Abundance abundance(const Rules &R, double rho, double T, double hd
   double xp = newton1(FuncNb3{R, c}, (1.0 - 0.0) / 2.0, 0.0, newton_tol(c.nnucl));
   if (xp < 0.0) xp = 0.0;
   if (xp > 1.0) xp = 1.0;
-  double etan, etap;
-  nuclear(R, kt, c.nnucl, xp, &etan, &etap);
   const double np = c.nnucl * xp, nn = c.nnucl - np;
-  const double etae = eeta(R, kt, np + c.ne0);
+  double etan, etap, etae;
+  degeneracies(R, kt, c.nnucl, xp, np + c.ne0, &etan, &etap, &etae);
 
   const double etaep = -etae - 2.0 / beta;
   Abundance a;
