@@ -58,6 +58,7 @@ UNITS = {
     "harm_cool.cu": ["-fmad=false"],     # the COOL_EOS step and Utoprim_5d
     "harm_dump.cu": ["-fmad=false"],     # the ASCII dump format
     "harm_adjoint.cu": ["-fmad=false"],  # the discrete adjoint (values identical to the step's)
+    "harm_hostio.cu": ["-fmad=false"],   # threaded copies of host arrays
     "harm_peak.cu": ["-fmad=false"],     # measured FP64 pipe rates (roofline denominators)
     "harm_nu.cu": ["-fmad=false"],       # COOL_EOS table generator on the device
 }

@@ -30,6 +30,7 @@
 
 #include "harm_common.cuh"
 #include "harm_bound.cuh"
+#include "harm_hostio.cuh"
 
 namespace harm {
 
@@ -659,6 +660,12 @@ __global__ void k_utoprim_batch(const double *U, const double *gcov, const doubl
   for (int k = 0; k < 8; k++) prim[t * 8 + k] = p[k];
 }
 
+void launch_utoprim_batch(cudaStream_t st, const double *U, const double *gcov, const double *gcon, const double *gdet,
+                          double *prim, int *ret, long n, double gam)
+{
+  k_utoprim_batch<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(U, gcov, gcon, gdet, prim, ret, n, gam);
+}
+
 // Utoprim_1dvsq2fix1 (which 1) or Utoprim_1dfix1 (which 2) over independent zones
 __global__ void k_utoprim_fix_batch(int which, const double *U, const double *gcov, const double *gcon,
                                     const double *gdet, const double *K, double *prim, int *ret, long n, double gam)
@@ -962,7 +969,6 @@ extern "C" void harm_destroy(harm_ctx *h)
                   x->lastT, x->coolgeo, x->cooldiag};
   for (void *p : ptrs)
     if (p) cudaFree(p);
-  if (x->pinned) cudaFreeHost(x->pinned);
   if (x->stream) cudaStreamDestroy(x->stream);
   delete h;
 }
@@ -972,7 +978,8 @@ static int put_prims(Ctx *x, const double *p, const signed char *pflag, double *
   const Dims &d = x->D;
   const int h0 = d.n3 > 1 ? 1 : 0;
   const size_t nb = (size_t)8 * d.cells() * sizeof(double);
-  CK(cudaMemcpyAsync(x->stage, p, nb, cudaMemcpyHostToDevice, x->stream));
+  int rc = copy_to_device(x->device, x->stream, x->stage, p, nb);
+  if (rc) return rc;
   if (pflag) CK(cudaMemcpyAsync(x->stage_flag, pflag, d.cells(), cudaMemcpyHostToDevice, x->stream));
   k_from_host<<<148 * 8, 256, 0, x->stream>>>(x->G, h0, x->stage, dst, pflag ? x->stage_flag : nullptr, x->pflag);
   CK(cudaGetLastError());
@@ -986,8 +993,8 @@ int harm::get_prims(Ctx *x, const double *src, double *p, signed char *pflag)
   k_to_host<<<148 * 8, 256, 0, x->stream>>>(x->G, h0, src, x->stage, x->pflag, pflag ? x->stage_flag : nullptr);
   CK(cudaGetLastError());
   const size_t nb = (size_t)8 * d.cells() * sizeof(double);
-  if (p) CK(cudaMemcpyAsync(p, x->stage, nb, cudaMemcpyDeviceToHost, x->stream));
   if (pflag) CK(cudaMemcpyAsync(pflag, x->stage_flag, d.cells(), cudaMemcpyDeviceToHost, x->stream));
+  if (p) return copy_to_host(x->device, x->stream, p, x->stage, nb);
   CK(cudaStreamSynchronize(x->stream));
   return HARM_OK;
 }
@@ -1250,6 +1257,8 @@ extern "C" int harm_utoprim_2d_batch(const double *U, const double *gcov, const 
 {
   if (!U || !gcov || !gcon || !gdet || !prim || !ret || n < 0) return fail_with(HARM_E_ARG, "null argument");
   if (n == 0) return HARM_OK;
+  int rc = HARM_OK;
+  if (utoprim_2d_lanes(U, gcov, gcon, gdet, prim, ret, n, gam, &rc)) return rc;
   // device copies, freed on every return
   struct Buffers {
     double *dU = nullptr, *da = nullptr, *db = nullptr, *dg = nullptr, *dp = nullptr;
@@ -1269,7 +1278,7 @@ extern "C" int harm_utoprim_2d_batch(const double *U, const double *gcov, const 
   CK(cudaMemcpy(db, gcon, n * 128, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(dg, gdet, n * 8, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(dp, prim, n * 64, cudaMemcpyHostToDevice));
-  k_utoprim_batch<<<(unsigned)((n + 127) / 128), 128>>>(dU, da, db, dg, dp, dr, n, gam);
+  launch_utoprim_batch(nullptr, dU, da, db, dg, dp, dr, n, gam);
   CK(cudaGetLastError());
   CK(cudaMemcpy(prim, dp, n * 64, cudaMemcpyDeviceToHost));
   CK(cudaMemcpy(ret, dr, n * sizeof(int), cudaMemcpyDeviceToHost));

@@ -76,8 +76,6 @@ struct Ctx {
   DevScalars *sc;
   cudaGraphExec_t graph_exec;
   int graph_steps;
-  double *pinned;                // pinned host buffer for the host-array entry points
-  size_t pinned_bytes;
   int mode;                      // HARM_FP64 or HARM_MIXED
   float *F1f, *F2f, *F3f;        // mixed mode: FP32 face fluxes [8][nc]
   float *geo32;                  // mixed mode: FP32 geometry [4 locations][GEO_N][ng]

@@ -1,0 +1,80 @@
+"""Copies of host arrays through the threaded lanes: sizes around the line where
+they begin and around their chunks, arrays that do not fill them, calls from several
+threads at once, and the batched inversion at its chunk edges."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def hc(harm_lib):
+    import harm_cool_b200
+    return harm_cool_b200
+
+
+# 8 MB is where the lanes begin (131,072 cells of 64 B): just below, just above, a
+# few chunks more, and a 3D array with phi ghost planes
+@pytest.mark.parametrize("shape", [(315, 406, 1), (316, 406, 1), (400, 500, 1), (60, 70, 40)])
+def test_state_round_trip(shape, hc):
+    pr = hc.torus_problem(*shape)
+    ctx = hc.Context(pr)
+    rng = np.random.default_rng(1)
+    p = rng.standard_normal(pr.shape + (8,))
+    fl = rng.integers(-100, 100, pr.shape).astype(np.int8)
+    if shape[2] > 1:  # the phi ghosts come back as periodic copies
+        for a in (p, fl):
+            a[0], a[-1] = a[-2], a[1]
+    ctx.put_prims(p, fl)
+    q, gl = ctx.get_prims(with_flags=True)
+    assert np.array_equal(p, q) and np.array_equal(fl, gl)
+    ctx.close()
+
+
+def test_contexts_in_threads(hc):
+    """one thread holds the lanes, the others copy plainly"""
+    pr = hc.torus_problem(420, 400, 1)
+    bad = []
+
+    def work(seed):
+        ctx = hc.Context(pr)
+        for k in range(4):
+            p = np.random.default_rng([seed, k]).standard_normal(pr.shape + (8,))
+            ctx.put_prims(p)
+            if not np.array_equal(ctx.get_prims(), p):
+                bad.append((seed, k))
+        ctx.close()
+    ts = [threading.Thread(target=work, args=(s,)) for s in range(4)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad
+
+
+@pytest.mark.parametrize("n", [1, 127, 2048, 2049, 16 * 2048 + 1, 170001])
+def test_batch_inversion_at_chunk_edges(n, hc):
+    """every zone as it comes out alone or in any other split of the batch"""
+    pr = hc.torus_problem(32, 32, 1)
+    g = pr.geometry
+    rng = np.random.default_rng(n)
+    m = 500
+    i, j = rng.integers(2, 34, m), rng.integers(2, 34, m)
+    gcov, gcon = g["gcov"][i, j, 3].reshape(m, 16), g["gcon"][i, j, 3].reshape(m, 16)
+    gdet = g["gdet"][i, j, 3]
+    prim = np.zeros((m, 8))
+    prim[:, 0], prim[:, 1] = 10. ** rng.uniform(-4, 0, m), 10. ** rng.uniform(-6, -2, m)
+    U = np.zeros((m, 8))
+    U[:, 0] = prim[:, 0] * gdet
+    U[:, 1] = -prim[:, 1] * gdet
+    U[:, 5:8] = 1e-3 * rng.standard_normal((m, 3))
+    ref = prim.copy()
+    ret = np.concatenate([hc.utoprim_2d_batch(U[k:k + 100], gcov[k:k + 100], gcon[k:k + 100], gdet[k:k + 100],
+                                              ref[k:k + 100], 4. / 3.) for k in range(0, m, 100)])
+    t = np.arange(n) % m
+    out = prim[t].copy()
+    got = hc.utoprim_2d_batch(U[t], gcov[t], gcon[t], gdet[t], out, 4. / 3.)
+    assert np.array_equal(got, ret[t])
+    assert np.array_equal(out, ref[t], equal_nan=True)
