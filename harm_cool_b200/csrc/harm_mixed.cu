@@ -8,7 +8,7 @@
 #define HARM_FLUX_MINB 8   // 64 registers
 #endif
 #ifndef HARM_CONS_MINB
-#define HARM_CONS_MINB 5   // 102 registers
+#define HARM_CONS_MINB 4   // 128 registers: update of 192x192x64 444 -> 426 us, 5 and 6 spill
 #endif
 #ifndef HARM_INV_MINB
 #define HARM_INV_MINB 4    // 128 registers

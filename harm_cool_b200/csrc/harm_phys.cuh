@@ -326,9 +326,16 @@ __device__ __forceinline__ int conn_slot(int k, int a, int b)
   return k * 10 + pair;
 }
 
-template <class R>
+// a point's connection entries: conn planes in memory
+struct ConnPlanes {
+  const double *conn;  // conn + gi
+  long ng;
+  __device__ __forceinline__ double operator()(int slot) const { return __ldg(conn + slot * ng); }
+};
+
+template <class R, class Conn>
 __device__ __forceinline__ void source_of_state(double gam, const R *pb, const StateT<R> &s, const Geo &q,
-                                                const double *__restrict__ conn, long ng, long gi, R *dU)
+                                                const Conn &conn, R *dU)
 {
   R mhd[4][4];
 #pragma unroll
@@ -339,10 +346,10 @@ __device__ __forceinline__ void source_of_state(double gam, const R *pb, const S
   for (int j = 0; j < 4; j++)
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      dU[UU] += mhd[j][k] * __ldg(conn + conn_slot(k, 0, j) * ng + gi);
-      dU[U1] += mhd[j][k] * __ldg(conn + conn_slot(k, 1, j) * ng + gi);
-      dU[U2] += mhd[j][k] * __ldg(conn + conn_slot(k, 2, j) * ng + gi);
-      dU[U3] += mhd[j][k] * __ldg(conn + conn_slot(k, 3, j) * ng + gi);
+      dU[UU] += mhd[j][k] * conn(conn_slot(k, 0, j));
+      dU[U1] += mhd[j][k] * conn(conn_slot(k, 1, j));
+      dU[U2] += mhd[j][k] * conn(conn_slot(k, 2, j));
+      dU[U3] += mhd[j][k] * conn(conn_slot(k, 3, j));
     }
 #pragma unroll
   for (int k = 0; k < 8; k++) dU[k] *= q.g;

@@ -188,9 +188,11 @@ constexpr float F32_NEWT_TOL = 1.e-5f;
 
 // source() (phys.c:165-207) in float: dU_nu = sqrt(-g) T^kappa_lambda
 // Gamma^lambda_{nu kappa}, on an FP32 copy of the connection (stored as
-// [k][min(nu,j)][max(nu,j)] like the FP64 planes); used away from the horizon
-__device__ __forceinline__ void source_f(float gam, const float *pr, const GeoF &q, const float *__restrict__ conn,
-                                         long ng, long gi, double *dU, int *fail)
+// [k][min(nu,j)][max(nu,j)] like the FP64 planes, conn(slot)); used away from the
+// horizon
+template <class Conn>
+__device__ __forceinline__ void source_f(float gam, const float *pr, const GeoF &q, const Conn &conn, double *dU,
+                                         int *fail)
 {
   StateF s;
   get_state_f(pr, q, s, fail);
@@ -209,7 +211,7 @@ __device__ __forceinline__ void source_f(float gam, const float *pr, const GeoF 
       for (int nu = 0; nu < 4; nu++) {
         const int lo = nu < j ? nu : j, hi = nu < j ? j : nu;
         const int pair = lo == 0 ? hi : lo == 1 ? 3 + hi : lo == 2 ? 5 + hi : 9;
-        acc[nu] += t * __ldg(conn + (long)(k * 10 + pair) * ng + gi);
+        acc[nu] += t * conn(k * 10 + pair);
       }
     }
 #pragma unroll

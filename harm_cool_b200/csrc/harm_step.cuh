@@ -491,14 +491,6 @@ __device__ __forceinline__ void flux_update(const Flux &FX, const Emf &emf, int 
   }
 }
 
-__device__ void source(double gam, const double *pb, const Geo &q, const double *__restrict__ conn, long ng, long gi,
-                       double *dU, int *fail)
-{
-  State s;
-  get_state(pb, q, s, fail);
-  source_of_state(gam, pb, s, q, conn, ng, gi, dU);
-}
-
 // What the update of a zone reads besides the state and the fluxes.
 struct ZoneData {
   const double *geo, *conn;
@@ -506,65 +498,194 @@ struct ZoneData {
   const double *floors, *katm;
 };
 
+// A block's zones in shared memory: 32 points of the (r, theta) grid, numbered row by
+// row, on PL phi planes.  The points' metric and connection are shared by the
+// planes; everything comes in one round trip to L2, asynchronously.
+template <bool FULL, int PL>
+struct ZoneShared {
+  double conn[40][32];           // (mixed, away from the horizon: floats, in the slots' low halves)
+  double geo[GEO_N][32];
+  double pb[8][PL][32];
+  double pi[FULL ? 8 : 1][PL][32];  // the predictor advances from pi == pb
+#if HARM_STEP_MIXED
+  float geo32[11][32];
+#endif
+};
+
+// Where the update takes a zone's operands from: the staged block (3D), or the planes
+// in memory (2D, where no other plane shares a point's 61 metric and connection
+// entries and staging them only delays the first use: 128x128 update 28.4 us
+// staged, 25.6 direct).
+struct ConnShared {
+  const double *c;  // the point's first entry
+  __device__ __forceinline__ double operator()(int slot) const { return c[slot * 32]; }
+};
+template <bool FULL, int PL>
+struct StagedZone {
+  const ZoneShared<FULL, PL> &S;
+  __device__ __forceinline__ double pb(int k) const { return S.pb[k][threadIdx.y][threadIdx.x]; }
+  __device__ __forceinline__ double pi(int k) const { return FULL ? S.pi[k][threadIdx.y][threadIdx.x] : pb(k); }
+  __device__ __forceinline__ ConnShared conn() const { return ConnShared{&S.conn[0][threadIdx.x]}; }
+  __device__ __forceinline__ void geo(Geo &q) const
+  {
+    const int x = threadIdx.x;
+    q.v00 = S.geo[0][x]; q.v01 = S.geo[1][x]; q.v03 = S.geo[2][x]; q.v11 = S.geo[3][x]; q.v13 = S.geo[4][x];
+    q.v22 = S.geo[5][x]; q.v33 = S.geo[6][x];
+    q.n00 = S.geo[7][x]; q.n01 = S.geo[8][x]; q.n03 = S.geo[9][x]; q.n10 = S.geo[10][x]; q.n11 = S.geo[11][x];
+    q.n13 = S.geo[12][x]; q.n22 = S.geo[13][x]; q.n30 = S.geo[14][x]; q.n31 = S.geo[15][x]; q.n33 = S.geo[16][x];
+    q.g = S.geo[17][x];
+    q.alpha = S.geo[18][x]; q.ialpha = S.geo[19][x]; q.ig = S.geo[20][x];
+  }
+#if HARM_STEP_MIXED
+  struct Conn32 {
+    const double *c;
+    __device__ __forceinline__ float operator()(int slot) const
+    {
+      return *reinterpret_cast<const float *>(c + slot * 32);
+    }
+  };
+  __device__ __forceinline__ Conn32 conn32() const { return Conn32{&S.conn[0][threadIdx.x]}; }
+  __device__ __forceinline__ void geo32(GeoF &q) const
+  {
+    const int x = threadIdx.x;
+    q.v00 = S.geo32[0][x]; q.v01 = S.geo32[1][x]; q.v03 = S.geo32[2][x]; q.v11 = S.geo32[3][x];
+    q.v13 = S.geo32[4][x]; q.v22 = S.geo32[5][x]; q.v33 = S.geo32[6][x];
+    q.n00 = S.geo32[7][x]; q.n01 = S.geo32[8][x]; q.n03 = S.geo32[9][x];
+    q.g = S.geo32[10][x];
+  }
+#endif
+};
+struct DirectZone {
+  const Grid &G;
+  const double *ppi, *ppb;
+  const ZoneData &Z;
+  long c, gi;
+  __device__ __forceinline__ double pb(int k) const { return __ldg(ppb + k * G.nc + c); }
+  __device__ __forceinline__ double pi(int k) const { return ppi[k * G.nc + c]; }
+  __device__ __forceinline__ ConnPlanes conn() const { return ConnPlanes{Z.conn + gi, G.ng}; }
+  __device__ __forceinline__ void geo(Geo &q) const { load_geo(geo_at(Z.geo, G, L_CENT), G.ng, gi, q); }
+#if HARM_STEP_MIXED
+  struct Conn32 {
+    const float *conn;
+    long ng;
+    __device__ __forceinline__ float operator()(int slot) const { return __ldg(conn + slot * ng); }
+  };
+  __device__ __forceinline__ Conn32 conn32() const { return Conn32{Z.conn32 + gi, G.ng}; }
+  __device__ __forceinline__ void geo32(GeoF &q) const
+  {
+    load_geo_f(Z.geo32 + (long)L_CENT * GEO_N * G.ng, G.ng, gi, q);
+  }
+#endif
+};
+#if HARM_STEP_MIXED
+// the entries of a point's FP32 metric that the source reads, as planes of geo32
+__device__ constexpr int source_plane(int e) { return e < 10 ? e : 17; }
+#endif
+
+// ok: the point is in the grid; in_plane: and so is this thread's plane
+template <bool FULL, int PL>
+__device__ __forceinline__ void stage_zone(const Grid &G, ZoneShared<FULL, PL> &S, const double *pi, const double *pb,
+                                           const ZoneData &Z, bool ok, bool in_plane, int h, int i, int j)
+{
+  const int x = threadIdx.x, y = threadIdx.y;
+  if (ok) {
+    const long gi = (long)i * G.sn2 + j;
+    const double *g = Z.geo + (long)L_CENT * GEO_N * G.ng + gi;
+#pragma unroll
+    for (int e = 0; e < GEO_N; e += PL)
+      if (e + y < GEO_N) __pipeline_memcpy_async(&S.geo[e + y][x], g + (e + y) * G.ng, 8);
+#if HARM_STEP_MIXED
+    if (i >= G.isrc32) {
+      const float *c = Z.conn32 + gi, *f = Z.geo32 + (long)L_CENT * GEO_N * G.ng + gi;
+#pragma unroll
+      for (int e = 0; e < 40; e += PL) __pipeline_memcpy_async(&S.conn[e + y][x], c + (e + y) * G.ng, 4);
+#pragma unroll
+      for (int e = 0; e < 11; e += PL)
+        if (e + y < 11) __pipeline_memcpy_async(&S.geo32[e + y][x], f + source_plane(e + y) * G.ng, 4);
+    } else
+#endif
+    {
+      const double *c = Z.conn + gi;
+#pragma unroll
+      for (int e = 0; e < 40; e += PL) __pipeline_memcpy_async(&S.conn[e + y][x], c + (e + y) * G.ng, 8);
+    }
+    if (in_plane) {
+      const long c = cidx(G, h, i, j);
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        __pipeline_memcpy_async(&S.pb[k][y][x], pb + k * G.nc + c, 8);
+        if (FULL) __pipeline_memcpy_async(&S.pi[k][y][x], pi + k * G.nc + c, 8);
+      }
+    }
+  }
+  __pipeline_commit();
+  __pipeline_wait_prior(0);
+  __syncthreads();
+}
+
 // U of zone (h, i, j) after the half step: flux_ct (step_ch.c:514-629,
 // 726-798), the flux boundary fixes (coord.c:264-324), source() (phys.c:165-207),
 // primtoU of pi and the flux divergence (step_ch.c:247-263).  The order of every
 // floating-point operation is the reference's.
-template <bool FULL, bool THREE_D, class Emf>
-__device__ __forceinline__ void cons_zone(const Grid &G, const double *__restrict__ pi, const double *__restrict__ pb,
-                                          const Flux &FX, const Emf &emf, const ZoneData &Z, const Geo &q, double Dt,
-                                          int h, int i, int j, double *U, int *fail)
+template <bool FULL, bool THREE_D, class Zone, class Emf>
+__device__ __forceinline__ void cons_zone(const Grid &G, const Zone &zone, const Flux &FX, const Emf &emf,
+                                          const Geo &q, double Dt, int h, int i, int j, double *U, int *fail)
 {
-  const long c = cidx(G, h, i, j);
-  const long gi = (long)i * G.sn2 + j;
   double dU[8];
+  double pz[8];
 #if HARM_STEP_MIXED
   if (i >= G.isrc32) {
     // away from the horizon: the connection source in float (harm_phys32.cuh)
     float pf32[8];
 #pragma unroll
-    for (int k = 0; k < 8; k++) pf32[k] = (float)__ldg(pb + k * G.nc + c);
+    for (int k = 0; k < 8; k++) pf32[k] = (float)zone.pb(k);
     GeoF qf;
-    load_geo_f(Z.geo32 + (long)L_CENT * GEO_N * G.ng, G.ng, gi, qf);
-    source_f((float)G.gam, pf32, qf, Z.conn32, G.ng, gi, dU, fail);
-    double pz[8];
+    zone.geo32(qf);
+    source_f((float)G.gam, pf32, qf, zone.conn32(), dU, fail);
 #pragma unroll
-    for (int k = 0; k < 8; k++) pz[k] = __ldg(pi + k * G.nc + c);
+    for (int k = 0; k < 8; k++) pz[k] = zone.pi(k);
     State s;
     get_state(pz, q, s, fail);
     primtoflux(G.gam, pz, s, 0, q.g, U);
   } else
 #endif
-  if (!FULL) {
-    // the predictor advances from pi == pb (advance(p, p, ...), step_ch.c:101):
-    // one state serves both source() and primtoU()
-    double pz[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) pz[k] = __ldg(pb + k * G.nc + c);
+  {
     State s;
-    get_state(pz, q, s, fail);
-    source_of_state(G.gam, pz, s, q, Z.conn, G.ng, gi, dU);
-    primtoflux(G.gam, pz, s, 0, q.g, U);
-  } else {
-    {
-      double pbz[8];
 #pragma unroll
-      for (int k = 0; k < 8; k++) pbz[k] = __ldg(pb + k * G.nc + c);
-      source(G.gam, pbz, q, Z.conn, G.ng, gi, dU, fail);
-    }
-    double pz[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) pz[k] = __ldg(pi + k * G.nc + c);
-    State s;
+    for (int k = 0; k < 8; k++) pz[k] = zone.pb(k);
     get_state(pz, q, s, fail);
+    source_of_state(G.gam, pz, s, q, zone.conn(), dU);
+    if (FULL) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) pz[k] = zone.pi(k);
+      get_state(pz, q, s, fail);
+    }  // the predictor (advance(p, p, ...), step_ch.c:101): one state serves both
     primtoflux(G.gam, pz, s, 0, q.g, U);
   }
   flux_update<THREE_D>(FX, emf, h, i, j, Dt, dU, U);
 }
 
+// The block of the update's first half: 32 points of the grid on four phi planes in
+// 3D, 128 points in 2D, numbered row by row.
+constexpr int ZONE_PLANES = 4;
+template <bool THREE_D>
+__device__ __forceinline__ bool zone_of_thread(const Grid &G, int &h, int &i, int &j)
+{
+  const int z = blockIdx.x * blockDim.x + threadIdx.x;
+  j = G.jstart + z % G.n2;
+  i = G.istart + z / G.n2;
+  h = THREE_D ? blockIdx.z * ZONE_PLANES + threadIdx.y : 0;
+  return i <= G.istop;
+}
+
 // Large grids take the update in two launches, so that each holds fewer
 // registers and more warps stay resident to cover FP64 latency: k_cons forms U
-// into Ub, k_invert inverts it.  Each block sweeps hb phi planes.
+// into Ub, k_invert inverts it.
+//
+// k_cons in 3D is bound by the latency of its loads: when each thread loaded its
+// zone's 61 metric and connection entries as it used them, 7.4 of 13 warps per issue
+// waited on memory.  Staged, once for four planes: update of 192x192x64 FP64 692 ->
+// 654 us, 288x256x256 5.54 -> 5.36 ms, 70x50x22 55 -> 49 us.
 template <bool FULL, bool THREE_D>
 __global__ void __launch_bounds__(128, HARM_CONS_MINB) k_cons(Grid G, const double *__restrict__ pi,
                                                               const double *__restrict__ pb,
@@ -572,25 +693,32 @@ __global__ void __launch_bounds__(128, HARM_CONS_MINB) k_cons(Grid G, const doub
                                                               const flux_t *__restrict__ F2,
                                                               const flux_t *__restrict__ F3, ZoneData Z,
                                                               const double *__restrict__ emf,
-                                                              double *__restrict__ Ub, int hb, DevScalars *sc)
+                                                              double *__restrict__ Ub, DevScalars *sc)
 {
   if (sc->halted) return;
-  const int j = G.jstart + blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = G.istart + blockIdx.y * blockDim.y + threadIdx.y;
-  if (i > G.istop || j > G.jstop) return;
+  int h, i, j, fail = 0;
+  const bool ok = zone_of_thread<THREE_D>(G, h, i, j), in = ok && h < G.n3;
   const double Dt = FULL ? sc->dt : 0.5 * sc->dt;
-  const int h0 = blockIdx.z * hb, h1 = min(G.n3, h0 + hb);
-  for (int h = h0; h < h1; h++) {
-    const long c = cidx(G, h, i, j);
-    int fail = 0;
-    Geo q;
-    load_geo(geo_at(Z.geo, G, L_CENT), G.ng, (long)i * G.sn2 + j, q);
-    double U[8];
-    cons_zone<FULL, THREE_D>(G, pi, pb, Flux{F1, F2, F3, G}, EmfPlanes{emf}, Z, q, Dt, h, i, j, U, &fail);
-#pragma unroll
-    for (int k = 0; k < 8; k++) Ub[k * G.nc + c] = U[k];
-    if (fail) record_fail(sc, fail, h + (THREE_D ? 1 : 0), i, j);
+  const long c = cidx(G, h, i, j);
+  const Flux FX{F1, F2, F3, G};
+  Geo q;
+  double U[8];
+  if (THREE_D) {
+    __shared__ ZoneShared<FULL, ZONE_PLANES> S;
+    stage_zone<FULL, ZONE_PLANES>(G, S, pi, pb, Z, ok, in, h, i, j);
+    if (!in) return;
+    const StagedZone<FULL, ZONE_PLANES> zone{S};
+    zone.geo(q);
+    cons_zone<FULL, THREE_D>(G, zone, FX, EmfPlanes{emf}, q, Dt, h, i, j, U, &fail);
+  } else {
+    if (!in) return;
+    const DirectZone zone{G, pi, pb, Z, c, (long)i * G.sn2 + j};
+    zone.geo(q);
+    cons_zone<FULL, THREE_D>(G, zone, FX, EmfPlanes{emf}, q, Dt, h, i, j, U, &fail);
   }
+#pragma unroll
+  for (int k = 0; k < 8; k++) Ub[k * G.nc + c] = U[k];
+  if (fail) record_fail(sc, fail, h + (THREE_D ? 1 : 0), i, j);
 }
 
 // the isentropic fall-backs (step_ch.c:277-300), kept out of line: most
@@ -730,25 +858,35 @@ __global__ void __launch_bounds__(128, HARM_UPD_MINB) k_update(Grid G, const dou
                                                                double *__restrict__ Ub, DevScalars *sc)
 {
   if (sc->halted) return;
-  const int f = blockIdx.x * 128 + threadIdx.x;
-  const int j = G.jstart + f % G.n2, i = G.istart + f / G.n2, h = blockIdx.z;
-  if (i > G.istop) return;
+  int h, i, j, fail = 0;
+  const bool ok = zone_of_thread<THREE_D>(G, h, i, j), in = ok && h < G.n3;
   const double Dt = FULL ? sc->dt : 0.5 * sc->dt;
   const long c = cidx(G, h, i, j);
-  int fail = 0;
-  Geo q;
-  load_geo(geo_at(Z.geo, G, L_CENT), G.ng, (long)i * G.sn2 + j, q);
-  double U[8], pz[8];
   const Flux FX{F1, F2, F3, G};
-  if (THREE_D) cons_zone<FULL, THREE_D>(G, pi, pb, FX, EmfPlanes{emf}, Z, q, Dt, h, i, j, U, &fail);
-  else cons_zone<FULL, THREE_D>(G, pi, pb, FX, EmfFaces{FX}, Z, q, Dt, h, i, j, U, &fail);
+  Geo q;
+  double U[8], pz[8];
+  if (THREE_D) {
+    __shared__ ZoneShared<FULL, ZONE_PLANES> S;
+    stage_zone<FULL, ZONE_PLANES>(G, S, pi, pb, Z, ok, in, h, i, j);
+    if (!in) return;
+    const StagedZone<FULL, ZONE_PLANES> zone{S};
+    zone.geo(q);
+    cons_zone<FULL, THREE_D>(G, zone, FX, EmfPlanes{emf}, q, Dt, h, i, j, U, &fail);
+#pragma unroll
+    for (int k = 0; k < 8; k++) pz[k] = zone.pi(k);
+  } else {
+    if (!in) return;
+    const DirectZone zone{G, pi, pb, Z, c, (long)i * G.sn2 + j};
+    zone.geo(q);
+    cons_zone<FULL, THREE_D>(G, zone, FX, EmfFaces{FX}, q, Dt, h, i, j, U, &fail);
+#pragma unroll
+    for (int k = 0; k < 8; k++) pz[k] = zone.pi(k);
+  }
   if (fail) record_fail(sc, fail, h + (THREE_D ? 1 : 0), i, j);
   if (REC) {
 #pragma unroll
     for (int k = 0; k < 8; k++) Ub[k * G.nc + c] = U[k];
   }
-#pragma unroll
-  for (int k = 0; k < 8; k++) pz[k] = pi[k * G.nc + c];
   invert_zone<REC, !THREE_D>(G, U, q, pz, Z, O, sc, FULL ? 1 : 0, h, i, j);
 }
 
@@ -789,27 +927,28 @@ void launch_update(Ctx *x, const double *pi, const double *pb, double *pf, doubl
   const dim3 eg(((G.n2 + 1) * (G.n1 + 1) + 127) / 128, 1, G.n3);
   if (G.n3 > 1) k_emf<true><<<eg, 128, 0, x->stream>>>(G, B.F1, B.F2, B.F3, x->emf, x->sc);
   else if (!fused) k_emf<false><<<eg, 128, 0, x->stream>>>(G, B.F1, B.F2, B.F3, x->emf, x->sc);
+  const dim3 cb = G.n3 > 1 ? dim3(32, ZONE_PLANES) : dim3(128);
+  const dim3 cg((G.n1 * G.n2 + cb.x - 1) / cb.x, 1, (G.n3 + ZONE_PLANES - 1) / ZONE_PLANES);
   if (fused) {
-    const dim3 ug((G.n1 * G.n2 + 127) / 128, 1, G.n3);
     if (G.n3 > 1)
-      k_update<FULL, true, false><<<ug, 128, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, O, nullptr, x->sc);
+      k_update<FULL, true, false><<<cg, cb, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, O, nullptr, x->sc);
 #if !HARM_STEP_MIXED
     else if (zrec)
-      k_update<FULL, false, true><<<ug, 128, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, O, Ub, x->sc);
+      k_update<FULL, false, true><<<cg, cb, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, O, Ub, x->sc);
 #endif
     else
-      k_update<FULL, false, false><<<ug, 128, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, O, nullptr, x->sc);
+      k_update<FULL, false, false><<<cg, cb, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, O, nullptr, x->sc);
     return;
   }
-  // phi planes a block sweeps: four, whose zones share the tile's geometry in L1,
+  // phi planes a block of k_invert sweeps: four, whose zones share the tile's geometry in L1,
   // where that still leaves eight blocks for every SM, one where it does not
   // (70x50x22: update 82 us with four, 55 with one)
   const int hb = zones >= 148L * 8 * 128 * 4 ? 4 : 1;
   const dim3 tile(x->tbx, x->tby);
   const dim3 zg((G.n2 + tile.x - 1) / tile.x, (G.n1 + tile.y - 1) / tile.y, (G.n3 + hb - 1) / hb);
   double *U = Ub ? Ub : x->Ubuf;
-  if (G.n3 > 1) k_cons<FULL, true><<<zg, tile, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, U, hb, x->sc);
-  else k_cons<FULL, false><<<zg, tile, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, U, hb, x->sc);
+  if (G.n3 > 1) k_cons<FULL, true><<<cg, cb, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, U, x->sc);
+  else k_cons<FULL, false><<<cg, cb, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, U, x->sc);
   if (G.n3 > 1) k_invert<false, false><<<zg, tile, 0, x->stream>>>(G, pi, U, Z, O, FULL ? 1 : 0, hb, x->sc);
 #if !HARM_STEP_MIXED
   else if (zrec) k_invert<true, true><<<zg, tile, 0, x->stream>>>(G, pi, U, Z, O, FULL ? 1 : 0, hb, x->sc);
