@@ -22,17 +22,23 @@
 // face.
 #define HARM_VARIANT cool
 #define HARM_STEP_MIXED 0
-// resident blocks of 128 threads per SM that the COOL_EOS kernels' register
-// budgets must allow (measured on a B200: 3 for the faces, 168 registers, is
-// 3 % faster than 1; the update kernels lose with more than 1)
+// Threads per block of the COOL_EOS kernels, and the resident blocks per SM that
+// their register budgets must allow (128 registers for the faces, 168 for the
+// update).  A zone's time varies with its solves, and a grid of 256x256 is under two
+// waves: small blocks and more of them resident even that out.  256x256 FP64 step:
+// 128 threads at 168 and 255 registers 2.03 ms, 64 threads at those 1.92, at these
+// 1.69; 97x75 mixed within 3 %.
+#ifndef HARM_COOL_THREADS
+#define HARM_COOL_THREADS 64
+#endif
 #ifndef HARM_COOL_FLUX_MINB
-#define HARM_COOL_FLUX_MINB 3
+#define HARM_COOL_FLUX_MINB 8
 #endif
 #ifndef HARM_COOL_CONS_MINB
-#define HARM_COOL_CONS_MINB 1
+#define HARM_COOL_CONS_MINB 6
 #endif
 #ifndef HARM_COOL_INV_MINB
-#define HARM_COOL_INV_MINB 1
+#define HARM_COOL_INV_MINB 6
 #endif
 #define HARM_FLUX_MINB 1
 #define HARM_CONS_MINB 1
@@ -133,14 +139,17 @@ __device__ __forceinline__ void reduce_dt(DevScalars *sc, int dir, double dtmin)
   if ((t & 31) == 0) red[t >> 5] = v;
   __syncthreads();
   if (t == 0) {
-    v = fmin(fmin(red[0], red[1]), fmin(red[2], red[3]));
+    const int nw = (blockDim.x * blockDim.y) >> 5;
+    for (int k = 1; k < nw; k++) v = fmin(v, red[k]);
     if (v < 1.e9) atomicMin(&sc->ndt_bits[dir - 1], (unsigned long long)__double_as_longlong(v));
   }
 }
 
+inline dim3 cool_tile() { return dim3(32, HARM_COOL_THREADS / 32); }
+
 // one thread per face; face ranges as k_flux's
 template <int DIR, bool FULL, bool F32>
-__global__ void __launch_bounds__(128, HARM_COOL_FLUX_MINB) k_flux_cool(Grid G, const double *__restrict__ pb, double *__restrict__ F,
+__global__ void __launch_bounds__(HARM_COOL_THREADS, HARM_COOL_FLUX_MINB) k_flux_cool(Grid G, const double *__restrict__ pb, double *__restrict__ F,
                                                    const double *__restrict__ geo, EosDev E, double *lastT,
                                                    DevScalars *sc)
 {
@@ -187,7 +196,7 @@ void launch_flux_cool_p(Ctx *x, const double *pb, bool rows)
           G, pb, x->F3, x->geo, E, x->lastT, x->sc);
     return;
   }
-  const dim3 b(x->tbx, x->tby);
+  const dim3 b = cool_tile();
   dim3 g1((G.n2 + 2 + b.x - 1) / b.x, (G.n1 + 1 + b.y - 1) / b.y, G.n3);
   dim3 g2((G.n2 + 1 + b.x - 1) / b.x, (G.n1 + 2 + b.y - 1) / b.y, G.n3);
   dim3 g3((G.n2 + 2 + b.x - 1) / b.x, (G.n1 + 2 + b.y - 1) / b.y, G.n3);
@@ -236,7 +245,7 @@ __device__ __noinline__ void source_cool(const EosDev &E, EosCursor &c, const do
 // precision): the source's and primtoU's pressures from the FP32 interpolation
 // (all else FP64, the accumulation of U included)
 template <bool FULL, bool THREE_D, bool F32>
-__global__ void __launch_bounds__(128, HARM_COOL_CONS_MINB) k_cons_cool(Grid G, const double *__restrict__ pi, const double *__restrict__ pb,
+__global__ void __launch_bounds__(HARM_COOL_THREADS, HARM_COOL_CONS_MINB) k_cons_cool(Grid G, const double *__restrict__ pi, const double *__restrict__ pb,
                                                    const double *__restrict__ F1, const double *__restrict__ F2,
                                                    const double *__restrict__ F3, const double *__restrict__ geo,
                                                    const double *__restrict__ conn, EosDev E, double *lastT,
@@ -295,7 +304,7 @@ __global__ void __launch_bounds__(128, HARM_COOL_CONS_MINB) k_cons_cool(Grid G, 
 // Utoprim_5d from the guess pi, no isentropic fall-backs under COOL_EOS; in 2D
 // (PUSH) the zone's ghost cells too
 template <bool PUSH>
-__global__ void __launch_bounds__(128, HARM_COOL_INV_MINB) k_invert_cool(Grid G, const double *__restrict__ pi,
+__global__ void __launch_bounds__(HARM_COOL_THREADS, HARM_COOL_INV_MINB) k_invert_cool(Grid G, const double *__restrict__ pi,
                                                      const double *__restrict__ Ub, ZoneOut O,
                                                      const double *__restrict__ geo,
                                                      const double *__restrict__ floors, EosDev E, double *lastT,
@@ -368,7 +377,7 @@ void launch_half(Ctx *x, const double *pi, const double *pb, double *pf, bool ro
 {
   const Grid &G = x->G;
   launch_flux_cool<FULL>(x, pb, rows);
-  const dim3 tile(x->tbx, x->tby);
+  const dim3 tile = cool_tile();
   const dim3 zg((G.n2 + tile.x - 1) / tile.x, (G.n1 + tile.y - 1) / tile.y, G.n3);
   launch_cons_cool<FULL>(x, pi, pb, zg, tile);
   launch_invert_cool(x, pi, pf, zg, tile, FULL ? 1 : 0);
@@ -523,7 +532,7 @@ int cool_time_kernels(Ctx *x, int reps, double *ms)
   cudaEvent_t ev[nev];
   for (auto &e : ev) CK(cudaEventCreate(&e));
   double acc[HARM_NKERNELS] = {0, 0, 0, 0, 0};
-  const dim3 tile(x->tbx, x->tby);
+  const dim3 tile = cool::cool_tile();
   const dim3 zg((G.n2 + tile.x - 1) / tile.x, (G.n1 + tile.y - 1) / tile.y, G.n3);
   for (int r = 0; r < reps; r++) {
     int e = 0, slot[nev];
