@@ -1092,57 +1092,88 @@ struct DevBuf {
   }
 };
 
-static int run_adjoint(Ctx *x, int nsteps, int every, double *J, double *grad, double *ms)
+// What a run of the adjoint needs besides the context: device buffers, streams,
+// events and the captured graphs of a step and of a segment's recording and
+// reversal.  Kept in the context for the next call with the same step counts (an
+// optimisation's iterations): making and freeing it, and setting the stack limit
+// that the driver sizes for each kernel by itself, took 13 of a 31.4 ms call at
+// 192x192, 50 steps, which is 18.4 ms now.  Freed with the context, by a call with other counts, and at the end of a
+// call where it holds more than KEEP_BYTES.
+constexpr size_t KEEP_BYTES = 2u << 30;
+
+struct Graph {
+  cudaGraphExec_t e = nullptr;
+  ~Graph() { if (e) cudaGraphExecDestroy(e); }
+};
+
+struct Work {
+  int nsteps = 0, every = 0, tbx = 0, tby = 0;  // what the graphs were captured for
+  size_t bytes = 0;
+  DevBuf B;
+  double *ck = nullptr, *pend = nullptr, *lam = nullptr, *W = nullptr, *vbuf = nullptr;
+  DevScalars *cks = nullptr, *scall = nullptr, *recs[2] = {};
+  double *recp[2] = {}, *recd[2] = {};
+  signed char *recf[2] = {}, *Wf = nullptr, *kinds = nullptr;
+  int *recn[2] = {}, *list = nullptr, *err = nullptr;
+  AdjScalars *as = nullptr;
+  std::vector<StepRec> rec[2];
+  cudaStream_t rs = nullptr, fs = nullptr;
+  // timing; forward done; records ready; reverse done
+  cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr, efwd = nullptr, erec[2] = {}, erev[2] = {};
+  cudaEvent_t efork[2] = {}, ejoin[2] = {};  // the two face directions, side by side
+  cudaEvent_t ecf = nullptr, ecj = nullptr;  // the corrector's update and source, side by side
+  Graph gstep, grec[2], grev[2];
+
+  template <class T>
+  T *get(size_t n)
+  {
+    bytes += n * sizeof(T);
+    return B.get<T>(n);
+  }
+  ~Work()
+  {
+    for (cudaEvent_t v : {e0, e1, e2, efwd, erec[0], erec[1], erev[0], erev[1], efork[0], efork[1], ejoin[0], ejoin[1],
+                          ecf, ecj})
+      if (v) cudaEventDestroy(v);
+    if (rs) cudaStreamDestroy(rs);
+    if (fs) cudaStreamDestroy(fs);
+  }
+  int init(const Grid &G, int n, int ev);
+};
+
+int Work::init(const Grid &G, int n, int ev)
 {
-  const Grid &G = x->G;
+  nsteps = n;
+  every = ev;
   const size_t nc = (size_t)G.nc, pl = 8 * nc;
-  // the dual-number kernels keep up to ~2.3 KB per thread in local memory
-  size_t stack = 0;
-  CK(cudaDeviceGetLimit(&stack, cudaLimitStackSize));
-  if (stack < 4096) CK(cudaDeviceSetLimit(cudaLimitStackSize, 4096));
-  // the caller's stack limit again on every return (after B's buffers are freed)
-  struct RestoreStack {
-    size_t s;
-    bool on;
-    ~RestoreStack()
-    {
-      if (on) cudaDeviceSetLimit(cudaLimitStackSize, s);
-    }
-  } restore_stack{stack, stack < 4096};
   const int nseg = (nsteps + every - 1) / every;
   const int nrec = every < nsteps ? every : nsteps;
-  DevBuf B;
   // checkpoints; per-step records of a segment, twice (segments alternate
   // between the two sets, so one is recomputed while the other is reversed);
   // the run state of every step; the adjoint state
-  double *ck = B.get<double>(pl * nseg);
-  DevScalars *cks = B.get<DevScalars>(nseg + 1);
-  double *pend = B.get<double>(pl);
-  DevScalars *scall = B.get<DevScalars>(2 * (size_t)nsteps);
-  double *recp[2], *recd[2];
-  signed char *recf[2];
-  DevScalars *recs[2];
-  int *recn[2];
+  ck = get<double>(pl * nseg);
+  cks = get<DevScalars>(nseg + 1);
+  pend = get<double>(pl);
+  scall = get<DevScalars>(2 * (size_t)nsteps);
   for (int b = 0; b < 2; b++) {
-    recp[b] = B.get<double>(pl * (nrec + 1));
-    recd[b] = B.get<double>((size_t)nrec * (7 * pl + 4 * nc));
-    recf[b] = B.get<signed char>((size_t)nrec * 4 * nc);
-    recs[b] = B.get<DevScalars>((size_t)nrec * 2);
-    recn[b] = B.get<int>((size_t)nrec * 2);
+    recp[b] = get<double>(pl * (nrec + 1));
+    recd[b] = get<double>((size_t)nrec * (7 * pl + 4 * nc));
+    recf[b] = get<signed char>((size_t)nrec * 4 * nc);
+    recs[b] = get<DevScalars>((size_t)nrec * 2);
+    recn[b] = get<int>((size_t)nrec * 2);
     if (!recp[b] || !recd[b] || !recf[b] || !recs[b] || !recn[b])
       return fail_with(HARM_E_CUDA, "device memory for the adjoint");
   }
-  double *lam = B.get<double>(6 * pl);  // next, cur, ph, U, F1, F2
-  double *W = B.get<double>(pl);
-  signed char *Wf = B.get<signed char>(nc);
-  int *list = B.get<int>(FAIL_CAP);
-  double *vbuf = B.get<double>((size_t)FAIL_CAP * 8);
-  signed char *kinds = B.get<signed char>(FAIL_CAP);
-  int *err = B.get<int>(1);
-  AdjScalars *as = B.get<AdjScalars>(1);
+  lam = get<double>(6 * pl);  // next, cur, ph, U, F1, F2
+  W = get<double>(pl);
+  Wf = get<signed char>(nc);
+  list = get<int>(FAIL_CAP);
+  vbuf = get<double>((size_t)FAIL_CAP * 8);
+  kinds = get<signed char>(FAIL_CAP);
+  err = get<int>(1);
+  as = get<AdjScalars>(1);
   if (!ck || !cks || !pend || !scall || !lam || !W || !Wf || !list || !vbuf || !kinds || !err || !as)
     return fail_with(HARM_E_CUDA, "device memory for the adjoint");
-  std::vector<StepRec> rec[2];
   for (int b = 0; b < 2; b++) {
     rec[b].resize(nrec);
     for (int r = 0; r < nrec; r++) {
@@ -1157,41 +1188,37 @@ static int run_adjoint(Ctx *x, int nsteps, int every, double *J, double *grad, d
       s.nfail[0] = recn[b] + 2 * r; s.nfail[1] = recn[b] + 2 * r + 1;
     }
   }
+  CK(cudaStreamCreateWithFlags(&rs, cudaStreamNonBlocking));
+  CK(cudaStreamCreateWithFlags(&fs, cudaStreamNonBlocking));
+  for (cudaEvent_t *e : {&e0, &e1, &e2}) CK(cudaEventCreate(e));
+  for (cudaEvent_t *e :
+       {&efwd, &erec[0], &erec[1], &erev[0], &erev[1], &efork[0], &efork[1], &ejoin[0], &ejoin[1], &ecf, &ecj})
+    CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  return HARM_OK;
+}
+
+static int run_adjoint(Ctx *x, Work &w, double *J, double *grad, double *ms)
+{
+  const Grid &G = x->G;
+  const size_t nc = (size_t)G.nc, pl = 8 * nc;
+  const int nsteps = w.nsteps, every = w.every;
+  const int nseg = (nsteps + every - 1) / every;
+  double *const ck = w.ck, *const pend = w.pend, *const lam = w.lam, *const W = w.W, *const vbuf = w.vbuf;
+  DevScalars *const cks = w.cks, *const scall = w.scall;
+  DevScalars *const *recs = w.recs;
+  double *const *recp = w.recp;
+  signed char *const Wf = w.Wf, *const kinds = w.kinds;
+  int *const list = w.list, *const err = w.err;
+  AdjScalars *const as = w.as;
+  std::vector<StepRec> *const rec = w.rec;
   // the adjoint of the state after the step being undone (A) and before it (B)
   double *const A = lam, *const Bl = lam + pl, *lh = lam + 2 * pl, *lU = lam + 3 * pl, *lF1 = lam + 4 * pl,
                 *lF2 = lam + 5 * pl;
   // the context's stream runs the forward pass and the recomputation, rs the
   // reverse sweep
-  cudaStream_t st = x->stream, rs = nullptr, fs = nullptr;
-  CK(cudaStreamCreateWithFlags(&rs, cudaStreamNonBlocking));
-  cudaEvent_t e0, e1, e2, efwd, erec[2], erev[2];  // timing; forward done; records ready; reverse done
-  cudaEvent_t efork[2], ejoin[2];                   // the two face directions, side by side
-  cudaEvent_t ecf, ecj;                             // the corrector's update and source, side by side
-  struct Guard {
-    cudaStream_t s, f;
-    std::vector<cudaEvent_t> e;
-    ~Guard()
-    {
-      for (cudaEvent_t v : e) cudaEventDestroy(v);
-      if (s) cudaStreamDestroy(s);
-      if (f) cudaStreamDestroy(f);
-    }
-  } guard{rs, nullptr, {}};
-  CK(cudaStreamCreateWithFlags(&fs, cudaStreamNonBlocking));
-  guard.f = fs;
-  for (cudaEvent_t *e : {&e0, &e1, &e2}) {
-    CK(cudaEventCreate(e));
-    guard.e.push_back(*e);
-  }
-  for (cudaEvent_t *e :
-       {&efwd, &erec[0], &erec[1], &erev[0], &erev[1], &efork[0], &efork[1], &ejoin[0], &ejoin[1], &ecf, &ecj}) {
-    CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-    guard.e.push_back(*e);
-  }
-  struct Graph {
-    cudaGraphExec_t e = nullptr;
-    ~Graph() { if (e) cudaGraphExecDestroy(e); }
-  };
+  const cudaStream_t st = x->stream, rs = w.rs, fs = w.fs;
+  const cudaEvent_t e0 = w.e0, e1 = w.e1, e2 = w.e2, efwd = w.efwd, ecf = w.ecf, ecj = w.ecj;
+  const cudaEvent_t *erec = w.erec, *erev = w.erev, *efork = w.efork, *ejoin = w.ejoin;
   auto capture = [&](Graph &g, auto &&body) -> int {
     cudaGraph_t gr;
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -1199,6 +1226,10 @@ static int run_adjoint(Ctx *x, int nsteps, int every, double *J, double *grad, d
     cudaError_t e = cudaStreamEndCapture(st, &gr);
     if (rc) return rc;
     if (e != cudaSuccess) return fail_with(HARM_E_CUDA, std::string("capture: ") + cudaGetErrorString(e));
+    if (g.e) {
+      cudaGraphExecDestroy(g.e);
+      g.e = nullptr;
+    }
     e = cudaGraphInstantiate(&g.e, gr, 0);
     cudaGraphDestroy(gr);
     if (e != cudaSuccess) return fail_with(HARM_E_CUDA, std::string("instantiate: ") + cudaGetErrorString(e));
@@ -1289,16 +1320,22 @@ static int run_adjoint(Ctx *x, int nsteps, int every, double *J, double *grad, d
   CK(cudaMemsetAsync(as, 0, sizeof(AdjScalars), st));
   CK(cudaMemsetAsync(lam, 0, 6 * pb, st));
   const int last0 = (nseg - 1) * every, lastlen = nsteps - last0, blast = (nseg - 1) & 1;
-  Graph gstep, grec[2], grev[2];
-  int rc = capture(gstep, [&] { return exact::launch_step(x); });
-  if (rc) return rc;
-  for (int b = 0; b < 2; b++) {
-    if (nseg > 1) {
-      rc = capture(grec[b], [&] { return record(b, every); });
+  Graph &gstep = w.gstep, *const grec = w.grec, *const grev = w.grev;
+  int rc = HARM_OK;
+  if (!gstep.e || w.tbx != x->tbx || w.tby != x->tby) {
+    w.tbx = 0;  // captured only once all of it is
+    rc = capture(gstep, [&] { return exact::launch_step(x); });
+    if (rc) return rc;
+    for (int b = 0; b < 2; b++) {
+      if (nseg > 1) {
+        rc = capture(grec[b], [&] { return record(b, every); });
+        if (rc) return rc;
+      }
+      rc = capture(grev[b], [&] { return reverse(b, every, st); });
       if (rc) return rc;
     }
-    rc = capture(grev[b], [&] { return reverse(b, every, st); });
-    if (rc) return rc;
+    w.tbx = x->tbx;
+    w.tby = x->tby;
   }
   // the run state recorded with segment seg's steps, kept for the checks at the end
   auto keep_scalars = [&](int seg, int len) -> int {
@@ -1395,6 +1432,12 @@ static int run_adjoint(Ctx *x, int nsteps, int every, double *J, double *grad, d
   return HARM_OK;
 }
 
+static void free_work(Ctx *x)
+{
+  delete (Work *)x->adj;
+  x->adj = nullptr;
+}
+
 }  // namespace adj
 }  // namespace harm
 
@@ -1409,5 +1452,24 @@ extern "C" int harm_adjoint_mass_in(harm_ctx *h, int nsteps, int checkpoint_ever
   if (x->cool) return fail_with(HARM_E_ARG, "the adjoint covers the gamma-law step, not COOL_EOS");
   if (x->mode != HARM_FP64) return fail_with(HARM_E_ARG, "the adjoint runs on the FP64 step");
   if (x->ntr) return fail_with(HARM_E_ARG, "the adjoint's recomputation would move the tracers again: detach them");
-  return adj::run_adjoint(x, nsteps, checkpoint_every, J, grad, ms);
+  adj::Work *w = (adj::Work *)x->adj;
+  if (w && (w->nsteps != nsteps || w->every != checkpoint_every)) {
+    adj::free_work(x);
+    w = nullptr;
+  }
+  int rc = HARM_OK;
+  if (!w) {
+    x->adj = w = new adj::Work();
+    x->adj_free = adj::free_work;
+    rc = w->init(x->G, nsteps, checkpoint_every);
+  }
+  if (!rc) rc = adj::run_adjoint(x, *w, J, grad, ms);
+  if (rc) {
+    // work may be in flight on its streams
+    cudaStreamSynchronize(x->stream);
+    if (w->rs) cudaStreamSynchronize(w->rs);
+    if (w->fs) cudaStreamSynchronize(w->fs);
+  }
+  if (rc || w->bytes > adj::KEEP_BYTES) adj::free_work(x);
+  return rc;
 }

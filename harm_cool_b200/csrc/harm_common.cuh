@@ -94,6 +94,8 @@ struct Ctx {
   bool cool_seed;                // the next step may meet zones without a guess
   double *coolgeo;               // [2][ng] r and |r tan theta| at zone centres (diag.c:225-249)
   double *cooldiag;              // COOL_EOS diagnostics scratch (harm_diag.cu)
+  void *adj;                     // the adjoint's buffers and graphs, kept between calls (harm_adjoint.cu)
+  void (*adj_free)(Ctx *);
 };
 
 __device__ __forceinline__ void record_fail(DevScalars *sc, int code, int h, int i, int j)

@@ -1,0 +1,64 @@
+"""The adjoint keeps its buffers and graphs in the context between calls: a call
+after others with the same or other step counts, another state, another tile or
+steps in between gives what a fresh context gives (the gradient's sums are atomic,
+so to their rounding: 1e-12 of its norm)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def hc(harm_lib):
+    import harm_cool_b200
+    return harm_cool_b200
+
+
+def start(hc, pr):
+    ctx = hc.Context(pr)
+    ctx.init_torus()
+    ctx.run(20)
+    return ctx
+
+
+def test_repeated_calls_match_a_fresh_context(hc):
+    pr = hc.torus_problem(40, 36, 1)
+    a = start(hc, pr)
+    p, t = a.get_prims(), a.time()
+    calls = [(6, 2, 1.0, None), (6, 2, 1.0, None), (6, 2, 1.01, None), (5, 3, 1.0, None), (1, 1, 1.0, None),
+             (6, 2, 1.0, (64, 2)), (3, 10, 0.99, None)]
+    for nsteps, every, scale, tile in calls:
+        q = p.copy()
+        q[..., 0] *= scale
+        if tile:
+            a.set_tile(*tile)
+        got = []
+        for ctx in (a, start(hc, pr)):
+            ctx.put_prims(q)
+            ctx.set_time(*t)
+            J, g, _ = ctx.adjoint_mass_in(nsteps, every)
+            got.append((J, g, ctx.get_prims(), ctx.time()))
+        (J, g, e, s), (J1, g1, e1, s1) = got
+        assert abs(J - J1) <= 1e-14 * abs(J1) and s == s1
+        assert np.array_equal(e, e1)
+        assert np.linalg.norm(g - g1) <= 1e-12 * np.linalg.norm(g1), (nsteps, every, scale)
+        a.run(2)
+    a.close()
+
+
+def test_a_failed_call_leaves_the_next_one_whole(hc):
+    pr = hc.torus_problem(24, 24, 1)
+    a, b = start(hc, pr), start(hc, pr)
+    p, t = a.get_prims(), a.time()
+    a.adjoint_mass_in(3, 2)
+    a.put_prims(p)
+    a.set_time(pr.params.tf - 1e-3, 1e-3)  # the steps reach tf: refused
+    with pytest.raises(hc.HarmError):
+        a.adjoint_mass_in(3, 2)
+    out = []
+    for ctx in (a, b):
+        ctx.put_prims(p)
+        ctx.set_time(*t)
+        out.append(ctx.adjoint_mass_in(3, 2)[:2])
+    assert abs(out[0][0] - out[1][0]) <= 1e-13 * abs(out[1][0])
+    assert np.linalg.norm(out[0][1] - out[1][1]) <= 1e-12 * np.linalg.norm(out[1][1])
