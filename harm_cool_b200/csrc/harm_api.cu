@@ -214,95 +214,119 @@ __device__ void repair_list(const Grid &G, double *P, signed char *pflag, const 
 }
 
 // Device scratch of repair_plane, in buffers that hold nothing between the
-// inversion and the next half step's fluxes.
+// inversion and the next half step's fluxes.  old, R and lkind are laid out by lines,
+// so that a line's rows are neighbours in memory: zone (i, j) of a plane is at
+// line_slot(i, j).
 struct RepairScratch {
   double *S;          // [8][nc] repaired zones, committed at the end
-  double *R;          // [2][nc] what the ordered pass needs of each failed zone
+  double *old;        // [2][nc] density and energy before the repairs, by lines
+  double *R;          // [2][nc] what the ordered pass needs of each failed zone, by lines
   signed char *kind;  // [nc] stencil kind, or NO_REPAIR
+  signed char *lkind; // the same by lines
 };
 constexpr signed char NO_REPAIR = 3;
+
+// 2i + j modulo the row's length tells a row's zones apart
+__device__ __forceinline__ long line_slot(const Grid &G, int i, int j)
+{
+  return (long)((2 * i + j) % G.sn2) * G.sn1 + i;
+}
 
 // The density and energy of the failed zones of plane h in loop order, by one
 // block, one thread per row (thread 0 the ghost row below the first).  Row i
 // works on column j = w - 2i at line w: the zones it reads in row i-1 are then
 // done, those in row i+1 still untouched.  A row hands its last result to the
 // next through shared memory; old values and the zones' kinds and floors are
-// loaded PF columns ahead.
-__device__ void repair_lines(const Grid &G, const double *P, const RepairScratch &W, int h)
+// loaded PF lines ahead, coalesced (laid out by zones, where a line's rows lie a row
+// apart, a 256x192 torus took 920 us for the whole repair; so 755, most of it the
+// chain of a line's instructions and its barrier, some 700 lines long).  Leaves the last
+// resorts' averages in R.
+__device__ void repair_lines(const Grid &G, const RepairScratch &W, int h)
 {
   constexpr int PF = 4;
   __shared__ double ring[2][2][512];
   const int t = threadIdx.x, i = G.istart - 1 + t;
   const bool row = t <= G.n1;
-  const int jl = G.jstop + 1;  // last column handed on (a ghost)
-  const double *Pr = P + RHO * G.nc, *Pu = P + UU * G.nc;
-  const long c0 = row ? cidx(G, h, i, 0) : 0;
-  // pipelines over columns: own old value at j + 1, next row's at j + 1, kind and
-  // R at j
+  const int js = G.jstart - 2, jl = G.jstop + 1;  // columns handled; the last is a ghost, handed on
+  const long base = (long)h * G.ng;
+  const double *Or = W.old + base, *Ou = W.old + G.nc + base;
+  double *Ra = W.R + base, *Rb = W.R + G.nc + base;
+  const signed char *Kd = W.lkind + base;
+  const int w0 = 2 * (G.istart - 1) + js, w1 = 2 * G.istop + jl;
+  // line w of row i as a slot; lines ahead wrap
+  auto slot = [&](int m, int ahead, int r) {
+    int k = m + ahead;
+    if (k >= G.sn2) k -= G.sn2;
+    return (long)k * G.sn1 + r;
+  };
+  // pipelines over lines: own old value one column on, next row's there, kind and
+  // R here
   double or_[PF], ou[PF], nr[PF], nu[PF], ra[PF], rb[PF];
   signed char kd[PF];
-  auto fetch = [&](int j, double &a, double &b, double &c, double &d, double &e, double &f, signed char &k) {
-    const int jn = min(j + 1, G.sn2 - 1), jk = min(j, G.sn2 - 1);
-    a = Pr[c0 + jn];
-    b = Pu[c0 + jn];
-    c = Pr[c0 + G.sn2 + jn];
-    d = Pu[c0 + G.sn2 + jn];
-    k = t == 0 ? NO_REPAIR : W.kind[c0 + jk];
-    e = W.R[c0 + jk];
-    f = W.R[G.nc + c0 + jk];
+  auto fetch = [&](int m, int ahead, int s) {
+    const long a = slot(m, ahead + 1, i), b = slot(m, ahead + 3, i + 1), c = slot(m, ahead, i);
+    or_[s] = Or[a];
+    ou[s] = Ou[a];
+    nr[s] = Or[b];
+    nu[s] = Ou[b];
+    kd[s] = Kd[c];
+    ra[s] = Ra[c];
+    rb[s] = Rb[c];
   };
-  // columns run from js: two ahead of the first zone, to gather the row before's values
-  const int js = G.jstart - 2;
-  if (row)
-#pragma unroll
-    for (int q = 0; q < PF; q++) fetch(js + q, or_[q], ou[q], nr[q], nu[q], ra[q], rb[q], kd[q]);
-  double pr0 = 0., pu0 = 0., pr1 = 0., pu1 = 0.;                  // row i-1 (repaired), columns j-1, j
-  double sr = 0., su = 0.;                                        // own (repaired), column j-1
-  double cr = row ? Pr[c0 + js] : 0., cu = row ? Pu[c0 + js] : 0.;  // own (old), column j
-  double n0r = 0., n0u = 0., n1r = 0., n1u = 0.;                  // row i+1 (old), columns j-1, j
-  if (row) { n1r = Pr[c0 + G.sn2 + js]; n1u = Pu[c0 + G.sn2 + js]; }
-  const int w0 = 2 * (G.istart - 1) + js, w1 = 2 * G.istop + jl;
-  int q = 0;
-  for (int w = w0; w <= w1; w++) {
+  double pr0 = 0., pu0 = 0., pr1 = 0., pu1 = 0.;      // row i-1 (repaired), columns j-1, j
+  double sr = 0., su = 0.;                            // own (repaired), column j-1
+  double cr = 0., cu = 0.;                            // own (old), column j
+  double n0r = 0., n0u = 0., n1r = 0., n1u = 0.;      // row i+1 (old), columns j-1, j
+  auto one_line = [&](int w, int m, int s) {
     const int j = w - 2 * i;
-    if (row && j >= js && j <= jl) {
-      const double pr2 = t > 0 ? ring[(w - 1) & 1][0][t - 1] : 0., pu2 = t > 0 ? ring[(w - 1) & 1][1][t - 1] : 0.;
-      double xr, xu, yr, yu, a, b;
-      signed char kind;
-      // the pipeline's slot of this column, refilled PF columns ahead
-#pragma unroll
-      for (int s = 0; s < PF; s++)
-        if (s == q) {
-          xr = or_[s]; xu = ou[s]; yr = nr[s]; yu = nu[s]; a = ra[s]; b = rb[s]; kind = kd[s];
-          fetch(j + PF, or_[s], ou[s], nr[s], nu[s], ra[s], rb[s], kd[s]);
-        }
-      q = q + 1 == PF ? 0 : q + 1;
-      double vr = cr, vu = cu;
-      if (j >= G.jstart && j <= G.jstop) {
-        if (kind < 2) {
-          vr = a;
-          vu = b;
-        } else if (kind == 2) {
-          // repair_zone's last resort, then fixup1zone's floors for a zone at rest
-          vr = 0.5 * (0.25 * (xr + sr + pr1 + n1r) + 0.25 * (yr + n0r + pr2 + pr0));
-          vu = 0.5 * (0.25 * (xu + su + pu1 + n1u) + 0.25 * (yu + n0u + pu2 + pu0));
-          W.S[RHO * G.nc + c0 + j] = vr;
-          W.S[UU * G.nc + c0 + j] = vu;
-          const double uf = div_rn(vu, UORHOMAX, 1. / UORHOMAX);
-          const double rf = a < uf ? uf : a;
-          if (vr < rf) vr = rf;
-          if (vu < b) vu = b;
-        }
+    if (row && j >= js - PF && j <= jl) {
+      if (j == js - PF) {  // the row's first column, as far ahead
+        const long a = slot(m, PF, i), b = slot(m, PF + 2, i + 1);
+        cr = Or[a];
+        cu = Ou[a];
+        n1r = Or[b];
+        n1u = Ou[b];
       }
-      ring[w & 1][0][t] = vr;
-      ring[w & 1][1][t] = vu;
-      pr0 = pr1; pu0 = pu1; pr1 = pr2; pu1 = pu2;
-      n0r = n1r; n0u = n1u; n1r = yr; n1u = yu;
-      sr = vr; su = vu;
-      cr = xr; cu = xu;
+      if (j >= js) {
+        const double pr2 = t > 0 ? ring[(w - 1) & 1][0][t - 1] : 0., pu2 = t > 0 ? ring[(w - 1) & 1][1][t - 1] : 0.;
+        const double xr = or_[s], xu = ou[s], yr = nr[s], yu = nu[s];
+        double vr = cr, vu = cu;
+        if (t > 0 && j >= G.jstart && j <= G.jstop && kd[s] != NO_REPAIR) {
+          if (kd[s] < 2) {
+            vr = ra[s];
+            vu = rb[s];
+          } else {
+            // repair_zone's last resort, then fixup1zone's floors for a zone at rest
+            vr = 0.5 * (0.25 * (xr + sr + pr1 + n1r) + 0.25 * (yr + n0r + pr2 + pr0));
+            vu = 0.5 * (0.25 * (xu + su + pu1 + n1u) + 0.25 * (yu + n0u + pu2 + pu0));
+            const long c = slot(m, 0, i);
+            Ra[c] = vr;
+            Rb[c] = vu;
+            const double uf = div_rn(vu, UORHOMAX, 1. / UORHOMAX);
+            const double rf = ra[s] < uf ? uf : ra[s];
+            if (vr < rf) vr = rf;
+            if (vu < rb[s]) vu = rb[s];
+          }
+        }
+        ring[w & 1][0][t] = vr;
+        ring[w & 1][1][t] = vu;
+        pr0 = pr1; pu0 = pu1; pr1 = pr2; pu1 = pu2;
+        n0r = n1r; n0u = n1u; n1r = yr; n1u = yu;
+        sr = vr; su = vu;
+        cr = xr; cu = xu;
+      }
+      fetch(m, PF, s);  // line w + PF into the pipeline slot just read
     }
     __syncthreads();
-  }
+  };
+  // from PF lines before the first, which only fill the pipelines
+  int m = ((w0 - PF) % G.sn2 + G.sn2) % G.sn2;
+  for (int w = w0 - PF; w <= w1; w += PF)
+#pragma unroll
+    for (int s = 0; s < PF; s++) {
+      one_line(w + s, m, s);
+      m = m + 1 == G.sn2 ? 0 : m + 1;
+    }
 }
 
 // Many failures: plane h by one cluster.  Within a plane zone (i, j) depends
@@ -317,7 +341,7 @@ __device__ void repair_lines(const Grid &G, const double *P, const RepairScratch
 // that later zones' stencils read, and then the plane is repaired again the plain
 // way, one line after another.  (That plain way for every zone took 3.0 ms a half
 // step for a 256x192 torus with 49,000 failed zones; a step of an ensemble that
-// holds it went from 6.1 to 2.65 ms with this one.)
+// holds it went from 6.1 to 2.2 ms with this one.)
 template <class Cluster>
 __device__ void repair_plane(const Grid &G, Cluster &cl, double *P, signed char *pflag, const RepairScratch &W, int h,
                              const double *__restrict__ geo, const double *__restrict__ floors, DevScalars *sc)
@@ -333,8 +357,10 @@ __device__ void repair_plane(const Grid &G, Cluster &cl, double *P, signed char 
     int any = 0;
     for (long g = tid; g < G.ng; g += nt) {
       const int i = (int)(g / G.sn2), j = (int)(g % G.sn2);
-      const long c = base + g;
+      const long c = base + g, l = base + line_slot(G, i, j);
       signed char kind = NO_REPAIR;
+      W.old[l] = P[RHO * G.nc + c];
+      W.old[G.nc + l] = P[UU * G.nc + c];
       if (i >= G.istart && i <= G.istop && j >= G.jstart && j <= G.jstop && pflag[c] == 0) {
         kind = (signed char)stencil_kind(G, pflag, c);
         any = 1;
@@ -344,8 +370,8 @@ __device__ void repair_plane(const Grid &G, Cluster &cl, double *P, signed char 
           repair_zone(G, P, c, kind, v);
           if (fix_zone(G, geo, floors, i, j, v, &fail) || fail) *again0 = 1;
           for (int k = 0; k < 8; k++) W.S[k * G.nc + c] = v[k];
-          W.R[c] = v[RHO];
-          W.R[G.nc + c] = v[UU];
+          W.R[l] = v[RHO];
+          W.R[G.nc + l] = v[UU];
         } else {
           // the floors of a zone at rest with this field (fixup1zone)
           v[RHO] = v[UU] = v[U1] = v[U2] = v[U3] = 0.;
@@ -359,26 +385,28 @@ __device__ void repair_plane(const Grid &G, Cluster &cl, double *P, signed char 
           double rf = __ldg(floors + g), uf = __ldg(floors + G.ng + g);
           if (rf < bsq / BSQORHOMAX) rf = bsq / BSQORHOMAX;
           if (uf < bsq / BSQOUMAX) uf = bsq / BSQOUMAX;
-          W.R[c] = rf;
-          W.R[G.nc + c] = uf;
+          W.R[l] = rf;
+          W.R[G.nc + l] = uf;
         }
       }
-      W.kind[c] = kind;
+      W.kind[c] = W.lkind[l] = kind;
     }
     if (!__syncthreads_or(any) && cl.num_blocks() == 1) return;  // (3D) no failure in this plane
     cl.sync();
-    if (rank == 0) repair_lines(G, P, W, h);
+    if (rank == 0) repair_lines(G, W, h);
     cl.sync();
     for (long g = tid; g < G.ng; g += nt) {
       const long c = base + g;
       if (W.kind[c] != 2) continue;
+      const int i = (int)(g / G.sn2), j = (int)(g % G.sn2);
+      const long l = base + line_slot(G, i, j);
       double v[8];
-      v[RHO] = W.S[RHO * G.nc + c];
-      v[UU] = W.S[UU * G.nc + c];
+      v[RHO] = W.R[l];
+      v[UU] = W.R[G.nc + l];
       v[U1] = v[U2] = v[U3] = 0.;
       for (int k = B1; k <= B3; k++) v[k] = P[k * G.nc + c];
       int fail = 0;
-      if (fix_zone(G, geo, floors, (int)(g / G.sn2), (int)(g % G.sn2), v, &fail) || fail) *again0 = 1;
+      if (fix_zone(G, geo, floors, i, j, v, &fail) || fail) *again0 = 1;
       for (int k = 0; k < 8; k++) W.S[k * G.nc + c] = v[k];
     }
     cl.sync();
@@ -754,7 +782,8 @@ int launch_bound(Ctx *x, double *P)
 static int launch_repairs(Ctx *x, double *P, int slot, bool rebound)
 {
   const Grid &G = x->G;
-  const RepairScratch W{x->Ubuf, x->emf, (signed char *)(x->emf + 2 * G.nc)};
+  // (the theta fluxes' buffer is free once the update has read it)
+  const RepairScratch W{x->Ubuf, x->F2, x->emf, (signed char *)(x->emf + 2 * G.nc), (signed char *)(x->F2 + 2 * G.nc)};
   // the one plane of a 2D grid gets a cluster of eight blocks for its parallel
   // passes; the planes of a 3D grid, one block each, fill the GPU between them
   cudaLaunchConfig_t cfg = {};
