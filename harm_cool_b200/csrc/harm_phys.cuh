@@ -806,6 +806,53 @@ __device__ __forceinline__ R ut_calc_3vel(const R *v, const Geo &q)
   return sqrt(DD);
 }
 
+// fixup1zone()'s floors in the drift frame (fixup.c:230-350): the velocities of a
+// zone whose floors were applied in a strong field, from its state s, the primitives
+// pre before the floors and pv after.  Out of line, on copies its caller makes where
+// it calls: few zones take it, and arrays whose address a call takes live in memory
+// for the whole kernel.
+template <class R>
+static __device__ __noinline__ void fixup_drift(double gam, const Geo &q, const StateT<R> &s, const R &bsq, R trans,
+                                                const R *pre, R *pv)
+{
+  if (trans > 1.) trans = 1.;
+  R betapar = -s.bcon[0] / ((bsq + SMALL) * s.ucon[0]);
+  R betasq = betapar * betapar * bsq;
+  double betasqmax = 1. - 1. / (GAMMAMAX * GAMMAMAX);
+  if (betasq > betasqmax) betasq = betasqmax;
+  R gdr = 1. / sqrt(1 - betasq);
+  R ucondr[4], Bcon[4], Bcov[4], vcon[4], ucon[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) ucondr[k] = gdr * (s.ucon[k] + betapar * s.bcon[k]);
+  Bcon[0] = 0.;
+  Bcon[1] = pv[B1]; Bcon[2] = pv[B2]; Bcon[3] = pv[B3];
+  lower(Bcon, q, Bcov);
+  R udotB = dot4(s.ucon, Bcov);
+  R Bsq = dot4(Bcon, Bcov);
+  R B = sqrt(Bsq);
+  R wold = pre[RHO] + pre[UU] * gam;
+  R QdotB = udotB * wold * s.ucon[0];
+  R wnew = pv[RHO] + pv[UU] * gam;
+  R x = 2. * QdotB / (B * wnew * ucondr[0] + SMALL);
+  R vpar = x / (ucondr[0] * (1. + sqrt(1. + x * x)));
+  R one_over_ucondr_t = 1. / ucondr[0];
+  vcon[0] = 1.;
+#pragma unroll
+  for (int k = 1; k < 4; k++) vcon[k] = vpar * Bcon[k] / (B + SMALL) + ucondr[k] * one_over_ucondr_t;
+  R ut = ut_calc_3vel(vcon, q);
+#pragma unroll
+  for (int k = 0; k < 4; k++) ucon[k] = ut * vcon[k];
+  // ucon_to_utcon (phys.c:255-270)
+  const double alpha = q.alpha;
+  R gm = alpha * ucon[0];
+  double be[4] = {0., q.n01 * alpha * alpha, 0. * alpha * alpha, q.n03 * alpha * alpha};
+#pragma unroll
+  for (int k = 1; k < 4; k++) {
+    R utc = ucon[k] + gm * be[k] / alpha;
+    pv[k + UU] = utc * trans + pre[k + UU] * (1. - trans);
+  }
+}
+
 // returns true if the zone's pflag must be set to -33 (gamma failure)
 template <class R>
 static __device__ bool fixup1zone(double gam, double rho_floor, double uu_floor, const Geo &q, R *pv, int *fail)
@@ -825,42 +872,15 @@ static __device__ bool fixup1zone(double gam, double rho_floor, double uu_floor,
   if (pv[UU] < uuflr) { pv[UU] = uuflr; dofloor = true; }
   R trans;
   if (dofloor && (trans = 10. * bsq / (pv[RHO] < pv[UU] ? pv[RHO] : pv[UU]) - 1.) > 0.) {
-    if (trans > 1.) trans = 1.;
-    R betapar = -s.bcon[0] / ((bsq + SMALL) * s.ucon[0]);
-    R betasq = betapar * betapar * bsq;
-    double betasqmax = 1. - 1. / (GAMMAMAX * GAMMAMAX);
-    if (betasq > betasqmax) betasq = betasqmax;
-    R gdr = 1. / sqrt(1 - betasq);
-    R ucondr[4], Bcon[4], Bcov[4], vcon[4], ucon[4];
+    const Geo qc = q;
+    const StateT<R> sc = s;
+    const R bc = bsq;
+    R old[8], v[8];
 #pragma unroll
-    for (int k = 0; k < 4; k++) ucondr[k] = gdr * (s.ucon[k] + betapar * s.bcon[k]);
-    Bcon[0] = 0.;
-    Bcon[1] = pv[B1]; Bcon[2] = pv[B2]; Bcon[3] = pv[B3];
-    lower(Bcon, q, Bcov);
-    R udotB = dot4(s.ucon, Bcov);
-    R Bsq = dot4(Bcon, Bcov);
-    R B = sqrt(Bsq);
-    R wold = pre[RHO] + pre[UU] * gam;
-    R QdotB = udotB * wold * s.ucon[0];
-    R wnew = pv[RHO] + pv[UU] * gam;
-    R x = 2. * QdotB / (B * wnew * ucondr[0] + SMALL);
-    R vpar = x / (ucondr[0] * (1. + sqrt(1. + x * x)));
-    R one_over_ucondr_t = 1. / ucondr[0];
-    vcon[0] = 1.;
+    for (int k = 0; k < 8; k++) { old[k] = pre[k]; v[k] = pv[k]; }
+    fixup_drift(gam, qc, sc, bc, trans, old, v);
 #pragma unroll
-    for (int k = 1; k < 4; k++) vcon[k] = vpar * Bcon[k] / (B + SMALL) + ucondr[k] * one_over_ucondr_t;
-    R ut = ut_calc_3vel(vcon, q);
-#pragma unroll
-    for (int k = 0; k < 4; k++) ucon[k] = ut * vcon[k];
-    // ucon_to_utcon (phys.c:255-270)
-    const double alpha = q.alpha;
-    R gm = alpha * ucon[0];
-    double be[4] = {0., q.n01 * alpha * alpha, 0. * alpha * alpha, q.n03 * alpha * alpha};
-#pragma unroll
-    for (int k = 1; k < 4; k++) {
-      R utc = ucon[k] + gm * be[k] / alpha;
-      pv[k + UU] = utc * trans + pre[k + UU] * (1. - trans);
-    }
+    for (int k = U1; k <= U3; k++) pv[k] = v[k];
   }
   R gamma;
   if (gamma_calc(pv, q, gamma)) return true;

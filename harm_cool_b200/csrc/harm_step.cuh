@@ -723,12 +723,16 @@ __global__ void __launch_bounds__(128, HARM_CONS_MINB) k_cons(Grid G, const doub
 
 // the isentropic fall-backs (step_ch.c:277-300), kept out of line: most
 // zones never take them, and inlined they crowd the kernel's hot code out of
-// the instruction cache
+// the instruction cache; which: 1 or 2, the last one tried
 static __device__ __noinline__ int inversion_fallbacks(double gam, double kap, const double *U, const Geo &q,
-                                                       double *pz)
+                                                       double *pz, int *which)
 {
   int flag = utoprim<1>(gam, kap, U, q, pz);
-  if (flag) flag = utoprim<2>(gam, kap, U, q, pz);
+  *which = 1;
+  if (flag) {
+    flag = utoprim<2>(gam, kap, U, q, pz);
+    *which = 2;
+  }
   return flag;
 }
 
@@ -791,21 +795,24 @@ __device__ __forceinline__ void invert_zone(const Grid &G, const double *U, cons
   const long gi = (long)i * G.sn2 + j;
   int fail = 0;
   int flag = utoprim<0, (bool)HARM_STEP_MIXED>(G.gam, 0., U, q, pz);
+  int which = 0;
+  if (flag) {
+    // on copies made here: arrays whose address a call takes would live in memory for
+    // the whole kernel, the Newton solve's operands among them
+    double Uc[8], pc[8];
+    const Geo qc = q;
+    int w;
+#pragma unroll
+    for (int k = 0; k < 8; k++) { Uc[k] = U[k]; pc[k] = pz[k]; }
+    flag = inversion_fallbacks(G.gam, __ldg(Z.katm + i), Uc, qc, pc, &w);
+#pragma unroll
+    for (int k = 0; k < 8; k++) pz[k] = pc[k];
+    which = w;
+  }
   if (REC) {
-    int which = 0;
-    if (flag) {
-      which = 1;
-      flag = utoprim<1>(G.gam, __ldg(Z.katm + i), U, q, pz);
-      if (flag) {
-        which = 2;
-        flag = utoprim<2>(G.gam, __ldg(Z.katm + i), U, q, pz);
-      }
-    }
 #pragma unroll
     for (int k = 0; k < 8; k++) O.zrec[k * G.nc + c] = pz[k];
     O.wrec[c] = (signed char)(flag ? -1 : which);
-  } else if (flag) {
-    flag = inversion_fallbacks(G.gam, __ldg(Z.katm + i), U, q, pz);
   }
   signed char fl = (signed char)flag;
   if (fixup1zone(G.gam, __ldg(Z.floors + gi), __ldg(Z.floors + G.ng + gi), q, pz, &fail)) fl = -33;
@@ -815,8 +822,12 @@ __device__ __forceinline__ void invert_zone(const Grid &G, const double *U, cons
 #pragma unroll
   for (int k = 0; k < 8; k++) O.pf[k * G.nc + c] = pz[k];
   O.pflag[c] = fl;
-  if (PUSH && (i == G.istart || i == G.istop || j <= G.jstart + 1 || j >= G.jstop - 1))
-    push_ghosts(G, O, Z.geo, sc, i, j, pz, fl);
+  if (PUSH && (i == G.istart || i == G.istop || j <= G.jstart + 1 || j >= G.jstop - 1)) {
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = pz[k];
+    push_ghosts(G, O, Z.geo, sc, i, j, v, fl);
+  }
   if (fail) record_fail(sc, fail, h + (G.n3 > 1 ? 1 : 0), i, j);
 }
 
