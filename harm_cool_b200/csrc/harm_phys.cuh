@@ -365,10 +365,10 @@ __device__ __forceinline__ R slope_lim(int lim, R y1, R y2, R y3)
     Dqp = 2. * (y3 - y2);
     R Dqc = 0.5 * (y3 - y1);
     s = Dqm * Dqp;
-    if (s <= 0.) return R(0.);
-    if (fabs(Dqm) < fabs(Dqp) && fabs(Dqm) < fabs(Dqc)) return Dqm;
-    if (fabs(Dqp) < fabs(Dqc)) return Dqp;
-    return Dqc;
+    // selected, not branched: a warp's zones differ
+    const bool a = fabs(Dqm) < fabs(Dqp) && fabs(Dqm) < fabs(Dqc), b = fabs(Dqp) < fabs(Dqc);
+    const R m = a ? Dqm : b ? Dqp : Dqc;
+    return s <= 0. ? R(0.) : m;
   }
   Dqm = (y2 - y1);
   Dqp = (y3 - y2);

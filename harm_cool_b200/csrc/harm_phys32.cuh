@@ -146,10 +146,9 @@ __device__ __forceinline__ float slope_lim_f(int lim, float y1, float y2, float 
     Dqp = 2.f * (y3 - y2);
     const float Dqc = 0.5f * (y3 - y1);
     s = Dqm * Dqp;
-    if (s <= 0.f) return 0.f;
-    if (fabsf(Dqm) < fabsf(Dqp) && fabsf(Dqm) < fabsf(Dqc)) return Dqm;
-    if (fabsf(Dqp) < fabsf(Dqc)) return Dqp;
-    return Dqc;
+    const bool a = fabsf(Dqm) < fabsf(Dqp) && fabsf(Dqm) < fabsf(Dqc), b = fabsf(Dqp) < fabsf(Dqc);
+    const float m = a ? Dqm : b ? Dqp : Dqc;
+    return s <= 0.f ? 0.f : m;
   }
   Dqm = (y2 - y1);
   Dqp = (y3 - y2);

@@ -73,6 +73,8 @@ __host__ __device__ __forceinline__ int face_rows(const Grid &G) { return DIR ==
 // directions: FP64 825 -> 699 us (the split alone, without the staging, 893),
 // mixed 447 -> 428; 288x256x256 FP64 6.77 -> 5.62 ms; 128x128 (launch included)
 // 27.7 -> 14.2 us.  64 and 56 registers (8 and 9 blocks) spill again: 756, 810 us.
+// With div_rn's shorter last step 663 us (FP64), and with the limiter selected instead
+// of branched 623 and 406; 80 registers (6 blocks) 637.
 constexpr int FLUX_FACES = 64;
 
 #if HARM_STEP_MIXED
@@ -151,15 +153,19 @@ __device__ __forceinline__ double flux_block(const Grid &G, int fb, int h, const
   face_t p[8];
   if (calc) {
     const face_t half = side ? (face_t)-0.5 : (face_t)0.5;
+    auto states = [&](int lim) {
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const face_t a = (face_t)S.p[k][side][s], b = (face_t)S.p[k][side + 1][s], e = (face_t)S.p[k][side + 2][s];
+      for (int k = 0; k < 8; k++) {
+        const face_t a = (face_t)S.p[k][side][s], b = (face_t)S.p[k][side + 1][s], e = (face_t)S.p[k][side + 2][s];
 #if HARM_STEP_MIXED
-      p[k] = b + half * slope_lim_f(G.lim, a, b, e);
+        p[k] = b + half * slope_lim_f(lim, a, b, e);
 #else
-      p[k] = b + half * slope_lim(G.lim, a, b, e);
+        p[k] = b + half * slope_lim(lim, a, b, e);
 #endif
-    }
+      }
+    };
+    if (G.lim == 0) states(0);  // one test for the eight, not one each
+    else states(G.lim);
   }
   __syncthreads();  // the stencil's space takes the exchange
   if (calc) {
