@@ -182,7 +182,7 @@ struct StepRec {
   signed char *fl1[2];           // the flags after the first bound_prim, flipped: 0 a failed zone [nc]
   int *nfail[2];                 // the failed zones fixup_utoprim then met (device int)
   double *ph;                    // the predictor's final state
-  DevScalars *sc[2];             // the run state before k_finalize (the corrector's Courant minima) and after
+  DevScalars *sc[2];             // the run state before k_mass (the corrector's Courant minima) and after
 };
 
 // kernels shared by both precisions (harm_api.cu)

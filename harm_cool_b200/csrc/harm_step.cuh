@@ -1020,7 +1020,7 @@ int launch_step_rec(Ctx *x, const StepRec &r)
   cudaMemcpyAsync(r.ph, x->ph, 8 * (size_t)x->G.nc * sizeof(double), cudaMemcpyDeviceToDevice, x->stream);
   rc = launch_half_rec<true>(x, x->p, x->ph, x->p, r);
   if (rc) return rc;
-  // the corrector's Courant minima, before k_finalize resets them
+  // the corrector's Courant minima, before k_mass resets them
   cudaMemcpyAsync(r.sc[0], x->sc, sizeof(DevScalars), cudaMemcpyDeviceToDevice, x->stream);
   launch_mass(x, bufs(x).F1);
   cudaMemcpyAsync(r.sc[1], x->sc, sizeof(DevScalars), cudaMemcpyDeviceToDevice, x->stream);
