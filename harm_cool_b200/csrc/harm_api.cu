@@ -1073,11 +1073,24 @@ __global__ void k_set_mass(DevScalars *sc, double mass_in, double mass_out)
   sc->mass_in = mass_in;
   sc->mass_out = mass_out;
 }
+// the context's device current for a launch, the caller's again after it
+struct OnDevice {
+  int was = -1;
+  explicit OnDevice(int device)
+  {
+    if (cudaGetDevice(&was) != cudaSuccess || was == device || cudaSetDevice(device) != cudaSuccess) was = -1;
+  }
+  ~OnDevice()
+  {
+    if (was >= 0) cudaSetDevice(was);
+  }
+};
 }  // namespace harm
 
 extern "C" int harm_set_time(harm_ctx *h, double t, double dt)
 {
   if (!h) return fail_with(HARM_E_ARG, "null context");
+  OnDevice on(h->x.device);
   k_set_time<<<1, 1, 0, h->x.stream>>>(h->x.sc, t, dt);
   CK(cudaGetLastError());
   return HARM_OK;
@@ -1097,6 +1110,7 @@ extern "C" int harm_get_time(harm_ctx *h, double *t, double *dt)
 extern "C" int harm_set_mass(harm_ctx *h, double mass_in, double mass_out)
 {
   if (!h) return fail_with(HARM_E_ARG, "null context");
+  OnDevice on(h->x.device);
   k_set_mass<<<1, 1, 0, h->x.stream>>>(h->x.sc, mass_in, mass_out);
   CK(cudaGetLastError());
   return HARM_OK;
@@ -1770,6 +1784,17 @@ static int ensemble_graph(harm_ensemble *e)
   return HARM_OK;
 }
 
+// the members' own streams first: what was queued there (steps, uploads, a time set)
+// comes before the ensemble's steps
+static int ensemble_after_members(harm_ensemble *e)
+{
+  for (size_t k = 0; k < e->members.size(); k++) {
+    CK(cudaEventRecord(e->join[k], e->members[k]->stream));
+    CK(cudaStreamWaitEvent(e->stream, e->join[k], 0));
+  }
+  return HARM_OK;
+}
+
 static int ensemble_status(harm_ensemble *e)
 {
   CK(cudaStreamSynchronize(e->stream));
@@ -1784,6 +1809,7 @@ extern "C" int harm_ensemble_run(harm_ensemble *e, int nsteps)
 {
   if (!e || nsteps < 0) return fail_with(HARM_E_ARG, "bad argument");
   int rc = ensemble_graph(e);
+  if (!rc) rc = ensemble_after_members(e);
   if (rc) return rc;
   for (int s = 0; s < nsteps; s++) CK(cudaGraphLaunch(e->exec, e->stream));
   return ensemble_status(e);
@@ -1793,6 +1819,7 @@ extern "C" int harm_ensemble_run_timed(harm_ensemble *e, int nsteps, double *ms)
 {
   if (!e || !ms || nsteps < 0) return fail_with(HARM_E_ARG, "bad argument");
   int rc = ensemble_graph(e);
+  if (!rc) rc = ensemble_after_members(e);
   if (rc) return rc;
   EventPair ev;
   CK(cudaEventCreate(&ev.a));
