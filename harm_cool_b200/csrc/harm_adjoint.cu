@@ -1147,7 +1147,7 @@ int Work::init(const Grid &G, int n, int ev)
   every = ev;
   const size_t nc = (size_t)G.nc, pl = 8 * nc;
   const int nseg = (nsteps + every - 1) / every;
-  const int nrec = every < nsteps ? every : nsteps;
+  const int nrec = every;
   // checkpoints; per-step records of a segment, twice (segments alternate
   // between the two sets, so one is recomputed while the other is reversed);
   // the run state of every step; the adjoint state
@@ -1326,7 +1326,9 @@ static int run_adjoint(Ctx *x, Work &w, double *J, double *grad, double *ms)
     w.tbx = 0;  // captured only once all of it is
     rc = capture(gstep, [&] { return exact::launch_step(x); });
     if (rc) return rc;
-    for (int b = 0; b < 2; b++) {
+    // for the sets that some segment of `every` steps uses (a single segment is
+    // recorded as the forward pass goes)
+    for (int b = 0; b < 2 && b < nsteps / every; b++) {
       if (nseg > 1) {
         rc = capture(grec[b], [&] { return record(b, every); });
         if (rc) return rc;
@@ -1452,8 +1454,10 @@ extern "C" int harm_adjoint_mass_in(harm_ctx *h, int nsteps, int checkpoint_ever
   if (x->cool) return fail_with(HARM_E_ARG, "the adjoint covers the gamma-law step, not COOL_EOS");
   if (x->mode != HARM_FP64) return fail_with(HARM_E_ARG, "the adjoint runs on the FP64 step");
   if (x->ntr) return fail_with(HARM_E_ARG, "the adjoint's recomputation would move the tracers again: detach them");
+  // a segment holds no more steps than there are (the records of one are sized so)
+  const int every = checkpoint_every < nsteps ? checkpoint_every : nsteps;
   adj::Work *w = (adj::Work *)x->adj;
-  if (w && (w->nsteps != nsteps || w->every != checkpoint_every)) {
+  if (w && (w->nsteps != nsteps || w->every != every)) {
     adj::free_work(x);
     w = nullptr;
   }
@@ -1461,7 +1465,7 @@ extern "C" int harm_adjoint_mass_in(harm_ctx *h, int nsteps, int checkpoint_ever
   if (!w) {
     x->adj = w = new adj::Work();
     x->adj_free = adj::free_work;
-    rc = w->init(x->G, nsteps, checkpoint_every);
+    rc = w->init(x->G, nsteps, every);
   }
   if (!rc) rc = adj::run_adjoint(x, *w, J, grad, ms);
   if (rc) {

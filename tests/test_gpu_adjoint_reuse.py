@@ -62,3 +62,39 @@ def test_a_failed_call_leaves_the_next_one_whole(hc):
         out.append(ctx.adjoint_mass_in(3, 2)[:2])
     assert abs(out[0][0] - out[1][0]) <= 1e-13 * abs(out[1][0])
     assert np.linalg.norm(out[0][1] - out[1][1]) <= 1e-12 * np.linalg.norm(out[1][1])
+
+
+@pytest.mark.parametrize("nsteps", [1, 4])
+def test_checkpoints_farther_apart_than_the_steps(nsteps, hc):
+    """One segment, however far apart the checkpoints are asked for: what
+    checkpoint_every = nsteps gives."""
+    pr = hc.torus_problem(24, 24, 1)
+    ctx = start(hc, pr)
+    p, t = ctx.get_prims(), ctx.time()
+    out = []
+    for every in (nsteps, nsteps + 1, 1000, 2 ** 31 - 1):
+        ctx.put_prims(p)
+        ctx.set_time(*t)
+        out.append(ctx.adjoint_mass_in(nsteps, every)[:2])
+    for J, g in out[1:]:
+        assert abs(J - out[0][0]) <= 1e-14 * abs(out[0][0])
+        assert np.linalg.norm(g - out[0][1]) <= 1e-12 * np.linalg.norm(out[0][1])
+    ctx.close()
+
+
+@pytest.mark.parametrize("nsteps,every", [(5, 5), (7, 4), (8, 4), (13, 4)])
+def test_one_two_and_more_segments_agree(nsteps, every, hc):
+    """Full and short last segments in either set of records, against checkpoints at
+    every step (the gradient's sums are atomic: 1e-12 of its norm)."""
+    pr = hc.torus_problem(24, 24, 1)
+    ctx = start(hc, pr)
+    p, t = ctx.get_prims(), ctx.time()
+    out = []
+    for e in (1, every, every):
+        ctx.put_prims(p)
+        ctx.set_time(*t)
+        out.append(ctx.adjoint_mass_in(nsteps, e)[:2])
+    for J, g in out[1:]:
+        assert abs(J - out[0][0]) <= 1e-14 * abs(out[0][0])
+        assert np.linalg.norm(g - out[0][1]) <= 1e-12 * np.linalg.norm(out[0][1])
+    ctx.close()
