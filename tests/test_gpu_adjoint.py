@@ -81,6 +81,21 @@ def test_state_direction_against_central_difference(nsteps, every):
     assert abs(ad_ - fd) <= TOL * abs(fd), (ad_, fd)
 
 
+def test_state_direction_on_a_grid_whose_update_takes_several_launches():
+    """above 56,832 zones the recomputation records from k_cons and k_invert"""
+    ctx = _context(241, 240)
+    ctx.init_torus()
+    p0 = ctx.get_prims()
+    v = _smooth_direction(p0.shape, seed=3)
+    scale = np.array([np.abs(p0[..., k]).max() for k in range(8)])
+    v *= np.abs(p0) + 1e-3 * scale * (np.arange(8) >= 2)
+    J, lam, _ = ctx.adjoint_mass_in(3, 2)
+    assert J == _mass_in_from(ctx, p0, 3)
+    fd = (_mass_in_from(ctx, p0 + H * v, 3) - _mass_in_from(ctx, p0 - H * v, 3)) / (2 * H)
+    ad_ = float(np.sum(lam * v))
+    assert abs(ad_ - fd) <= TOL * abs(fd), (ad_, fd)
+
+
 def test_checkpoint_spacing_does_not_change_the_gradient():
     """one segment recorded on the forward pass (9), full segments of odd and
     even length replayed from graphs (3, 2, 4), partial last segments (2, 4)"""
