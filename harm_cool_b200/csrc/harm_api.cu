@@ -111,12 +111,15 @@ __global__ void k_bound(Grid G, double *P, signed char *pflag, const double *__r
 // the last-resort average reads every neighbour and so sees earlier repairs.
 // A half step's inversion writes the flags flipped and lists the failed zones
 // (k_fu_flip does both for flags that come from the host); k_repair repairs them.
-// For a few failures (up to FIX_LIST_MAX, about 2 us each in the worst case, against
-// some 100 us for a plane) one block sorts the list into loop order, precomputes the
-// stencil repairs in parallel and then replays the whole list in order on one
-// thread, recomputing any zone whose stencil choice changed or that needs the
-// last-resort average.  For more, each phi plane (a repair reads only its own
-// plane) is repaired by repair_plane.
+// Up to FIX_LIST_MAX failures go through one block, which sorts the list into loop
+// order, precomputes the stencil repairs in parallel and then replays the whole list in
+// order on one thread, recomputing any zone whose stencil choice changed or that needs
+// the last-resort average.  For more, each phi plane (a repair reads only its own
+// plane) is repaired by repair_plane.  The list takes 0.8 us a zone where failures lie
+// apart and 2.1 where they touch, the planes 10 us and some 25 for the first lines of
+// touching ones: 10 zones 11 and 22 us against 10 and 27, 32 zones 29 and 64 against 13
+// and 47.  Half a step of 256x192 with 33, 100, 512, 5,000 and all zones failed in a
+// square: 47, 80, 170, 430 and 567 us; scattered 33, 512 and 5,000: 14, 46 and 480.
 
 __global__ void k_fu_flip(Grid G, signed char *pflag, int *list, DevScalars *sc, int slot)
 {
@@ -225,11 +228,66 @@ struct RepairScratch {
   signed char *lkind; // the same by lines
 };
 constexpr signed char NO_REPAIR = 3;
+// A line of repair_sweep costs as much as this many of repair_lines, whose lines are
+// all of the plane's: 2.5 us (a chain of loads from where the zones lie) against 0.57
+// (loaded ahead, coalesced) at 256x192 and 384x384, 3.4 against 0.92 at 192x192x64.
+constexpr int SWEEP_LINE = 4;
+
+// The lines 2i + j = const of a plane's active zones, numbered from the first: a bit
+// for each that holds zones to repair, or for each 2^shift of them where a plane has more
+// lines than bits.
+constexpr int LINE_WORDS = 256;
+
+__device__ __forceinline__ int line_count(const Grid &G) { return 2 * (G.n1 - 1) + G.n2; }
+__device__ __forceinline__ int line_shift(int nl)
+{
+  int s = 0;
+  while ((nl - 1) >> s >= 32 * LINE_WORDS) s++;
+  return s;
+}
+
+__device__ __forceinline__ void mark_line(unsigned *bits, int shift, int k)
+{
+  k >>= shift;
+  const unsigned m = 1u << (k & 31);
+  if (!(bits[k >> 5] & m)) atomicOr(bits + (k >> 5), m);
+}
+
+// the first line from k on whose bit is set; nl where there is none
+__device__ __forceinline__ int next_line(const unsigned *bits, int shift, int nl, int k)
+{
+  while (k < nl) {
+    const int g = k >> shift;
+    const unsigned b = bits[g >> 5] >> (g & 31);
+    if (b & 1) return k;
+    k = (b ? g + __ffs((int)b) - 1 : (g | 31) + 1) << shift;
+  }
+  return nl;
+}
+
+// rows [lo, hi] of the active zones on line w
+__device__ __forceinline__ void line_rows(const Grid &G, int w, int &lo, int &hi)
+{
+  lo = (w - G.jstop + 1) / 2;
+  hi = (w - G.jstart) / 2;
+  if (lo < G.istart) lo = G.istart;
+  if (hi > G.istop) hi = G.istop;
+}
 
 // 2i + j modulo the row's length tells a row's zones apart
 __device__ __forceinline__ long line_slot(const Grid &G, int i, int j)
 {
   return (long)((2 * i + j) % G.sn2) * G.sn1 + i;
+}
+
+// fixup1zone's floors of the density and energy of a zone at rest, rf and uf those its
+// place and field give
+__device__ __forceinline__ void floor_at_rest(double &r, double &u, double rf, double uf)
+{
+  const double ur = div_rn(u, UORHOMAX, 1. / UORHOMAX);
+  if (rf < ur) rf = ur;
+  if (r < rf) r = rf;
+  if (u < uf) u = uf;
 }
 
 // The density and energy of the failed zones of plane h in loop order, by one
@@ -238,9 +296,9 @@ __device__ __forceinline__ long line_slot(const Grid &G, int i, int j)
 // done, those in row i+1 still untouched.  A row hands its last result to the
 // next through shared memory; old values and the zones' kinds and floors are
 // loaded PF lines ahead, coalesced (laid out by zones, where a line's rows lie a row
-// apart, a 256x192 torus took 920 us for the whole repair; so 755, most of it the
-// chain of a line's instructions and its barrier, some 700 lines long).  Leaves the last
-// resorts' averages in R.
+// apart, a 256x192 torus with every zone failed took 920 us for the whole repair; so 567,
+// most of it the chain of a line's instructions and its barrier, some 700 lines long).
+// Leaves the last resorts' averages in R.
 __device__ void repair_lines(const Grid &G, const RepairScratch &W, int h)
 {
   constexpr int PF = 4;
@@ -302,10 +360,7 @@ __device__ void repair_lines(const Grid &G, const RepairScratch &W, int h)
             const long c = slot(m, 0, i);
             Ra[c] = vr;
             Rb[c] = vu;
-            const double uf = div_rn(vu, UORHOMAX, 1. / UORHOMAX);
-            const double rf = ra[s] < uf ? uf : ra[s];
-            if (vr < rf) vr = rf;
-            if (vu < rb[s]) vu = rb[s];
+            floor_at_rest(vr, vu, ra[s], rb[s]);
           }
         }
         ring[w & 1][0][t] = vr;
@@ -329,103 +384,193 @@ __device__ void repair_lines(const Grid &G, const RepairScratch &W, int h)
     }
 }
 
+// The same for a plane whose last resorts lie on few lines: those lines alone, in order,
+// by one block.  The zones are read where they lie: a failed neighbour earlier in loop
+// order from R, every other from P, which still holds the state before the repairs.
+// Leaves the last resorts' averages in old, their floored values in R.
+__device__ void repair_sweep(const Grid &G, const double *P, const signed char *pflag, const RepairScratch &W, int h,
+                             const unsigned *bits)
+{
+  const int w0 = 2 * G.istart + G.jstart, nl = line_count(G), shift = line_shift(nl);
+  const long base = (long)h * G.ng, s = G.sn2;
+  for (int k = next_line(bits, shift, nl, 0); k < nl; k = next_line(bits, shift, nl, k + 1)) {
+    int lo, hi;
+    line_rows(G, w0 + k, lo, hi);
+    for (int i = lo + (int)threadIdx.x; i <= hi; i += blockDim.x) {
+      const int j = w0 + k - 2 * i;
+      const long c = cidx(G, h, i, j), l = base + line_slot(G, i, j);
+      if (W.lkind[l] != 2 || pflag[c] != 0) continue;
+      double v[2];
+#pragma unroll
+      for (int q = 0; q < 2; q++) {
+        const double *X = P + q * G.nc, *R = W.R + q * G.nc;
+        auto repaired = [&](int di, int dj) {
+          const int ii = i + di, jj = j + dj;
+          const long cc = c + di * s + dj;
+          const bool f = ii >= G.istart && jj >= G.jstart && jj <= G.jstop && pflag[cc] == 0;
+          return f ? R[base + line_slot(G, ii, jj)] : X[cc];
+        };
+        // repair_zone's last resort
+        v[q] = 0.5 * (0.25 * (X[c + 1] + repaired(0, -1) + repaired(-1, 0) + X[c + s])
+                      + 0.25 * (X[c + s + 1] + X[c + s - 1] + repaired(-1, 1) + repaired(-1, -1)));
+      }
+      W.old[l] = v[0];
+      W.old[G.nc + l] = v[1];
+      floor_at_rest(v[0], v[1], W.R[l], W.R[G.nc + l]);
+      W.R[l] = v[0];
+      W.R[G.nc + l] = v[1];
+    }
+    __syncthreads();
+  }
+}
+
 // Many failures: plane h by one cluster.  Within a plane zone (i, j) depends
 // only on (i-1, j-1..j+1) and (i, j-1), all on earlier lines 2i + j = const, so
 // sweeping those lines in order gives the loop order's results.  What a last
 // resort reads of its neighbours is their density and energy alone, and it
 // leaves the zone at rest, so that its floors but for u/50 follow from its field.
-// So the ordered pass (repair_lines, a line of a few additions and comparisons)
-// carries only those two, and everything else runs in parallel around it:
-// stencil repairs and floors before, the last resorts' velocities after.  All of
-// it is done on copies and committed at the end: a gamma failure changes a flag
-// that later zones' stencils read, and then the plane is repaired again the plain
-// way, one line after another.  (That plain way for every zone took 3.0 ms a half
-// step for a 256x192 torus with 49,000 failed zones; a step of an ensemble that
-// holds it went from 6.1 to 2.2 ms with this one.)
+// So the ordered pass carries only those two, and everything else runs in parallel
+// around it: stencil repairs (of good zones, which no repair changes) and floors before,
+// the last resorts' velocities after.  All of it is done on copies and committed at the
+// end: a gamma failure changes a flag that later zones' stencils read, and then the plane
+// is repaired again the plain way, one line after another.  (That plain way for every zone
+// took 3.0 ms a half step for a 256x192 torus with 49,000 failed zones; a step of an
+// ensemble that holds it went from 6.1 to 2.2 ms with this one.)
 template <class Cluster>
-__device__ void repair_plane(const Grid &G, Cluster &cl, double *P, signed char *pflag, const RepairScratch &W, int h,
-                             const double *__restrict__ geo, const double *__restrict__ floors, DevScalars *sc)
+__device__ void repair_plane(const Grid &G, Cluster &cl, double *P, signed char *pflag, const int *list, int n,
+                             const RepairScratch &W, int h, const double *__restrict__ geo,
+                             const double *__restrict__ floors, DevScalars *sc)
 {
-  __shared__ int again;
+  __shared__ int again, nlast;            // lines with a last resort
+  __shared__ unsigned lines[LINE_WORDS];  // their bits
   const int rank = (int)cl.block_rank(), tid = rank * blockDim.x + threadIdx.x, nt = (int)cl.num_blocks() * blockDim.x;
-  const bool lines = G.n1 + 1 <= (int)blockDim.x;  // one thread per row
-  if (threadIdx.x == 0) again = lines ? 0 : 1;
+  const int w0 = 2 * G.istart + G.jstart, nl = line_count(G), shift = line_shift(nl);
+  const bool rows = G.n1 + 1 <= (int)blockDim.x;  // repair_lines: one thread per row
+  // With a quarter of the zones failed the last resorts lie on a quarter of the lines or
+  // more, and those are not counted (10 to 30 us of a repair's 300 to 1,100).  The
+  // failed zones come from the list while it holds them all, else from the flags, with
+  // repair_lines' copies made on the way.
+  const bool most = rows && 4L * n >= (long)G.n1 * G.n2 * G.n3;
+  const bool listed = n <= FAIL_CAP && !most, copy = rows && !listed;
+  const long base = (long)h * G.ng;
+  const int ng = (int)G.ng, m = listed ? n : ng;
+  for (int t = threadIdx.x; t < LINE_WORDS; t += blockDim.x) lines[t] = 0;
+  if (threadIdx.x == 0) again = nlast = 0;
   cl.sync();
   int *again0 = cl.map_shared_rank(&again, 0);
-  if (lines) {
-    const long base = (long)h * G.ng;
-    int any = 0;
-    for (long g = tid; g < G.ng; g += nt) {
-      const int i = (int)(g / G.sn2), j = (int)(g % G.sn2);
-      const long c = base + g, l = base + line_slot(G, i, j);
-      signed char kind = NO_REPAIR;
-      W.old[l] = P[RHO * G.nc + c];
-      W.old[G.nc + l] = P[UU * G.nc + c];
-      if (i >= G.istart && i <= G.istop && j >= G.jstart && j <= G.jstop && pflag[c] == 0) {
-        kind = (signed char)stencil_kind(G, pflag, c);
-        any = 1;
-        double v[8];
-        if (kind < 2) {
-          int fail = 0;
-          repair_zone(G, P, c, kind, v);
-          if (fix_zone(G, geo, floors, i, j, v, &fail) || fail) *again0 = 1;
-          for (int k = 0; k < 8; k++) W.S[k * G.nc + c] = v[k];
-          W.R[l] = v[RHO];
-          W.R[G.nc + l] = v[UU];
-        } else {
-          // the floors of a zone at rest with this field (fixup1zone)
-          v[RHO] = v[UU] = v[U1] = v[U2] = v[U3] = 0.;
-          for (int k = B1; k <= B3; k++) v[k] = P[k * G.nc + c];
-          Geo q;
-          load_geo(geo_at(geo, G, L_CENT), G.ng, g, q);
-          State s;
-          int fail = 0;
-          get_state(v, q, s, &fail);
-          const double bsq = dot4(s.bcon, s.bcov);
-          double rf = __ldg(floors + g), uf = __ldg(floors + G.ng + g);
-          if (rf < bsq / BSQORHOMAX) rf = bsq / BSQORHOMAX;
-          if (uf < bsq / BSQOUMAX) uf = bsq / BSQOUMAX;
-          W.R[l] = rf;
-          W.R[G.nc + l] = uf;
-        }
-      }
-      W.kind[c] = W.lkind[l] = kind;
+  unsigned *lines0 = cl.map_shared_rank(lines, 0);
+  auto in_grid = [&](int i, int j) { return i >= G.istart && i <= G.istop && j >= G.jstart && j <= G.jstop; };
+  auto copy_old = [&](long c, long l, bool failed) {
+    W.old[l] = P[RHO * G.nc + c];
+    W.old[G.nc + l] = P[UU * G.nc + c];
+    if (!failed) W.lkind[l] = NO_REPAIR;
+  };
+  int any = 0;
+  for (int k = tid; k < m; k += nt) {
+    const int g = listed ? (int)(list[k] - base) : k;
+    if (g < 0 || g >= ng) continue;  // another plane's
+    const int i = g / G.sn2, j = g % G.sn2;
+    const long c = base + g;
+    const long l = base + line_slot(G, i, j);
+    const bool failed = listed || (in_grid(i, j) && pflag[c] == 0);
+    if (copy) copy_old(c, l, failed);
+    if (!failed) {
+      W.kind[c] = NO_REPAIR;
+      continue;
     }
-    if (!__syncthreads_or(any) && cl.num_blocks() == 1) return;  // (3D) no failure in this plane
+    const int kind = stencil_kind(G, pflag, c);
+    any = 1;
+    W.kind[c] = W.lkind[l] = (signed char)kind;
+    if (kind == 2 && !most) mark_line(lines, shift, 2 * i + j - w0);
+    double v[8];
+    if (kind < 2) {
+      int fail = 0;
+      repair_zone(G, P, c, kind, v);
+      if (fix_zone(G, geo, floors, i, j, v, &fail) || fail) *again0 = 1;
+      for (int q = 0; q < 8; q++) W.S[q * G.nc + c] = v[q];
+      W.R[l] = v[RHO];
+      W.R[G.nc + l] = v[UU];
+    } else {
+      // the floors of a zone at rest with this field (fixup1zone)
+      v[RHO] = v[UU] = v[U1] = v[U2] = v[U3] = 0.;
+      for (int q = B1; q <= B3; q++) v[q] = P[q * G.nc + c];
+      Geo q;
+      load_geo(geo_at(geo, G, L_CENT), G.ng, g, q);
+      State s;
+      int fail = 0;
+      get_state(v, q, s, &fail);
+      const double bsq = dot4(s.bcon, s.bcov);
+      double rf = __ldg(floors + g), uf = __ldg(floors + G.ng + g);
+      if (rf < bsq / BSQORHOMAX) rf = bsq / BSQORHOMAX;
+      if (uf < bsq / BSQOUMAX) uf = bsq / BSQOUMAX;
+      W.R[l] = rf;
+      W.R[G.nc + l] = uf;
+    }
+  }
+  if (!__syncthreads_or(any) && cl.num_blocks() == 1) return;  // (3D) no failure in this plane
+  if (!most && rank != 0)
+    for (int t = threadIdx.x; t < LINE_WORDS; t += blockDim.x)
+      if (lines[t]) atomicOr(lines0 + t, lines[t]);
+  cl.sync();
+  if (!most) {
+    for (int t = threadIdx.x; t < LINE_WORDS; t += blockDim.x)
+      if (lines0[t]) atomicAdd(&nlast, __popc(lines0[t]) << shift);
+    __syncthreads();
+  }
+  if ((most || nlast) && !*again0) {
+    const bool sweep = !rows || (!most && SWEEP_LINE * nlast < nl);
+    const double *avg = sweep ? W.old : W.R;
+    if (sweep) {
+      if (rank == 0) repair_sweep(G, P, pflag, W, h, lines);
+    } else {
+      if (listed) {
+        for (int g = tid; g < ng; g += nt) {
+          const int i = g / G.sn2, j = g % G.sn2;
+          copy_old(base + g, base + line_slot(G, i, j), in_grid(i, j) && pflag[base + g] == 0);
+        }
+        cl.sync();
+      }
+      if (rank == 0) repair_lines(G, W, h);
+    }
     cl.sync();
-    if (rank == 0) repair_lines(G, W, h);
-    cl.sync();
-    for (long g = tid; g < G.ng; g += nt) {
+    for (int k = tid; k < m; k += nt) {
+      const int g = listed ? (int)(list[k] - base) : k;
       const long c = base + g;
-      if (W.kind[c] != 2) continue;
-      const int i = (int)(g / G.sn2), j = (int)(g % G.sn2);
+      if (g < 0 || g >= ng || W.kind[c] != 2) continue;
+      const int i = g / G.sn2, j = g % G.sn2;
       const long l = base + line_slot(G, i, j);
       double v[8];
-      v[RHO] = W.R[l];
-      v[UU] = W.R[G.nc + l];
+      v[RHO] = avg[l];
+      v[UU] = avg[G.nc + l];
       v[U1] = v[U2] = v[U3] = 0.;
-      for (int k = B1; k <= B3; k++) v[k] = P[k * G.nc + c];
+      for (int q = B1; q <= B3; q++) v[q] = P[q * G.nc + c];
       int fail = 0;
       if (fix_zone(G, geo, floors, i, j, v, &fail) || fail) *again0 = 1;
-      for (int k = 0; k < 8; k++) W.S[k * G.nc + c] = v[k];
+      for (int q = 0; q < 8; q++) W.S[q * G.nc + c] = v[q];
     }
-    cl.sync();
-    if (!*again0)
-      for (long g = tid; g < G.ng; g += nt) {
-        const long c = base + g;
-        if (W.kind[c] == NO_REPAIR) continue;
-        for (int k = 0; k < 8; k++) P[k * G.nc + c] = W.S[k * G.nc + c];
-      }
   }
-  if (*again0 && rank == 0) {
-    const int w0 = 2 * G.istart + G.jstart, w1 = 2 * G.istop + G.jstop;
-    for (int w = w0; w <= w1; w++) {
-      // i such that j = w - 2i lies in [jstart, jstop]
-      int ilo = (w - G.jstop + 1) / 2, ihi = (w - G.jstart) / 2;
-      if (ilo < G.istart) ilo = G.istart;
-      if (ihi > G.istop) ihi = G.istop;
-      for (int i = ilo + (int)threadIdx.x; i <= ihi; i += blockDim.x)
-        if (pflag[cidx(G, h, i, w - 2 * i)] == 0) repair_in_place(G, P, pflag, geo, floors, sc, h, i, w - 2 * i);
+  cl.sync();
+  if (!*again0) {
+    for (int k = tid; k < m; k += nt) {
+      const int g = listed ? (int)(list[k] - base) : k;
+      const long c = base + g;
+      if (g < 0 || g >= ng || W.kind[c] == NO_REPAIR) continue;
+      for (int q = 0; q < 8; q++) P[q * G.nc + c] = W.S[q * G.nc + c];
+    }
+  } else if (rank == 0) {
+    for (int k = threadIdx.x; k < m; k += blockDim.x) {
+      const int g = listed ? (int)(list[k] - base) : k;
+      if (g < 0 || g >= ng || W.kind[base + g] == NO_REPAIR) continue;
+      mark_line(lines, shift, 2 * (g / G.sn2) + g % G.sn2 - w0);
+    }
+    __syncthreads();
+    for (int k = next_line(lines, shift, nl, 0); k < nl; k = next_line(lines, shift, nl, k + 1)) {
+      int lo, hi;
+      line_rows(G, w0 + k, lo, hi);
+      for (int i = lo + (int)threadIdx.x; i <= hi; i += blockDim.x) {
+        const int j = w0 + k - 2 * i;
+        if (pflag[cidx(G, h, i, j)] == 0) repair_in_place(G, P, pflag, geo, floors, sc, h, i, j);
+      }
       __syncthreads();
     }
   }
@@ -444,7 +589,7 @@ __global__ void __launch_bounds__(512) k_repair(Grid G, double *P, signed char *
   if (n <= FIX_LIST_MAX) {
     if (blockIdx.x == 0) repair_list(G, P, pflag, list, n, fixbuf, geo, floors, sc);
   } else {
-    repair_plane(G, cl, P, pflag, W, (int)(blockIdx.x / cl.num_blocks()), geo, floors, sc);
+    repair_plane(G, cl, P, pflag, list, n, W, (int)(blockIdx.x / cl.num_blocks()), geo, floors, sc);
   }
   if (rebound) {  // 2D: the one cluster makes the ghost cells again
     cl.sync();

@@ -52,7 +52,7 @@ struct TrParams {
 };
 
 constexpr int FAIL_CAP = 8192;     // failed zones listed
-constexpr int FIX_LIST_MAX = 32;   // up to this many, repaired through the sorted list
+constexpr int FIX_LIST_MAX = 12;   // up to this many, repaired through the sorted list (harm_api.cu)
 
 struct Ctx {
   Grid G;

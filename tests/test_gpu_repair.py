@@ -11,7 +11,7 @@ import pytest
 from helpers import active, make_oracle
 
 pytestmark = pytest.mark.gpu
-LIST = 32  # FIX_LIST_MAX
+LIST = 12  # FIX_LIST_MAX
 
 
 @pytest.fixture(scope="module")
@@ -78,4 +78,52 @@ def test_gamma_failures_repair_in_loop_order(shape, hc, oracle_built):
     g = pr.geometry["gcov"]
     g[sick, 3, 2, 2] *= -1e4
     f = flags(shape, shape[0] * shape[1] * shape[2] // 4, seed=5)
+    repair_both(hc, pr, f, expect_marks=True)
+
+
+def clump(shape, count, at=(0, 0)):
+    """count failures side by side in every phi plane but the second, in a near square
+    whose first zone is at"""
+    n1, n2, n3 = shape
+    f = np.zeros((n3, n1, n2), dtype=np.int8)
+    w = min(max(int(np.ceil(np.sqrt(count))), -(-count // (n2 - at[1]))), n1 - at[0])
+    q = np.zeros((w, -(-count // w)), dtype=np.int8)
+    q.reshape(-1)[:count] = 1
+    f[:, at[0]:at[0] + w, at[1]:at[1] + q.shape[1]] = q
+    if n3 > 1:
+        f[1] = 0
+    return f
+
+
+# few lines with last resorts (swept alone), most of them (the ordered pass over all),
+# more failures than the list holds (8,192) of either kind, more rows than the ordered
+# pass has threads (511), and more lines than bits (8,192)
+@pytest.mark.parametrize("shape,f", [
+    ((60, 80, 1), [(40, (0, 0))]), ((60, 80, 1), [(100, (50, 70)), (60, (3, 2))]), ((60, 80, 1), [(900, (20, 30))]),
+    ((60, 80, 1), [(4300, (0, 0))]), ((200, 100, 1), [(8192, (5, 5))]), ((200, 100, 1), [(8193, (5, 5))]),
+    ((150, 330, 1), [(8200, (0, 100))]), ((520, 40, 1), [(35, (500, 3))]), ((530, 40, 1), [(20000, (0, 0))]),
+    ((8, 8300, 1), [(64, (0, 8000)), (50, (1, 4))]), ((8, 8300, 1), [(9000, (0, 100))]),
+    ((24, 20, 6), [(30, (3, 4))]), ((24, 20, 6), [(400, (0, 0))]), ((70, 50, 10), [(1200, (10, 0))]),
+    ((70, 50, 10), [(60, (60, 30)), (80, (0, 0))])])
+def test_clumps_match_oracle(shape, f, hc, oracle_built):
+    fail = np.zeros((shape[2],) + shape[:2], dtype=np.int8)
+    for count, at in f:
+        fail |= clump(shape, count, at)
+    repair_both(hc, hc.torus_problem(*shape), fail)
+
+
+@pytest.mark.parametrize("shape,count", [((20, 24, 1), 32), ((20, 24, 1), 33), ((12, 10, 4), 32), ((12, 10, 4), 33),
+                                         ((200, 100, 1), 9000), ((40, 36, 8), 9000), ((256, 192, 1), 700)])
+def test_scattered_failures_match_oracle(shape, count, hc, oracle_built):
+    repair_both(hc, hc.torus_problem(*shape), flags(shape, count))
+
+
+@pytest.mark.parametrize("shape,count", [((60, 80, 1), 50), ((200, 100, 1), 9000), ((24, 20, 6), 60)])
+def test_gamma_failures_in_clumps(shape, count, hc, oracle_built):
+    """as test_gamma_failures_repair_in_loop_order, on few lines and beyond the list"""
+    pr = hc.torus_problem(*shape)
+    rng = np.random.default_rng(8)
+    sick = rng.random((shape[0] + 4, shape[1] + 4)) < 0.3
+    pr.geometry["gcov"][sick, 3, 2, 2] *= -1e4
+    f = clump(shape, count, (10, 3)) | flags(shape, count // 2, seed=5)
     repair_both(hc, pr, f, expect_marks=True)
