@@ -1218,18 +1218,6 @@ __global__ void k_set_mass(DevScalars *sc, double mass_in, double mass_out)
   sc->mass_in = mass_in;
   sc->mass_out = mass_out;
 }
-// the context's device current for a launch, the caller's again after it
-struct OnDevice {
-  int was = -1;
-  explicit OnDevice(int device)
-  {
-    if (cudaGetDevice(&was) != cudaSuccess || was == device || cudaSetDevice(device) != cudaSuccess) was = -1;
-  }
-  ~OnDevice()
-  {
-    if (was >= 0) cudaSetDevice(was);
-  }
-};
 }  // namespace harm
 
 extern "C" int harm_set_time(harm_ctx *h, double t, double dt)

@@ -167,6 +167,19 @@ int fail_with(int code, const std::string &msg);
       return ::harm::fail_with(HARM_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// a device current for some calls, the caller's again after them
+struct OnDevice {
+  int was = -1;
+  explicit OnDevice(int device)
+  {
+    if (cudaGetDevice(&was) != cudaSuccess || was == device || cudaSetDevice(device) != cudaSuccess) was = -1;
+  }
+  ~OnDevice()
+  {
+    if (was >= 0) cudaSetDevice(was);
+  }
+};
+
 inline dim3 zone_grid(const Grid &G) { return dim3((G.n2 + 31) / 32, (G.n1 + 3) / 4, G.n3); }
 
 // What the discrete adjoint (harm_adjoint.cu) keeps of one recomputed step;

@@ -42,6 +42,7 @@ bool HostLanes::init(int device)
 {
   device_ = device;
   n_ = 0;
+  OnDevice on(device);
   const int want = std::max(1, std::min<int>(HOST_LANES, (int)std::thread::hardware_concurrency()));
   for (int k = 0; k < want; k++) {
     HostLane &l = lane[k];
@@ -87,6 +88,7 @@ template <class Body>
 cudaError_t HostLanes::run(const Body &body)
 {
   cudaError_t err[HOST_LANES];
+  OnDevice on(device_);  // and the caller's again
   auto one = [&](int k) {
     err[k] = cudaSetDevice(device_);
     if (err[k] == cudaSuccess) err[k] = body(lane[k], k);
