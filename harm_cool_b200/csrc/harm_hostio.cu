@@ -14,8 +14,8 @@
 
 #include <algorithm>
 #include <cstring>
+#include <exception>
 #include <mutex>
-#include <system_error>
 #include <thread>
 
 namespace harm {
@@ -85,8 +85,9 @@ HostLanes *HostLanes::hold(int device)
 void HostLanes::release() { slot(device_).held.unlock(); }
 
 template <class Body>
-cudaError_t HostLanes::run(const Body &body)
+cudaError_t HostLanes::run(const Body &body, long parts)
 {
+  const int n = (int)std::min<long>(n_, parts);
   cudaError_t err[HOST_LANES];
   OnDevice on(device_);  // and the caller's again
   auto one = [&](int k) {
@@ -96,16 +97,18 @@ cudaError_t HostLanes::run(const Body &body)
   std::thread t[HOST_LANES];
   int started = 1;
   try {
-    for (; started < n_; started++) t[started] = std::thread(one, started);
-  } catch (const std::system_error &) {
-    // no more threads: the caller takes the remaining lanes' parts too
+    for (; started < n; started++) t[started] = std::thread(one, started);
+  } catch (const std::exception &) {
+    // no more threads, or memory for them: the caller takes the remaining lanes' parts too
   }
   one(0);
-  for (int k = started; k < n_; k++) one(k);
+  for (int k = started; k < n; k++) one(k);
   for (int k = 1; k < started; k++) t[k].join();
-  for (int k = 0; k < n_; k++)
-    if (err[k] != cudaSuccess) return err[k];
-  return cudaSuccess;
+  const cudaError_t *bad = std::find_if(err, err + n, [](cudaError_t e) { return e != cudaSuccess; });
+  if (bad == err + n) return cudaSuccess;
+  // a lane that stopped early left work in flight on its buffers: not into the next call
+  for (int k = 0; k < n; k++) cudaStreamSynchronize(lane[k].st);
+  return *bad;
 }
 
 #define LANE(call)                                \
@@ -139,7 +142,7 @@ int copy_to_host(int device, cudaStream_t st, void *dst, const void *src, size_t
           b ^= 1;
         }
         return cudaSuccess;
-      }));
+      }, (long)nc));
       return HARM_OK;
     }
   }
@@ -166,7 +169,7 @@ int copy_to_device(int device, cudaStream_t st, void *dst, const void *src, size
           LANE(cudaEventRecord(l.done[b], l.st));
         }
         return cudaStreamSynchronize(l.st);
-      }));
+      }, (long)nc));
       return HARM_OK;
     }
   }
@@ -221,7 +224,7 @@ bool utoprim_2d_lanes(const double *U, const double *gcov, const double *gcon, c
       }
       return cudaSuccess;
     };
-    return nc == 1 ? body(h.L->lane[0], 0) : h.L->run(body);
+    return h.L->run(body, nc);
   }();
   *rc = e == cudaSuccess ? HARM_OK
                          : fail_with(HARM_E_CUDA, std::string("harm_utoprim_2d_batch: ") + cudaGetErrorString(e));

@@ -23,10 +23,11 @@ public:
   static HostLanes *hold(int device);
   void release();
   int n() const { return n_; }
-  // body(lane, index) on every lane, each on a thread of its own with the device
-  // current; the first error
+  // body(lane, index) on every lane, or on as many as there are parts to a call, each
+  // on a thread of its own (the first on the caller's) with the device current; the first
+  // error, with nothing left in flight after one
   template <class Body>
-  cudaError_t run(const Body &body);
+  cudaError_t run(const Body &body, long parts);
 
   HostLane lane[HOST_LANES];
 

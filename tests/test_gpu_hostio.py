@@ -78,3 +78,38 @@ def test_batch_inversion_at_chunk_edges(n, hc):
     got = hc.utoprim_2d_batch(U[t], gcov[t], gcon[t], gdet[t], out, 4. / 3.)
     assert np.array_equal(got, ret[t])
     assert np.array_equal(out, ref[t], equal_nan=True)
+
+
+def test_batch_inversions_in_threads(hc):
+    """one thread holds the lanes, the others take the plain path: the same results"""
+    pr = hc.torus_problem(32, 32, 1)
+    g = pr.geometry
+    n = 60000
+    rng = np.random.default_rng(2)
+    i, j = rng.integers(2, 34, n), rng.integers(2, 34, n)
+    gcov, gcon = g["gcov"][i, j, 3].reshape(n, 16), g["gcon"][i, j, 3].reshape(n, 16)
+    gdet = g["gdet"][i, j, 3]
+    prim = np.zeros((n, 8))
+    prim[:, 0], prim[:, 1] = 10. ** rng.uniform(-4, 0, n), 10. ** rng.uniform(-6, -2, n)
+    U = np.zeros((n, 8))
+    U[:, 0] = prim[:, 0] * gdet
+    U[:, 1] = -prim[:, 1] * gdet
+    U[:, 5:8] = 1e-3 * rng.standard_normal((n, 3))
+    ref = prim.copy()
+    ret = hc.utoprim_2d_batch(U, gcov, gcon, gdet, ref, 4. / 3.)
+    bad = []
+    start = threading.Barrier(6)
+
+    def work(k):
+        start.wait()
+        for _ in range(8):
+            out = prim.copy()
+            got = hc.utoprim_2d_batch(U, gcov, gcon, gdet, out, 4. / 3.)
+            if not (np.array_equal(got, ret) and np.array_equal(out, ref, equal_nan=True)):
+                bad.append(k)
+    ts = [threading.Thread(target=work, args=(k,)) for k in range(6)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not bad

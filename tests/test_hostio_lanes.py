@@ -249,7 +249,7 @@ def driver(tmp_path_factory):
     return str(d / "lanes")
 
 
-@pytest.mark.parametrize("what", ["copies", "device"])
+@pytest.mark.parametrize("what", ["copies", "device", "errors"])
 def test_lanes(what, driver):
     r = subprocess.run([driver, what], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
