@@ -278,7 +278,14 @@ extern "C" int harm_eos_batch(harm_eos *e, int what, int precision, long n, cons
   CK(cudaMemcpy(B.r, rho0, n * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(B.uu, u, n * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(B.T, lastT, n * sizeof(double), cudaMemcpyHostToDevice));
-  harm::k_eos_batch<<<(unsigned)((n + 127) / 128), 128>>>(e->d, what, precision == HARM_MIXED, n, B.t, B.r, B.uu,
+  // batch calls on tracked tables evaluate the general way throughout: what the
+  // tabulated cubics are checked against
+  harm::EosDev d = e->d;
+  if (d.miss) {
+    d.cub = nullptr;
+    d.cub32 = nullptr;
+  }
+  harm::k_eos_batch<<<(unsigned)((n + 127) / 128), 128>>>(d, what, precision == HARM_MIXED, n, B.t, B.r, B.uu,
                                                            B.T, B.o);
   CK(cudaGetLastError());
   CK(cudaMemcpy(out, B.o, n * sizeof(double), cudaMemcpyDeviceToHost));

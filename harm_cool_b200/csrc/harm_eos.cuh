@@ -280,10 +280,11 @@ __device__ __noinline__ void eos_value_w(const EosDev &E, const double *__restri
 // without writing its outputs, cache4d.c:899-911).  e and p inside a 4 x 4 window
 // with T, its difference points and rho in the second intervals -- all but the
 // table's edges and points on a node -- take the rows' cubics from the table made
-// of them; nothing is marked missing there, so tracked tables go the general way.
-// That leaves two divisions a window of the twelve, and four windows fewer: a
-// 256x256 step's face kernels 300 -> 151 us, the update's two 200 and 470 -> 120
-// and 384 us.
+// of them.  A NaN node makes its row's cubic, and so the value, NaN; a tracked table's
+// evaluation then goes the general way too, which marks the nodes.  That leaves two
+// divisions a window of the twelve, and four windows fewer: a 256x256 step's face kernels
+// 300 -> 151 us, the update's two 200 and 470 -> 120 and 384 us; a step on tracked tables,
+// the general way throughout, 2.28 -> 1.44 ms, of 97x75 mixed 0.88 -> 0.55.
 template <bool DER>
 __device__ __noinline__ bool eos_value(const EosDev &E, int tab, int d, double rho, int x0, int sx, double T,
                                        double &val, double &der)
@@ -291,7 +292,7 @@ __device__ __noinline__ bool eos_value(const EosDev &E, int tab, int d, double r
   if (!(T >= __ldg(E.ya)) || !(T <= __ldg(E.ya + E.ny - 1))) return false;
   int y0, sy;
   eos_window(E.ny, E.ya, T, y0, sy);
-  if (E.cub && !E.miss && d <= EOS_P && sx == 4 && sy == 4) {
+  if (E.cub && d <= EOS_P && sx == 4 && sy == 4) {
     const double xi = __ldg(E.ya + y0 + 1), xr = __ldg(E.ya + y0 + 2);
     const double h = T * 1.0E-6;  // spline_akima_der's points (akima.c:259-298)
     const double tm = T - h, tp = T + h;
@@ -312,7 +313,7 @@ __device__ __noinline__ bool eos_value(const EosDev &E, int tab, int d, double r
       const double *rec = E.xrec + 8 * x0;
       val = akima_window_rec(xw, row, rec, rho);
       if (DER) der = akima_window_rec(xw, rowd, rec, rho);
-      return true;
+      if (!E.miss || val == val) return true;
     }
   }
   const double *plane = E.val + ((long)d * E.ntab + tab) * E.nx * E.ny;
@@ -614,6 +615,20 @@ __device__ __noinline__ void eos_value_wf(const EosDev &E, const float *__restri
   if (DER) akima_window_f<SX, false>(xw, rowd, rho, der, unused);
 }
 
+// whether four rows' cubics come from computed nodes alone: a NaN node makes its row's
+// c1 NaN (the value need not show it, a node derivative in float can leave a NaN row
+// out).  For tracked tables only, and out of line: tested on the way, the cubics cost
+// untracked tables 3 % of a mixed 97x75 step.
+static __device__ __noinline__ bool eos_rows_whole(const float4 *src, int ny)
+{
+  bool whole = true;
+  for (int r = 0; r < 4; r++) {
+    const float c1 = __ldg(src + (long)r * ny).z;
+    whole = whole && c1 == c1;
+  }
+  return whole;
+}
+
 // d: EOS_E or EOS_P; the rows' cubics from their table as in eos_value
 template <bool DER>
 __device__ __noinline__ bool eos_value_f(const EosDev &E, int tab, int d, float rho, int x0, int sx, float T,
@@ -622,10 +637,10 @@ __device__ __noinline__ bool eos_value_f(const EosDev &E, int tab, int d, float 
   if (!(T >= __ldg(E.ya32)) || !(T <= __ldg(E.ya32 + E.ny - 1))) return false;
   int y0, sy;
   eos_window_f(E.ny, E.ya32, T, y0, sy);
-  if (E.cub32 && !E.miss && sx == 4 && sy == 4) {
+  if (E.cub32 && sx == 4 && sy == 4) {
     const float xi = __ldg(E.ya32 + y0 + 1), xr = __ldg(E.ya32 + y0 + 2);
-    if (T > xi && !(T > xr)) {
-      const float4 *src = E.cub32 + (((long)d * E.ntab + tab) * E.nx + x0) * E.ny + y0 + 1;
+    const float4 *src = E.cub32 + (((long)d * E.ntab + tab) * E.nx + x0) * E.ny + y0 + 1;
+    if (T > xi && !(T > xr) && (!E.miss || eos_rows_whole(src, E.ny))) {
       float xw[4], row[4], rowd[4], unused;
       const float u = T - xi;
 #pragma unroll
