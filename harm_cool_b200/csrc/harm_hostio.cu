@@ -4,7 +4,8 @@
 // HOST_LANES threads each move every HOST_LANES-th chunk through two pinned buffers
 // of their own, so that page faults, host copies and the link overlap.  On 16 host
 // cores: reading back 288x256x256 (1.25 GB) 290 -> about 55 ms, Utoprim_2d of
-// 100,003 host zones (46 MB) 10.5 -> 2.5 ms.
+// 100,003 host zones (46 MB) 10.5 -> 2.5 ms.  An array the caller has pinned goes in one
+// copy (1.25 GB 23 ms; through the lanes 32).
 //
 // The lanes of a device are made by the first large copy there (64 MB pinned and
 // as much on the device at most, held until the process ends) and belong to one
@@ -22,8 +23,11 @@ namespace harm {
 
 namespace {
 constexpr int MAX_DEVICES = 16;
-// below this the threads cost more than they save
-constexpr size_t LANES_MIN = 8u << 20;
+// Below these the threads cost more than they save (ms, plain against lanes): to the
+// device 8.5 MB 0.47, 0.49, 9.7 MB 0.53, 0.50, 16.6 MB 0.86, 0.68; to the host, where now
+// and then a thread wakes late, 8.5 MB 0.47, 0.57 to 0.78, 16.6 MB 0.86, 0.69 to 1.02,
+// 21 MB 1.08, 0.79 to 0.97.
+constexpr size_t TO_DEVICE_MIN = 10u << 20, TO_HOST_MIN = 20u << 20;
 
 struct Slot {
   std::mutex held;
@@ -35,6 +39,14 @@ Slot &slot(int device)
 {
   static Slot *s = new Slot[MAX_DEVICES];  // outlives every caller; the process's end takes it
   return s[device];
+}
+// memory the driver knows (pinned, managed) goes over the link as it is, in one copy
+bool pageable(const void *p)
+{
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
+  cudaGetLastError();
+  return true;
 }
 }  // namespace
 
@@ -119,7 +131,7 @@ cudaError_t HostLanes::run(const Body &body, long parts)
 
 int copy_to_host(int device, cudaStream_t st, void *dst, const void *src, size_t n)
 {
-  if (n >= LANES_MIN) {
+  if (n >= TO_HOST_MIN && pageable(dst)) {
     HoldLanes h(device);
     if (h.L) {
       CK(cudaStreamSynchronize(st));  // the layout kernel before; the lanes' streams need no event then
@@ -153,7 +165,7 @@ int copy_to_host(int device, cudaStream_t st, void *dst, const void *src, size_t
 
 int copy_to_device(int device, cudaStream_t st, void *dst, const void *src, size_t n)
 {
-  if (n >= LANES_MIN) {
+  if (n >= TO_DEVICE_MIN && pageable(src)) {
     HoldLanes h(device);
     if (h.L) {
       CK(cudaStreamSynchronize(st));  // earlier readers of dst

@@ -15,9 +15,11 @@ def hc(harm_lib):
     return harm_cool_b200
 
 
-# 8 MB is where the lanes begin (131,072 cells of 64 B): just below, just above, a
-# few chunks more, and a 3D array with phi ghost planes
-@pytest.mark.parametrize("shape", [(315, 406, 1), (316, 406, 1), (400, 500, 1), (60, 70, 40)])
+# the lanes begin at 10 MB to the device (163,840 cells of 64 B) and at 20 MB to the host:
+# just below and above each, whole and broken chunks between, and a 3D array with phi ghost
+# planes
+@pytest.mark.parametrize("shape", [(315, 406, 1), (316, 406, 1), (400, 400, 1), (400, 402, 1), (400, 500, 1),
+                                   (568, 568, 1), (568, 570, 1), (700, 700, 1), (60, 70, 40), (60, 70, 100)])
 def test_state_round_trip(shape, hc):
     pr = hc.torus_problem(*shape)
     ctx = hc.Context(pr)
@@ -33,9 +35,36 @@ def test_state_round_trip(shape, hc):
     ctx.close()
 
 
+@pytest.mark.parametrize("shape", [(120, 128, 1), (600, 600, 1), (60, 70, 100)])
+def test_pinned_arrays(shape, hc):
+    """arrays the caller has pinned take one copy straight over the link"""
+    import ctypes
+    import torch
+    pr = hc.torus_problem(*shape)
+    ctx = hc.Context(pr)
+    pinned = torch.empty(pr.shape + (8,), dtype=torch.float64, pin_memory=True).numpy()
+    pinned[...] = np.random.default_rng(1).standard_normal(pinned.shape)
+    if shape[2] > 1:
+        pinned[0], pinned[-1] = pinned[-2], pinned[1]
+    p = pinned.copy()
+    ctx.put_prims(pinned)
+    assert np.array_equal(ctx.get_prims(), p)
+    pinned[...] = 0.
+    ctx.lib.harm_get_prims(ctx.h, pinned.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), None)
+    assert np.array_equal(pinned, p)
+    ctx.init_torus()
+    q = ctx.get_prims()
+    ctx.step_ch_host(q)
+    ctx.init_torus()
+    pinned[...] = ctx.get_prims()
+    ctx.step_ch_host(pinned)
+    assert np.array_equal(pinned, q)
+    ctx.close()
+
+
 def test_contexts_in_threads(hc):
     """one thread holds the lanes, the others copy plainly"""
-    pr = hc.torus_problem(420, 400, 1)
+    pr = hc.torus_problem(600, 600, 1)
     bad = []
 
     def work(seed):

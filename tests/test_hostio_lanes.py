@@ -161,7 +161,8 @@ int main(int argc, char **argv)
   cudaStreamCreateWithFlags(&st, 0);
   std::vector<char> dev(N), host = pattern(N, 1), back(N);
   if (what == "copies") {
-    for (size_t n : {(size_t)1000, (size_t)(8u << 20) - 8, (size_t)(8u << 20), (size_t)(12u << 20) + 8, N}) {
+    for (size_t n : {(size_t)1000, (size_t)(10u << 20) - 8, (size_t)(10u << 20), (size_t)(12u << 20) + 8,
+                     (size_t)(20u << 20) - 8, (size_t)(20u << 20), N}) {
       std::fill(dev.begin(), dev.end(), 0);
       EXPECT(copy_to_device(0, st, dev.data(), host.data(), n) == 0);
       cudaStreamSynchronize(st);
@@ -249,7 +250,7 @@ def driver(tmp_path_factory):
     return str(d / "lanes")
 
 
-@pytest.mark.parametrize("what", ["copies", "device", "errors"])
+@pytest.mark.parametrize("what", ["copies", "pinned", "device", "errors"])
 def test_lanes(what, driver):
     r = subprocess.run([driver, what], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
