@@ -383,7 +383,7 @@ def run_ours(args, world, rank, local):
 def run_ensemble(args):
     """64 seeded 2D tori (N1, N2 from {96,128,192,256}, a, Rmax, beta drawn) advanced
     as one ensemble -- one CUDA graph launch per step, mixed precision, tiles chosen
-    by the autotuner per resolution -- against the same 64 tori run one after the
+    by the autotuner for the resolutions that use them -- against the same 64 tori run one after the
     other on the plain FP64 path.  Aggregate zone-cycles/s over all members.  Some
     draws fail the inversion in most zones every step and run far slower than the
     rest; the same comparison is also reported without them."""

@@ -684,7 +684,8 @@ class Context:
         return ids, X, st
 
     def set_tile(self, bx, by):
-        """Threads per block of the face and zone kernels (bx theta x by r, 128 in all)."""
+        """Threads per block of the inversion (bx theta x by r, 128 in all) on grids of more
+        than 56,832 zones; elsewhere the kernels' blocks have shapes of their own."""
         _check(self.lib.harm_set_tile(self.h, bx, by))
 
     def tile(self):
@@ -693,7 +694,8 @@ class Context:
         return bx.value, by.value
 
     def autotune_tile(self, steps=3):
-        """Time each candidate tile on this state (restored afterwards); keep the fastest."""
+        """Time each candidate tile on this state (restored afterwards) and keep the
+        fastest; where the tile changes nothing, keep the one that is set."""
         bx, by = ctypes.c_int(), ctypes.c_int()
         _check(self.lib.harm_autotune_tile(self.h, steps, ctypes.byref(bx), ctypes.byref(by)))
         return bx.value, by.value

@@ -1108,6 +1108,7 @@ struct Graph {
 
 struct Work {
   int nsteps = 0, every = 0, tbx = 0, tby = 0;  // what the graphs were captured for
+  bool captured = false;
   size_t bytes = 0;
   DevBuf B;
   double *ck = nullptr, *pend = nullptr, *lam = nullptr, *W = nullptr, *vbuf = nullptr;
@@ -1322,8 +1323,8 @@ static int run_adjoint(Ctx *x, Work &w, double *J, double *grad, double *ms)
   const int last0 = (nseg - 1) * every, lastlen = nsteps - last0, blast = (nseg - 1) & 1;
   Graph &gstep = w.gstep, *const grec = w.grec, *const grev = w.grev;
   int rc = HARM_OK;
-  if (!gstep.e || w.tbx != x->tbx || w.tby != x->tby) {
-    w.tbx = 0;  // captured only once all of it is
+  if (!w.captured || (tile_in_use(x) && (w.tbx != x->tbx || w.tby != x->tby))) {
+    w.captured = false;  // until all of it is
     rc = capture(gstep, [&] { return exact::launch_step(x); });
     if (rc) return rc;
     // for the sets that some segment of `every` steps uses (a single segment is
@@ -1338,6 +1339,7 @@ static int run_adjoint(Ctx *x, Work &w, double *J, double *grad, double *ms)
     }
     w.tbx = x->tbx;
     w.tby = x->tby;
+    w.captured = true;
   }
   // the run state recorded with segment seg's steps, kept for the checks at the end
   auto keep_scalars = [&](int seg, int len) -> int {

@@ -1751,7 +1751,7 @@ extern "C" int harm_set_tile(harm_ctx *h, int bx, int by)
 {
   if (!h || !tile_ok(bx, by)) return fail_with(HARM_E_ARG, "tile must be bx x by = 128 threads, bx a multiple of 8");
   Ctx *x = &h->x;
-  if (x->tbx != bx || x->tby != by) invalidate_graph(x);
+  if (tile_in_use(x) && (x->tbx != bx || x->tby != by)) invalidate_graph(x);
   x->tbx = bx;
   x->tby = by;
   return HARM_OK;
@@ -1767,12 +1767,18 @@ extern "C" int harm_get_tile(harm_ctx *h, int *bx, int *by)
 
 // Times `steps` ordinary steps per candidate tile, each trial from the same
 // saved state (primitives, flags, run scalars), and keeps the fastest; the
-// state is restored afterwards, so the run continues as if untouched.
+// state is restored afterwards, so the run continues as if untouched.  Where no
+// kernel's blocks have the tile's shape there is nothing to choose.
 extern "C" int harm_autotune_tile(harm_ctx *h, int steps, int *bx, int *by)
 {
   if (!h || steps < 1) return fail_with(HARM_E_ARG, "bad argument");
   Ctx *x = &h->x;
   if (x->cool) return fail_with(HARM_E_ARG, "the tile autotuner is for the gamma-law step");
+  if (!tile_in_use(x)) {
+    if (bx) *bx = x->tbx;
+    if (by) *by = x->tby;
+    return sync_status(x);
+  }
   static const int cand[][2] = {{32, 4}, {64, 2}, {16, 8}, {128, 1}};
   const size_t pb = (size_t)8 * x->G.nc * sizeof(double);
   DevScalars s0;
@@ -1884,7 +1890,8 @@ static int ensemble_graph(harm_ensemble *e)
   bool same = e->exec != nullptr;
   for (size_t k = 0; k < e->members.size() && same; k++) {
     const Ctx *x = e->members[k];
-    same = x->mode == e->mode[k] && x->tbx == e->tbx[k] && x->tby == e->tby[k] && x->ntr == e->ntr[k];
+    same = x->mode == e->mode[k] && x->ntr == e->ntr[k] &&
+           (!tile_in_use(x) || (x->tbx == e->tbx[k] && x->tby == e->tby[k]));
   }
   if (same) return HARM_OK;
   if (e->exec) {

@@ -82,7 +82,7 @@ struct Ctx {
   float *conn32;                 // mixed mode: FP32 connection [40][ng]
   double *Ubuf;                  // conserved variables between the two update launches [8][nc]
   double *emf;                   // flux_ct's corner EMFs e1, e2, e3 [3][nc] (k_emf)
-  int tbx, tby;                  // tile of the zone and face kernels: theta x r threads, 128 in all
+  int tbx, tby;                  // tile of the inversion's blocks on large grids: theta x r threads, 128 in all
   long ntr;                      // tracer particles
   double *trX;                   // [3][ntr] code coordinates X1, X2, X3
   int *trids;                    // [ntr][3] labels (i, j, h)
@@ -179,6 +179,18 @@ struct OnDevice {
     if (was >= 0) cudaSetDevice(was);
   }
 };
+
+// The update in one launch up to this many zones (three resident blocks of 128 on
+// every SM, one wave), in two or three launches above, whose lighter kernels keep
+// more warps resident: 251x187 (47k zones) FP64 update 37 us in one launch against
+// 39 in three with k_emf, before the launches saved around it.
+constexpr int UPD_MINB = 3;
+constexpr long FUSED_ZONES = 148L * UPD_MINB * 128;
+inline bool fused_update(const Grid &G) { return (long)G.n1 * G.n2 * G.n3 <= FUSED_ZONES; }
+
+// whether a step of this context has blocks of its tile's shape: the inversion above
+// FUSED_ZONES (the other kernels' blocks have shapes of their own)
+inline bool tile_in_use(const Ctx *x) { return !x->cool && !fused_update(x->G); }
 
 inline dim3 zone_grid(const Grid &G) { return dim3((G.n2 + 31) / 32, (G.n1 + 3) / 4, G.n3); }
 

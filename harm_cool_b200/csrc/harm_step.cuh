@@ -30,9 +30,6 @@
 #ifndef HARM_INV_MINB
 #define HARM_INV_MINB 1
 #endif
-#ifndef HARM_UPD_MINB
-#define HARM_UPD_MINB 3
-#endif
 
 namespace harm {
 namespace HARM_VARIANT {
@@ -867,7 +864,7 @@ __global__ void __launch_bounds__(128, HARM_INV_MINB) k_invert(Grid G, const dou
 // launch and the repair with its bound_prim in another, a 2D step is 7 launches
 // instead of 22: 128x128 FP64 85.8 -> 69 us, 251x187 mixed 87 -> 71 us.
 template <bool FULL, bool THREE_D, bool REC>
-__global__ void __launch_bounds__(128, HARM_UPD_MINB) k_update(Grid G, const double *pi, const double *pb,
+__global__ void __launch_bounds__(128, UPD_MINB) k_update(Grid G, const double *pi, const double *pb,
                                                                const flux_t *__restrict__ F1,
                                                                const flux_t *__restrict__ F2,
                                                                const flux_t *__restrict__ F3, ZoneData Z,
@@ -923,12 +920,6 @@ inline Bufs bufs(Ctx *x)
 #endif
 }
 
-// The update in one launch up to this many zones (three resident blocks of 128 on
-// every SM, one wave), in two or three launches above, whose lighter kernels keep
-// more warps resident: 251x187 (47k zones) FP64 update 37 us in one launch against
-// 39 in three with k_emf, before the launches saved around it.
-constexpr long FUSED_ZONES = 148L * HARM_UPD_MINB * 128;
-
 // Ub, zrec, wrec: the adjoint's recomputation keeps U, the inversion's output and
 // which inversion gave it there
 template <bool FULL>
@@ -940,7 +931,7 @@ void launch_update(Ctx *x, const double *pi, const double *pb, double *pf, doubl
   const ZoneData Z{x->geo, x->conn, x->geo32, x->conn32, x->floors, x->katm};
   const ZoneOut O{pf, x->pflag, x->fail_list, zrec, wrec};
   const long zones = (long)G.n1 * G.n2 * G.n3;
-  const bool fused = zones <= FUSED_ZONES;
+  const bool fused = fused_update(G);
   const dim3 eg(((G.n2 + 1) * (G.n1 + 1) + 127) / 128, 1, G.n3);
   if (G.n3 > 1) k_emf<true><<<eg, 128, 0, x->stream>>>(G, B.F1, B.F2, B.F3, x->emf, x->sc);
   else if (!fused) k_emf<false><<<eg, 128, 0, x->stream>>>(G, B.F1, B.F2, B.F3, x->emf, x->sc);

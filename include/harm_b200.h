@@ -274,14 +274,18 @@ int harm_tracers_get(harm_ctx *ctx, int *ids, double *X, signed char *status);
 
 /* ---- tile shapes (no reference counterpart: the reference runs on CPUs) ---- */
 
-/* Threads per block of the face and zone kernels: bx along theta by by along r,
-   bx * by = 128, bx a multiple of 8 (default 32 x 4). */
+/* Threads per block of the gamma-law step's inversion on grids of more than 56,832
+   zones, whose update takes several launches: bx along theta by by along r,
+   bx * by = 128, bx a multiple of 8 (default 32 x 4).  The other kernels' blocks, and
+   all of them on smaller grids and with COOL_EOS, have shapes of their own: there the
+   tile changes nothing. */
 int harm_set_tile(harm_ctx *ctx, int bx, int by);
 int harm_get_tile(harm_ctx *ctx, int *bx, int *by);
 
 /* Autotuner: times `steps` steps with each candidate tile (32x4, 64x2, 16x8,
    128x1), every trial from the same saved state, restores that state, keeps
-   the fastest tile and returns it in *bx, *by (either may be NULL). */
+   the fastest tile and returns it in *bx, *by (either may be NULL).  Where the tile
+   changes nothing it times nothing and returns the tile that is set. */
 int harm_autotune_tile(harm_ctx *ctx, int steps, int *bx, int *by);
 
 /* ---- ensembles: many independent grids on one GPU (no reference counterpart:
@@ -293,7 +297,8 @@ typedef struct harm_ensemble harm_ensemble;
    member by one step_ch() with its own dt, as harm_step_ch would; the members'
    step sequences are captured as parallel branches of one CUDA graph, launched
    once per ensemble step.  The members stay usable on their own; a member whose
-   precision or tile changes is re-captured at the next run. */
+   precision, tracers or (where it matters) tile changes is re-captured at the next
+   run. */
 int harm_ensemble_create(harm_ctx *const *members, int n, harm_ensemble **out);
 void harm_ensemble_destroy(harm_ensemble *ens);
 

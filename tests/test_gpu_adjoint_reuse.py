@@ -98,3 +98,21 @@ def test_one_two_and_more_segments_agree(nsteps, every, hc):
         assert abs(J - out[0][0]) <= 1e-14 * abs(out[0][0])
         assert np.linalg.norm(g - out[0][1]) <= 1e-12 * np.linalg.norm(out[0][1])
     ctx.close()
+
+
+def test_another_tile_where_the_tile_is_used(hc):
+    """above 56,832 zones the kept graphs are captured again for another tile"""
+    pr = hc.torus_problem(241, 240, 1)
+    ctx = start(hc, pr)
+    p, t = ctx.get_prims(), ctx.time()
+    out = []
+    for tile in ((32, 4), (64, 2), (64, 2), (8, 16)):
+        ctx.put_prims(p)
+        ctx.set_time(*t)
+        ctx.set_mass(0., 0.)  # J is a difference of the counter
+        ctx.set_tile(*tile)
+        out.append(ctx.adjoint_mass_in(3, 2)[:2])
+    for J, g in out[1:]:
+        assert J == out[0][0]
+        assert np.linalg.norm(g - out[0][1]) <= 1e-12 * np.linalg.norm(out[0][1])
+    ctx.close()

@@ -90,3 +90,36 @@ def test_autotune_keeps_the_state(hc):
     other.run(5)
     c.run(2)
     np.testing.assert_array_equal(c.get_prims(), other.get_prims())
+
+
+@pytest.mark.parametrize("shape,used", [((40, 36, 1), False), ((237, 239, 1), False), ((241, 240, 1), True),
+                                        ((30, 32, 8), False)])
+def test_autotune_chooses_where_the_tile_is_used(shape, used, hc):
+    """up to 56,832 zones no kernel has blocks of the tile's shape: the tile that is
+    set stays, a shape outside the candidates included"""
+    c = hc.Context(hc.torus_problem(*shape))
+    c.init_torus()
+    c.set_tile(8, 16)
+    c.run(1)
+    p, t = c.get_prims(), c.time()
+    for _ in range(3):
+        tile = c.autotune_tile(steps=1)
+        assert c.tile() == tile
+        assert tile in ((32, 4), (64, 2), (16, 8), (128, 1)) if used else tile == (8, 16)
+    assert np.array_equal(c.get_prims(), p) and c.time() == t
+    c.close()
+
+
+@pytest.mark.parametrize("shape", [(241, 240, 1), (101, 97, 6)])
+def test_tile_shape_does_not_change_results_where_it_is_used(shape, hc):
+    pr = hc.torus_problem(*shape)
+    ref = _fresh(hc, pr)
+    ref.run(2)
+    c = _fresh(hc, pr)
+    for tile in [(64, 2), (16, 8), (128, 1), (8, 16)]:
+        c.init_torus()
+        c.set_tile(*tile)
+        c.run(2)
+        np.testing.assert_array_equal(c.get_prims(), ref.get_prims())
+        assert c.time() == ref.time()
+    c.close()
