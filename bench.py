@@ -32,15 +32,19 @@ sys.path.insert(0, ROOT)
 
 
 
-def kernels_per_step(n3, cool=False):
-    """Kernel launches of one step.  Per half step: the flux kernel, the corner EMFs,
-    the conserved update, the inversion, bound_prim, the repair and bound_prim in
-    3D; in 2D the flux kernel, the update (one launch) and the repair, and with
-    COOL_EOS a flux kernel per direction and the update in two launches.  Then the
-    sums with the dt update, and with COOL_EOS the tracers."""
-    if cool:
-        return 2 * 5 + 2
-    return 2 * (7 if n3 > 1 else 3) + 1
+FUSED_ZONES = 148 * 3 * 128  # zones up to which the step's update is one launch
+
+
+def kernels_per_step(n1, n2, n3, cool=False, tracers=False):
+    """Kernel launches of one step.  Per half step: the flux kernel; the update, one
+    launch up to FUSED_ZONES zones, two above, with the corner EMFs before it in 3D and
+    above that size; the repair; in 3D bound_prim before and after the repair.  COOL_EOS:
+    a flux kernel per direction and the update in two launches.  Then the sums with the
+    dt update, and the tracers where there are any."""
+    three_d, large = n3 > 1, n1 * n2 * n3 > FUSED_ZONES
+    flux = (3 if three_d else 2) if cool else 1
+    update = 2 if cool else (2 if large else 1) + (1 if three_d or large else 0)
+    return 2 * (flux + update + (3 if three_d else 1)) + 1 + (1 if tracers else 0)
 
 
 METRIC = "zone-cycles/s 288x256x256 GRMHD step_ch: FP64, mixed precision beside it"
@@ -343,7 +347,7 @@ def run_ours(args, world, rank, local):
                     "d2h_bytes_per_step": bytes_host, "steps": args.e2e_steps,
                     "path": "harm_run_host: per step upload, step, download, each upload overlapped with the "
                             "previous step's download"},
-            "gpu_launches": kernels_per_step(args.n3) * args.steps,
+            "gpu_launches": kernels_per_step(args.n1, args.n2, args.n3) * args.steps,
             "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak,
                          "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
                          "algorithmic_bytes": alg, "peak_source": peak_kind,
@@ -665,7 +669,7 @@ def run_cool(args):
                     "steps": args.e2e_steps,
                     "path": "harm_run_host: per step upload, step, download, each upload overlapped with the "
                             "previous step's download"},
-            "gpu_launches": kernels_per_step(1, cool=True) * args.steps,
+            "gpu_launches": kernels_per_step(n, n, 1, cool=True, tracers=args.cool_tracers > 0) * args.steps,
             "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": None, "algorithmic_bytes": alg,
                          "peak_source": peak_kind,
