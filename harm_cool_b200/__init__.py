@@ -128,6 +128,7 @@ _SIGNATURES = {
     "harm_sync": (ctypes.c_int, [ctypes.c_void_p]),
     "harm_run_timed": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, _DP]),
     "harm_adjoint_mass_in": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_int, _DP, _DP, _DP]),
+    "harm_adjoint_release": (ctypes.c_int, [ctypes.c_void_p]),
     "harm_step_ch_host_timed": (ctypes.c_int, [ctypes.c_void_p, _DP, ctypes.c_int, _DP]),
     "harm_run_host": (ctypes.c_int, [ctypes.c_void_p, _DP, ctypes.c_int]),
     "harm_time_kernels": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, _DP]),
@@ -637,12 +638,17 @@ class Context:
         the current state and returns (J, grad, ms) -- J the mass that crossed the
         inner boundary (the change of mass_in, diag.c:578), grad = dJ/dp of the state
         at the call in get_prims' layout, ms the device time of the forward pass and
-        of the reverse sweep."""
+        of the reverse sweep.  Up to 2 GB of device memory stay with the context for the
+        next call (adjoint_release)."""
         J = ctypes.c_double()
         grad = np.zeros(self.shape + (NPR,))
         ms = (ctypes.c_double * 2)()
         _check(self.lib.harm_adjoint_mass_in(self.h, nsteps, checkpoint_every, ctypes.byref(J), _dp(grad), ms))
         return J.value, grad, (ms[0], ms[1])
+
+    def adjoint_release(self):
+        """Free the device memory that adjoint_mass_in keeps for its next call."""
+        _check(self.lib.harm_adjoint_release(self.h))
 
     def restart_read(self, path):
         """restart_init(): state, time, mass counters and tracers from a restart file."""

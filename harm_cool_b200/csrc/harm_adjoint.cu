@@ -1097,8 +1097,10 @@ struct DevBuf {
 // reversal.  Kept in the context for the next call with the same step counts (an
 // optimisation's iterations): making and freeing it, and setting the stack limit
 // that the driver sizes for each kernel by itself, took 13 of a 31.4 ms call at
-// 192x192, 50 steps, which is 18.4 ms now.  Freed with the context, by a call with other counts, and at the end of a
-// call where it holds more than KEEP_BYTES.
+// 192x192, 50 steps, which is 18.4 ms now.  Freed with the context, by
+// harm_adjoint_release, by a call with other counts, where the context goes to the mixed
+// step or to COOL_EOS (which the adjoint refuses), and at the end of a call where it
+// holds more than KEEP_BYTES.
 constexpr size_t KEEP_BYTES = 2u << 30;
 
 struct Graph {
@@ -1478,4 +1480,11 @@ extern "C" int harm_adjoint_mass_in(harm_ctx *h, int nsteps, int checkpoint_ever
   }
   if (rc || w->bytes > adj::KEEP_BYTES) adj::free_work(x);
   return rc;
+}
+
+extern "C" int harm_adjoint_release(harm_ctx *h)
+{
+  if (!h) return harm::fail_with(HARM_E_ARG, "null context");
+  harm::release_adjoint(&h->x);
+  return HARM_OK;
 }

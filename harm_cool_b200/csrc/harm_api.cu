@@ -1137,7 +1137,7 @@ extern "C" void harm_destroy(harm_ctx *h)
   if (!h) return;
   Ctx *x = &h->x;
   if (x->graph_exec) cudaGraphExecDestroy(x->graph_exec);
-  if (x->adj) x->adj_free(x);
+  release_adjoint(x);
   void *ptrs[] = {x->p, x->ph, x->F1, x->F2, x->F3, x->pflag, x->geo, x->conn, x->floors, x->katm,
                   x->stage, x->stage_flag, x->fail_list, x->fix_buf, x->partials, x->sc,
                   x->F1f, x->F2f, x->F3f, x->geo32, x->conn32, x->Ubuf, x->emf, x->trX, x->trids, x->trst,
@@ -1310,6 +1310,7 @@ extern "C" int harm_set_precision(harm_ctx *h, int mode)
     cudaGraphExecDestroy(x->graph_exec);
     x->graph_exec = nullptr;
   }
+  if (mode == HARM_MIXED) release_adjoint(x);
   x->mode = mode;
   return HARM_OK;
 }

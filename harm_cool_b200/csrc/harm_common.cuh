@@ -98,6 +98,11 @@ struct Ctx {
   void (*adj_free)(Ctx *);
 };
 
+inline void release_adjoint(Ctx *x)
+{
+  if (x->adj) x->adj_free(x);
+}
+
 __device__ __forceinline__ void record_fail(DevScalars *sc, int code, int h, int i, int j)
 {
   if (atomicCAS(&sc->fail_code, 0, code) == 0) {

@@ -444,6 +444,7 @@ extern "C" int harm_set_eos(harm_ctx *h, const harm_eos *eos)
     x->cool_seed = true;
   }
   invalidate_graph(x);
+  release_adjoint(x);
   x->eos = eos->d;
   x->cool = true;
   return HARM_OK;

@@ -121,6 +121,10 @@ int harm_init_torus(harm_ctx *ctx, const harm_grid_spec *g, const harm_torus_spe
 int harm_put_prims(harm_ctx *ctx, const double *p, const signed char *pflag);
 int harm_get_prims(harm_ctx *ctx, double *p, signed char *pflag);
 
+/* harm_set_time and harm_set_mass are queued on the context's stream and return without
+   waiting for it: an error of earlier work comes back from a later call that waits
+   (harm_sync, harm_get_time, harm_run, ...).  harm_set_time also clears a recorded
+   failure. */
 int harm_set_time(harm_ctx *ctx, double t, double dt);
 int harm_get_time(harm_ctx *ctx, double *t, double *dt);
 int harm_set_mass(harm_ctx *ctx, double mass_in, double mass_out);
@@ -225,10 +229,15 @@ int harm_dump_write(harm_ctx *ctx, const harm_restart_header *hdr, const harm_gr
    sweep with its recomputation (ms[1]).  The call allocates device memory for
    the checkpoints and for two segments' records (about 20 MB per step of a
    segment at 192x192), works on the context's stream and on two streams of
-   its own, and returns when the results are in J and grad.  Refused for 3D,
-   COOL_EOS, the mixed step and attached tracers; HARM_E_ADJOINT if a step
-   fails. */
+   its own, and returns when the results are in J and grad.  Up to 2 GB of that
+   memory stays with the context for the next call, until harm_destroy,
+   harm_adjoint_release, a call with another nsteps or checkpoint_every, or a switch
+   to the mixed step or COOL_EOS; a call that needs more frees it all before it
+   returns.  Refused for 3D, COOL_EOS, the mixed step and attached tracers;
+   HARM_E_ADJOINT if a step fails. */
 int harm_adjoint_mass_in(harm_ctx *ctx, int nsteps, int checkpoint_every, double *J, double *grad, double *ms);
+/* Free what harm_adjoint_mass_in keeps in the context. */
+int harm_adjoint_release(harm_ctx *ctx);
 
 /* ---- diagnostics ---- */
 
@@ -321,7 +330,8 @@ int harm_fixup1zone(harm_ctx *ctx, long n, const int *hij, double *pv, signed ch
 
 /* Utoprim_2d() (utoprim_2d.c:126, decs.h:608) over n independent zones on the
    device: U[n][8], gcov[n][16], gcon[n][16], gdet[n], prim[n][8] (guess in,
-   result out), ret[n] (the reference's return code).  Host arrays. */
+   result out), ret[n] (the reference's return code).  Host arrays.  When a CUDA call
+   fails, prim and ret may already hold some zones' results. */
 int harm_utoprim_2d_batch(const double *U, const double *gcov, const double *gcon,
                           const double *gdet, double *prim, int *ret, long n, double gam);
 

@@ -116,3 +116,39 @@ def test_another_tile_where_the_tile_is_used(hc):
         assert J == out[0][0]
         assert np.linalg.norm(g - out[0][1]) <= 1e-12 * np.linalg.norm(out[0][1])
     ctx.close()
+
+
+def test_kept_memory_is_given_back(hc):
+    """by harm_adjoint_release, by another precision and by COOL_EOS; the next call makes
+    it again"""
+    import torch
+    from harm_cool_b200 import eos_tables as et
+    pr = hc.torus_problem(64, 64, 1)
+    ctx = start(hc, pr)
+    p, t = ctx.get_prims(), ctx.time()
+    eos = hc.Eos(*et.build_tables(et.zone_radii(pr), gam=pr.params.gam))
+    ctx.set_precision(ctx.MIXED)  # the buffers of both, made once
+    ctx.set_eos(eos)
+    ctx.set_eos(None)
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+    out = []
+    for release in (ctx.adjoint_release, lambda: ctx.set_precision(ctx.MIXED), lambda: ctx.set_eos(eos),
+                    ctx.adjoint_release):
+        ctx.set_precision(ctx.FP64)
+        ctx.set_eos(None)
+        ctx.put_prims(p)
+        ctx.set_time(*t)
+        ctx.set_mass(0., 0.)
+        out.append(ctx.adjoint_mass_in(20, 20)[:2])
+        before = free()
+        release()
+        assert free() - before > 50e6  # 20 records twice of some 2 MB each
+        ctx.adjoint_release()          # nothing kept: no error
+    for J, g in out[1:]:
+        assert J == out[0][0]
+        assert np.linalg.norm(g - out[0][1]) <= 1e-12 * np.linalg.norm(out[0][1])
+    ctx.close()
+    eos.close()
