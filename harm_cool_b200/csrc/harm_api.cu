@@ -1122,9 +1122,12 @@ extern "C" int harm_create(const harm_params *prm, const double *gcov, const dou
       cudaMemcpy(x->coolgeo, hcg.data(), hcg.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(x->katm, katm, d.sn1 * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemcpy(x->sc, &s0, sizeof(s0), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemset(x->p, 0, st) != cudaSuccess || cudaMemset(x->ph, 0, st) != cudaSuccess ||
-      cudaMemset(x->F1, 0, st) != cudaSuccess || cudaMemset(x->F2, 0, st) != cudaSuccess ||
-      cudaMemset(x->pflag, 0, G.nc) != cudaSuccess) {
+      // (on the context's stream, ahead of all that follows there)
+      cudaMemsetAsync(x->p, 0, st, x->stream) != cudaSuccess ||
+      cudaMemsetAsync(x->ph, 0, st, x->stream) != cudaSuccess ||
+      cudaMemsetAsync(x->F1, 0, st, x->stream) != cudaSuccess ||
+      cudaMemsetAsync(x->F2, 0, st, x->stream) != cudaSuccess ||
+      cudaMemsetAsync(x->pflag, 0, G.nc, x->stream) != cudaSuccess) {
     harm_destroy(h);
     return fail_with(HARM_E_CUDA, "upload");
   }
