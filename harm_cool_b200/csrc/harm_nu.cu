@@ -16,10 +16,11 @@
 // harm_nu.cuh), and the warps of a node share its independent solves
 // (degeneracies, FuncNb3).
 //
-// 24 warps per SM (80 registers a thread): the warps' long FP64 latency chains
-// (exp, log, division) need that many to keep the FP64 pipe busy; with one warp a
-// node, measured 1.13x faster than 16 at 128 registers, which were 1.44x faster
-// than 12 at 168.
+// Resident per SM: eight nodes of three warps, 24 warps at 80 registers a thread, or two
+// nodes of nine, 18 warps at 96.  The warps' long FP64 latency chains (exp, log,
+// division) want many to keep the FP64 pipe busy: with one warp a node, 24 at 80
+// registers measured 1.13x faster than 16 at 128, which were 1.44x faster than 12 at
+// 168.  Nine warps run where the nodes are too few for that to matter.
 //
 // Tables are launched one per kernel over several streams without waiting in
 // between, so the blocks of a table still on its slowest nodes share the SMs
@@ -39,7 +40,9 @@ const Rules *host_rules();
 
 __constant__ Rules c_rules;
 
-constexpr int NODE_WARPS_SM = 24;  // resident warps per SM that the register budget allows (80 registers)
+// resident warps per SM that the register budget must allow, in whole nodes (768 threads:
+// eight nodes of TEAM3, two of TEAM9)
+constexpr int NODE_WARPS_SM = 24;
 // Up to this many nodes a node gets nine warps, above it three.  Few nodes wait on
 // the slowest of them, which nine warps finish sooner; many nodes fill the GPU, and
 // then the nine wait for one another too often.  Measured (ms, nine against three;
