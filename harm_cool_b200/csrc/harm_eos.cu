@@ -214,7 +214,14 @@ extern "C" int harm_eos_create(const harm_eos_desc *dsc, const double *xaxis, co
     d.cub32 = e->cub32;
     d.xrec = e->xrec;
   } else {
-    cudaGetLastError();  // an allocation that failed
+    // an allocation failed: no memory held for nothing
+    cudaGetLastError();
+    cudaFree(e->cub);
+    cudaFree(e->cub32);
+    cudaFree(e->xrec);
+    e->cub = nullptr;
+    e->cub32 = nullptr;
+    e->xrec = nullptr;
   }
   *out = e;
   return HARM_OK;

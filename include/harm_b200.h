@@ -164,10 +164,10 @@ int harm_step_ch_host_timed(harm_ctx *ctx, double *p, int nsteps, double *ms);
 
 /* Runs reps ordinary steps launched kernel by kernel with a CUDA event after
    each, and returns the average device time per launch of each kind, into
-   ms[HARM_NKERNELS] in this order: flux (all three directions), update
-   (flux-CT + source + inversion + floors), bound_prim, fixup_utoprim (flag
-   flip + repair), diagnostics (flux and mass sums, next dt, per step).  The
-   state advances by reps steps. */
+   ms[HARM_NKERNELS] in this order: flux (all directions), update (flux-CT + source
+   + inversion + floors + flags; in 2D the ghost cells too), bound_prim (3D; 0 in 2D),
+   fixup_utoprim with the bound_prim after it, diagnostics (flux and mass sums, next
+   dt, per step).  The state advances by reps steps. */
 #define HARM_NKERNELS 5
 int harm_time_kernels(harm_ctx *ctx, int reps, double *ms);
 
@@ -411,6 +411,9 @@ typedef struct harm_eos_desc {
   double gam;
   double l_unit;                    /* L_UNIT (cm) */
 } harm_eos_desc;
+/* Device memory: 40 B a node for the values, 8 for their float copies, and 96 for cubics
+   formed from them, which are left out where there is no room (the evaluations are slower
+   then, their results the same). */
 int harm_eos_create(const harm_eos_desc *desc, const double *xaxis, const double *yaxis,
                     const double *values, const double *hdfac, harm_eos **out);
 int harm_eos_destroy(harm_eos *eos);
