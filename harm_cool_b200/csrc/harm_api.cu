@@ -118,8 +118,8 @@ __global__ void k_bound(Grid G, double *P, signed char *pflag, const double *__r
 // plane) is repaired by repair_plane.  The list takes 0.8 us a zone where failures lie
 // apart and 2.1 where they touch, the planes 10 us and some 25 for the first lines of
 // touching ones: 10 zones 11 and 22 us against 10 and 27, 32 zones 29 and 64 against 13
-// and 47.  Half a step of 256x192 with 33, 100, 512, 5,000 and all zones failed in a
-// square: 47, 80, 170, 430 and 567 us; scattered 33, 512 and 5,000: 14, 46 and 480.
+// and 47.  Half a step of 256x192, random states, with 33, 100, 512, 5,000 and all zones
+// failed in a square: 47, 80, 170, 430 and 567 us; scattered 33, 512 and 5,000: 14, 46, 480.
 
 __global__ void k_fu_flip(Grid G, signed char *pflag, int *list, DevScalars *sc, int slot)
 {
@@ -296,8 +296,9 @@ __device__ __forceinline__ void floor_at_rest(double &r, double &u, double rf, d
 // done, those in row i+1 still untouched.  A row hands its last result to the
 // next through shared memory; old values and the zones' kinds and floors are
 // loaded PF lines ahead, coalesced (laid out by zones, where a line's rows lie a row
-// apart, a 256x192 torus with every zone failed took 920 us for the whole repair; so 567,
-// most of it the chain of a line's instructions and its barrier, some 700 lines long).
+// apart, that took a fifth longer: the repair of a 256x192 torus whose inversions all fail
+// takes 820 us so, most of it the chain of a line's instructions and its barrier, some 700
+// lines long).
 // Leaves the last resorts' averages in R.
 __device__ void repair_lines(const Grid &G, const RepairScratch &W, int h)
 {
