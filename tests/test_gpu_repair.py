@@ -96,15 +96,15 @@ def clump(shape, count, at=(0, 0)):
 
 
 # few lines with last resorts (swept alone), most of them (the ordered pass over all),
-# more failures than the list holds (8,192) of either kind, more rows than the ordered
-# pass has threads (511), and more lines than bits (8,192)
+# more failures than the list holds (8,192) of either kind and more than a quarter of the
+# zones, more rows than the ordered pass has threads (511), and more lines than bits (8,192)
 @pytest.mark.parametrize("shape,f", [
     ((60, 80, 1), [(40, (0, 0))]), ((60, 80, 1), [(100, (50, 70)), (60, (3, 2))]), ((60, 80, 1), [(900, (20, 30))]),
     ((60, 80, 1), [(4300, (0, 0))]), ((200, 100, 1), [(8192, (5, 5))]), ((200, 100, 1), [(8193, (5, 5))]),
     ((150, 330, 1), [(8200, (0, 100))]), ((520, 40, 1), [(35, (500, 3))]), ((530, 40, 1), [(20000, (0, 0))]),
     ((8, 8300, 1), [(64, (0, 8000)), (50, (1, 4))]), ((8, 8300, 1), [(9000, (0, 100))]),
     ((24, 20, 6), [(30, (3, 4))]), ((24, 20, 6), [(400, (0, 0))]), ((70, 50, 10), [(1200, (10, 0))]),
-    ((70, 50, 10), [(60, (60, 30)), (80, (0, 0))])])
+    ((70, 50, 10), [(60, (60, 30)), (80, (0, 0))]), ((96, 80, 8), [(1300, (20, 30))])])
 def test_clumps_match_oracle(shape, f, hc, oracle_built):
     fail = np.zeros((shape[2],) + shape[:2], dtype=np.int8)
     for count, at in f:
@@ -113,12 +113,14 @@ def test_clumps_match_oracle(shape, f, hc, oracle_built):
 
 
 @pytest.mark.parametrize("shape,count", [((20, 24, 1), 32), ((20, 24, 1), 33), ((12, 10, 4), 32), ((12, 10, 4), 33),
-                                         ((200, 100, 1), 9000), ((40, 36, 8), 9000), ((256, 192, 1), 700)])
+                                         ((200, 100, 1), 9000), ((40, 36, 8), 9000), ((256, 192, 1), 700),
+                                         ((96, 80, 8), 8192), ((96, 80, 8), 9000), ((96, 80, 8), 15360)])
 def test_scattered_failures_match_oracle(shape, count, hc, oracle_built):
     repair_both(hc, hc.torus_problem(*shape), flags(shape, count))
 
 
-@pytest.mark.parametrize("shape,count", [((60, 80, 1), 50), ((200, 100, 1), 9000), ((24, 20, 6), 60)])
+@pytest.mark.parametrize("shape,count", [((60, 80, 1), 50), ((200, 100, 1), 9000), ((150, 330, 1), 8200),
+                                         ((24, 20, 6), 60), ((96, 80, 8), 1200)])
 def test_gamma_failures_in_clumps(shape, count, hc, oracle_built):
     """as test_gamma_failures_repair_in_loop_order, on few lines and beyond the list"""
     pr = hc.torus_problem(*shape)
