@@ -972,6 +972,7 @@ void invalidate_graph(Ctx *x)
     cudaGraphExecDestroy(x->graph_exec);
     x->graph_exec = nullptr;
   }
+  x->plain_steps = 0;
 }
 
 int launch_step(Ctx *x)
@@ -1310,10 +1311,7 @@ extern "C" int harm_set_precision(harm_ctx *h, int mode)
     for (size_t k = 0; k < hc.size(); k++) hcf[k] = (float)hc[k];
     CK(cudaMemcpy(x->conn32, hcf.data(), hcf.size() * sizeof(float), cudaMemcpyHostToDevice));
   }
-  if (mode != x->mode && x->graph_exec) {
-    cudaGraphExecDestroy(x->graph_exec);
-    x->graph_exec = nullptr;
-  }
+  if (mode != x->mode) invalidate_graph(x);
   if (mode == HARM_MIXED) release_adjoint(x);
   x->mode = mode;
   return HARM_OK;
@@ -1339,12 +1337,18 @@ static int step_graph(Ctx *x)
   return HARM_OK;
 }
 
-// one step: the graph, one launch for the host instead of one per kernel (32x32:
-// set_time, step_ch_host and get_time 165 -> 140 us); the seeding step of COOL_EOS, which comes once,
-// kernel by kernel
+// One step: the graph, one launch for the host instead of one per kernel (32x32:
+// set_time, step_ch_host and get_time 165 -> 140 us).  Making it costs as much as some ten
+// steps' launches, so a context's first PLAIN_STEPS single steps, unless a run has made
+// it, go kernel by kernel, as does the seeding step of COOL_EOS, which comes once.
+constexpr int PLAIN_STEPS = 8;
 static int one_step(Ctx *x)
 {
   if (x->cool && x->cool_seed) return launch_step(x);
+  if (!x->graph_exec && x->plain_steps < PLAIN_STEPS) {
+    x->plain_steps++;
+    return launch_step(x);
+  }
   int rc = step_graph(x);
   if (rc) return rc;
   CK(cudaGraphLaunch(x->graph_exec, x->stream));

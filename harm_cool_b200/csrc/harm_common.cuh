@@ -75,7 +75,7 @@ struct Ctx {
   int nparts;
   DevScalars *sc;
   cudaGraphExec_t graph_exec;
-  int graph_steps;
+  int plain_steps;               // single steps launched kernel by kernel, before there is a graph (one_step)
   int mode;                      // HARM_FP64 or HARM_MIXED
   float *F1f, *F2f, *F3f;        // mixed mode: FP32 face fluxes [8][nc]
   float *geo32;                  // mixed mode: FP32 geometry [4 locations][GEO_N][ng]
