@@ -37,14 +37,14 @@ FUSED_ZONES = 148 * 3 * 128  # zones up to which the step's update is one launch
 
 def kernels_per_step(n1, n2, n3, cool=False, tracers=False):
     """Kernel launches of one step.  Per half step: the flux kernel; the update, one
-    launch up to FUSED_ZONES zones, two above, with the corner EMFs before it in 3D and
-    above that size; the repair; in 3D bound_prim before and after the repair.  COOL_EOS:
-    a flux kernel per direction and the update in two launches.  Then the sums with the
+    launch up to FUSED_ZONES zones, two above, with the corner EMFs before it and bound_prim
+    after it in 3D and above that size; the repair, in 3D with another bound_prim.
+    COOL_EOS: a flux kernel per direction and the update in two launches.  Then the sums with the
     dt update, and the tracers where there are any."""
     three_d, large = n3 > 1, n1 * n2 * n3 > FUSED_ZONES
     flux = (3 if three_d else 2) if cool else 1
-    update = 2 if cool else (2 if large else 1) + (1 if three_d or large else 0)
-    return 2 * (flux + update + (3 if three_d else 1)) + 1 + (1 if tracers else 0)
+    update = 2 + (1 if three_d else 0) if cool else (2 if large else 1) + (2 if three_d or large else 0)
+    return 2 * (flux + update + (2 if three_d else 1)) + 1 + (1 if tracers else 0)
 
 
 METRIC = "zone-cycles/s 288x256x256 GRMHD step_ch: FP64, mixed precision beside it"

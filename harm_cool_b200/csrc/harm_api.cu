@@ -15,8 +15,8 @@
 //
 // One step (step_ch.c:90-140) is, on one stream and without host sync:
 //   predictor : k_flux, then k_update or k_emf, k_cons, k_invert (dt/2) [flux-CT,
-//               source, inversion, floors, flags; in 2D the ghosts too],
-//               (3D) k_bound, k_repair, (3D) k_bound
+//               source, inversion, floors, flags; in 2D in one launch the ghosts too],
+//               else k_bound, k_repair, (3D) k_bound
 //   corrector : the same with dt and the Courant minima
 //   k_mass (diagnostic sums, next dt)
 #include <cooperative_groups.h>

@@ -193,6 +193,12 @@ constexpr int UPD_MINB = 3;
 constexpr long FUSED_ZONES = 148L * UPD_MINB * 128;
 inline bool fused_update(const Grid &G) { return (long)G.n1 * G.n2 * G.n3 <= FUSED_ZONES; }
 
+// whether the gamma-law update writes the ghosts (bound_prim) itself: the 2D update in one
+// launch.  In the inversion of larger grids the code that writes them costs more than
+// the launch it saves, though few zones take it: mixed 384x384 62 us a step against 42 and
+// two launches of 4, 1000x700 214 against 160, FP64 296 against 251.
+inline bool update_writes_ghosts(const Grid &G) { return G.n3 == 1 && fused_update(G); }
+
 // whether a step of this context has blocks of its tile's shape: the inversion above
 // FUSED_ZONES (the other kernels' blocks have shapes of their own)
 inline bool tile_in_use(const Ctx *x) { return !x->cool && !fused_update(x->G); }

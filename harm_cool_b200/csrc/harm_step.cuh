@@ -788,7 +788,8 @@ static __device__ __noinline__ void push_ghosts(const Grid &G, const ZoneOut &O,
 // Utoprim_2d with the isentropic fall-backs (step_ch.c:265-300) and fixup()
 // (fixup.c:142-383) of one zone; pz holds the guess (pi).  REC: also keep the
 // inversion's output before fixup() and which inversion gave it, for the discrete
-// adjoint's recomputation.  PUSH (2D): write the zone's ghost cells too.
+// adjoint's recomputation.  PUSH (2D, in the one-launch update): write the zone's ghost
+// cells too.
 template <bool REC, bool PUSH>
 __device__ __forceinline__ void invert_zone(const Grid &G, const double *U, const Geo &q, double *pz,
                                             const ZoneData &Z, const ZoneOut &O, DevScalars *sc, int slot, int h,
@@ -834,7 +835,7 @@ __device__ __forceinline__ void invert_zone(const Grid &G, const double *U, cons
   if (fail) record_fail(sc, fail, h + (G.n3 > 1 ? 1 : 0), i, j);
 }
 
-template <bool REC, bool PUSH>
+template <bool REC>
 __global__ void __launch_bounds__(128, HARM_INV_MINB) k_invert(Grid G, const double *__restrict__ pi,
                                                                const double *__restrict__ Ub, ZoneData Z, ZoneOut O,
                                                                int slot, int hb, DevScalars *sc)
@@ -854,7 +855,7 @@ __global__ void __launch_bounds__(128, HARM_INV_MINB) k_invert(Grid G, const dou
       U[k] = __ldg(Ub + k * G.nc + c);
       pz[k] = pi[k * G.nc + c];
     }
-    invert_zone<REC, PUSH>(G, U, q, pz, Z, O, sc, slot, h, i, j);
+    invert_zone<REC, false>(G, U, q, pz, Z, O, sc, slot, h, i, j);
   }
 }
 
@@ -957,22 +958,24 @@ void launch_update(Ctx *x, const double *pi, const double *pb, double *pf, doubl
   double *U = Ub ? Ub : x->Ubuf;
   if (G.n3 > 1) k_cons<FULL, true><<<cg, cb, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, U, x->sc);
   else k_cons<FULL, false><<<cg, cb, 0, x->stream>>>(G, pi, pb, B.F1, B.F2, B.F3, Z, x->emf, U, x->sc);
-  if (G.n3 > 1) k_invert<false, false><<<zg, tile, 0, x->stream>>>(G, pi, U, Z, O, FULL ? 1 : 0, hb, x->sc);
 #if !HARM_STEP_MIXED
-  else if (zrec) k_invert<true, true><<<zg, tile, 0, x->stream>>>(G, pi, U, Z, O, FULL ? 1 : 0, hb, x->sc);
+  if (zrec) {
+    k_invert<true><<<zg, tile, 0, x->stream>>>(G, pi, U, Z, O, FULL ? 1 : 0, hb, x->sc);
+    return;
+  }
 #endif
-  else k_invert<false, true><<<zg, tile, 0, x->stream>>>(G, pi, U, Z, O, FULL ? 1 : 0, hb, x->sc);
+  k_invert<false><<<zg, tile, 0, x->stream>>>(G, pi, U, Z, O, FULL ? 1 : 0, hb, x->sc);
 }
 
 // advance() + fixup + bound_prim + fixup_utoprim + bound_prim (step_ch.c:101-117);
-// in 2D the update writes the ghosts
+// a 2D update in one launch writes the ghosts
 template <bool FULL>
 void launch_half(Ctx *x, const double *pi, const double *pb, double *pf)
 {
   Bufs B = bufs(x);
   launch_flux<FULL>(x->G, x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc);
   launch_update<FULL>(x, pi, pb, pf);
-  if (x->G.n3 > 1) launch_bound(x, pf);
+  if (!update_writes_ghosts(x->G)) launch_bound(x, pf);
   launch_repair(x, pf, FULL ? 1 : 0);
 }
 
@@ -998,6 +1001,7 @@ static int launch_half_rec(Ctx *x, const double *pi, const double *pb, double *p
   launch_flux<FULL>(x->G, x->stream, pb, B.F1, B.F2, B.F3, x->geo, x->geo32, x->sc, FULL ? r.ctop : nullptr);
   CK(cudaMemcpyAsync(r.F1rho[s], B.F1 + RHO * nc, nc * sizeof(double), cudaMemcpyDeviceToDevice, x->stream));
   launch_update<FULL>(x, pi, pb, pf, r.Ub[s], r.Z[s], r.wz[s]);
+  if (!update_writes_ghosts(x->G)) launch_bound(x, pf);
   CK(cudaMemcpyAsync(r.X1[s], pf, 8 * nc * sizeof(double), cudaMemcpyDeviceToDevice, x->stream));
   CK(cudaMemcpyAsync(r.fl1[s], x->pflag, nc, cudaMemcpyDeviceToDevice, x->stream));
   CK(cudaMemcpyAsync(r.nfail[s], &x->sc->nfail[s], sizeof(int), cudaMemcpyDeviceToDevice, x->stream));
@@ -1022,7 +1026,7 @@ int launch_step_rec(Ctx *x, const StepRec &r)
 
 // reps ordinary steps, one kernel at a time with an event after each, so
 // every kernel is timed inside the sequence it runs in; slots: flux, update,
-// bound_prim (3D; in 2D the update writes the ghosts), fixup_utoprim with the
+// bound_prim (where the update does not write the ghosts), fixup_utoprim with the
 // bound_prim after it, diagnostics
 int time_kernels(Ctx *x, int reps, double *ms)
 {
@@ -1044,7 +1048,7 @@ int time_kernels(Ctx *x, int reps, double *ms)
       if (full) launch_update<true>(x, pi, pb, pf);
       else launch_update<false>(x, pi, pb, pf);
       slot[e] = 1; CK(cudaEventRecord(ev[e++], x->stream));
-      if (G.n3 > 1) {
+      if (!update_writes_ghosts(G)) {
         launch_bound(x, pf);
         slot[e] = 2; CK(cudaEventRecord(ev[e++], x->stream));
       }

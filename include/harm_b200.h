@@ -165,8 +165,8 @@ int harm_step_ch_host_timed(harm_ctx *ctx, double *p, int nsteps, double *ms);
 /* Runs reps ordinary steps launched kernel by kernel with a CUDA event after
    each, and returns the average device time per launch of each kind, into
    ms[HARM_NKERNELS] in this order: flux (all directions), update (flux-CT + source
-   + inversion + floors + flags; in 2D the ghost cells too), bound_prim (3D; 0 in 2D),
-   fixup_utoprim with the bound_prim after it, diagnostics (flux and mass sums, next
+   + inversion + floors + flags; in 2D up to 56,832 zones and with COOL_EOS the ghost
+   cells too), bound_prim (0 where the update writes the ghosts), fixup_utoprim with the bound_prim after it, diagnostics (flux and mass sums, next
    dt, per step).  The state advances by reps steps. */
 #define HARM_NKERNELS 5
 int harm_time_kernels(harm_ctx *ctx, int reps, double *ms);

@@ -21,10 +21,10 @@ def test_fused_size_is_the_sources():
     assert bench.FUSED_ZONES == int(sms) * minb * int(threads)
 
 
-# 2D: flux, update, repair, or flux, emf, cons, invert, repair; 3D: flux, emf, update (or
+# 2D: flux, update, repair, or flux, emf, cons, invert, bound, repair; 3D: flux, emf, update (or
 # cons, invert), bound, repair, bound; and the sums once a step
 @pytest.mark.parametrize("grid,count", [((128, 128, 1), 2 * 3 + 1), ((444, 128, 1), 2 * 3 + 1),
-                                        ((445, 128, 1), 2 * 5 + 1), ((256, 256, 1), 2 * 5 + 1),
+                                        ((445, 128, 1), 2 * 6 + 1), ((256, 256, 1), 2 * 6 + 1),
                                         ((24, 20, 6), 2 * 6 + 1), ((70, 50, 22), 2 * 7 + 1),
                                         ((288, 256, 256), 2 * 7 + 1)])
 def test_gamma_law_launches(grid, count):

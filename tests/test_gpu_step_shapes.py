@@ -83,3 +83,27 @@ def test_mixed_step_tracks_oracle_across_the_launch_rules(shape, hc, oracle_buil
     l1 = l1_rel(active(pr, ctx.get_prims()), active(pr, o.p))
     assert l1[0] <= 1e-6, l1
     ctx.close()
+
+
+@pytest.mark.parametrize("shape", [(40, 36, 1), (241, 240, 1), (24, 20, 6)])
+def test_single_steps_before_and_after_the_graph(shape, hc):
+    """a context's first single steps are launched kernel by kernel, later ones from the
+    graph, and after a change of precision kernel by kernel again: the same steps"""
+    pr = hc.torus_problem(*shape)
+    a, b = hc.Context(pr), hc.Context(pr)
+    for c in (a, b):
+        c.init_torus()
+    for n, mode in ((11, a.FP64), (2, a.MIXED), (9, a.FP64)):
+        for c in (a, b):
+            c.set_precision(mode)
+        a.run(n)
+        for k in range(n):
+            if k % 2:
+                b.step_ch()
+            else:
+                p = b.get_prims()
+                b.step_ch_host(p)
+        np.testing.assert_array_equal(a.get_prims(), b.get_prims())
+        assert a.time() == b.time()
+    a.close()
+    b.close()
