@@ -1338,10 +1338,10 @@ static int step_graph(Ctx *x)
 }
 
 // One step: the graph, one launch for the host instead of one per kernel (32x32:
-// set_time, step_ch_host and get_time 165 -> 140 us).  Making it costs as much as some ten
+// set_time, step_ch_host and get_time 165 -> 140 us).  Making it costs as much as five to ten
 // steps' launches, so a context's first PLAIN_STEPS single steps, unless a run has made
 // it, go kernel by kernel, as does the seeding step of COOL_EOS, which comes once.
-constexpr int PLAIN_STEPS = 8;
+constexpr int PLAIN_STEPS = 5;
 static int one_step(Ctx *x)
 {
   if (x->cool && x->cool_seed) return launch_step(x);
